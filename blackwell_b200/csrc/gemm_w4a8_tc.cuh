@@ -100,6 +100,14 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// True on one lane of a converged warp.  tcgen05 instructions take their operands from uniform registers: where one lane alone
+// runs the issuing loop, the compiler moves the operands there lane by lane, 45 cycles per MMA and per commit (measured, 64
+// columns); where the whole warp runs it and an elected lane issues, an MMA costs its 32 cycles in the pipe and a commit nothing.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // D = A * B (accumulate == 0) or D += A * B.
 __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                           uint32_t accumulate) {

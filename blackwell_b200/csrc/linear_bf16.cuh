@@ -224,7 +224,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     unsigned char* stage0 = smem + 1024;
     float* part = reinterpret_cast<float*>(stage0);
     static_assert(!SPLIT || NT * kTcRows * 4 <= S * BYTES, "accumulator tile");
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31;   // the warp index is uniform
     auto full = [&](int i) { return smem_u32(&bars[i]); };
     auto empty = [&](int i) { return smem_u32(&bars[S + i]); };
     auto dfull = [&](int i) { return smem_u32(&bars[2 * S + i]); };
@@ -248,7 +248,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *tmem_ptr;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
     pdl_trigger();
 
     const int rtiles = (a.N + kTcRows - 1) / kTcRows, ttiles = (a.T + NT - 1) / NT, tiles = rtiles * ttiles;
@@ -293,18 +293,20 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 for (int i = max(0, n - S); i < n; ++i) mbar_wait(full(i % S), (i / S) & 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(NT);
-            int n = 0, w = 0;
-            bool ok = true;
-            for (int tile = first; tile < tiles && ok; tile += stride, ++w) {
-                const int d = w % NACC;
-                if (!wait(dempty(d), ((w / NACC) & 1) ^ 1)) { ok = false; break; }
+        // the whole warp walks the loop, one elected lane issues (see elect_one)
+        const uint32_t idesc = idesc_bf16(NT);
+        const bool elected = tc::elect_one();
+        int n = 0, w = 0;
+        bool ok = true;
+        for (int tile = first; tile < tiles && ok; tile += stride, ++w) {
+            const int d = w % NACC;
+            if (!(ok = __all_sync(0xffffffffu, wait(dempty(d), ((w / NACC) & 1) ^ 1)))) break;
+            tc::tc_fence_after();
+            for (int kb = kb0; kb < kb1; ++kb, ++n) {
+                const int s = n % S;
+                if (!(ok = __all_sync(0xffffffffu, wait(full(s), (n / S) & 1)))) break;
                 tc::tc_fence_after();
-                for (int kb = kb0; kb < kb1; ++kb, ++n) {
-                    const int s = n % S;
-                    if (!wait(full(s), (n / S) & 1)) { ok = false; break; }
-                    tc::tc_fence_after();
+                if (elected) {
                     const uint64_t da = desc_sw128(smem_u32(stage0 + s * BYTES));
                     const uint64_t db = desc_sw128(smem_u32(stage0 + s * BYTES + kTcRows * 128));
 #pragma unroll
@@ -312,8 +314,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         tc_mma_f16(tmem + d * NT, da + 2 * k, db + 2 * k, idesc, kb > kb0 || k > 0);
                     tc::tc_commit(empty(s));
                 }
-                if (ok) tc::tc_commit(dfull(d));
+                __syncwarp();
             }
+            if (ok && elected) tc::tc_commit(dfull(d));
+            __syncwarp();
         }
     } else if (warp >= 4) {
         const int quarter = warp & 3, half = (warp - 4) >> 2;
