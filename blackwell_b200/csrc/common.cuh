@@ -116,6 +116,18 @@ __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Shared memory of another block of the cluster, and the cluster's barrier.
+__device__ __forceinline__ float ld_dsmem(uint32_t addr, uint32_t rank) {
+    uint32_t ra;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ----------------------------------------------------------- integer helpers
 // Signed 8-bit x 8-bit 4-way dot product with 32-bit accumulate.
 __device__ __forceinline__ int dp4a_ss(uint32_t a, uint32_t b, int c) {

@@ -7,8 +7,8 @@
 #include <mutex>
 
 #include "../../include/blackwell_b200.h"
+#include "act_prep.cuh"
 #include "gemm_w4a8_tc.cuh"
-#include "gemv_w4_stream.cuh"
 #include "host_util.h"
 
 namespace bw {
@@ -30,29 +30,9 @@ namespace tc {
 __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int M, int Mpad,
                                                      int nchunks) {
     __shared__ float part[8];
-    __shared__ float rstd_s;
     const int m = blockIdx.y, t = threadIdx.x;
     const int nkb = a.K / 16;
-    float rstd = 1.f;
-    const bool needs_norm = (a.xkind == kXFloatNorm);
-    if (needs_norm && m < M) {
-        float ss = 0.f;
-        const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride);
-        for (int i = t; i < a.K / 4; i += 256) {
-            const float4 f = __ldg(p + i);
-            ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); ss = fmaf(f.z, f.z, ss); ss = fmaf(f.w, f.w, ss);
-        }
-        ss = warp_sum(ss);
-        if ((t & 31) == 0) part[t >> 5] = ss;
-        __syncthreads();
-        if (t == 0) {
-            float tot = 0.f;
-            for (int w = 0; w < 8; ++w) tot += part[w];
-            rstd_s = rsqrtf(tot / (float)a.K + a.eps);
-        }
-        __syncthreads();
-        rstd = rstd_s;
-    }
+    const float rstd = a.xkind == kXFloatNorm && m < M ? row_rstd(a, m, t, part) : 1.f;
     const int kb = blockIdx.x * 256 + t;
     if (kb >= nchunks * kBlocksPerChunk) return;
     uint32_t e[2] = {0, 0}, o[2] = {0, 0};
@@ -71,72 +51,23 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
 // prologue).  Grid (ceil(K / 1024), M), 256 threads; starts early under programmatic dependent launch.
 __global__ void __launch_bounds__(256) prep_plain_kernel(int8_t* xq, float* xs, const GemvArgs a, int M) {
     __shared__ float part[8];
-    __shared__ float rstd_s;
     pdl_trigger();
     pdl_wait();   // the activations come from the kernel before
     const int m = blockIdx.y, t = threadIdx.x;
-    float rstd = 1.f;
-    if (a.xkind == kXFloatNorm) {
-        float ss = 0.f;
-        const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride);
-        for (int i = t; i < a.K / 4; i += 256) {
-            const float4 f = __ldg(p + i);
-            ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); ss = fmaf(f.z, f.z, ss); ss = fmaf(f.w, f.w, ss);
-        }
-        ss = warp_sum(ss);
-        if ((t & 31) == 0) part[t >> 5] = ss;
-        __syncthreads();
-        if (t == 0) {
-            float tot = 0.f;
-            for (int w = 0; w < 8; ++w) tot += part[w];
-            rstd_s = rsqrtf(tot / (float)a.K + a.eps);
-        }
-        __syncthreads();
-        rstd = rstd_s;
-    }
+    const float rstd = a.xkind == kXFloatNorm ? row_rstd(a, m, t, part) : 1.f;
     // Four consecutive elements per thread, four threads per k-block (K % 32 == 0, so a block's threads are valid or
-    // not together); the element arithmetic is that of make_xblock, the rounding that of quantize_block.
+    // not together).
     const int e0 = (blockIdx.x * 256 + t) * 4;
     const bool valid = e0 < a.K;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (valid) {
-        if (a.xkind == kXHalf) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __half*>(a.x) + (size_t)m * a.x_stride + e0));
-            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-            v[0] = f0.x; v[1] = f0.y; v[2] = f1.x; v[3] = f1.y;
-        } else {
-            const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride + e0));
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-            if (a.xkind == kXFloatNorm) {
-                const float4 gw = __ldg(reinterpret_cast<const float4*>(a.norm_w + e0));
-                v[0] = v[0] * gw.x * rstd; v[1] = v[1] * gw.y * rstd; v[2] = v[2] * gw.z * rstd; v[3] = v[3] * gw.w * rstd;
-            } else if (a.xkind == kXSwiglu) {
-                const float4 u = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a.x2) + (size_t)m * a.x_stride + e0));
-                v[0] = silu_mul(v[0], u.x); v[1] = silu_mul(v[1], u.y); v[2] = silu_mul(v[2], u.z); v[3] = silu_mul(v[3], u.w);
-            }
-        }
-    }
+    if (valid) load_elements<4>(a, m, e0, rstd, v);
     float am = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
     if (!valid) return;
     const float sc = quant_scale_i8(am);
-    const float rcp = 1.0f / sc;
     uint32_t qb[4];
-    bool exact_needed = !(am < 3.0e38f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float r = v[i] * rcp;
-        const float mg = r + kMagicFloat;
-        const float ri = mg - kMagicFloat;
-        exact_needed |= !(fabsf(fabsf(r - ri) - 0.5f) > 3e-5f);
-        qb[i] = __float_as_uint(mg);
-    }
-    if (exact_needed) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) qb[i] = (uint32_t)quant_i8(v[i], sc);
-    }
+    round_elements<4>(v, am, sc, qb);
     *reinterpret_cast<uint32_t*>(xq + (size_t)m * a.K + e0) = prmt(prmt(qb[0], qb[1], 0x0040), prmt(qb[2], qb[3], 0x0040), 0x5410);
     if ((t & 3) == 0) xs[(size_t)m * (a.K / 16) + (e0 >> 4)] = sc;
 }
@@ -592,6 +523,8 @@ static EncodeTiledFn encode_fn() {
 
 // Per-device scratch: activation chunks, K-split partials, tickets (kept zero between calls).
 static GrowScratch g_tc_scratch;
+// The block of the tensor-core kernels (gemm_w4a8_wide.cu works in it too): arrival counters first.
+cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p) { return g_tc_scratch.get(bytes, (size_t)16 << 20, st, p); }
 cudaError_t reserve_scratch(size_t bytes) {
     unsigned char* p = nullptr;
     return bytes ? g_tc_scratch.get(bytes, (size_t)16 << 20, nullptr, &p) : cudaSuccess;

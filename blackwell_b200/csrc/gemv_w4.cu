@@ -6,6 +6,7 @@
 
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -32,6 +33,13 @@ void set_ksplit_override(int v);
 void set_ablate(int v);
 cudaError_t prepare_plain(const GemvArgs& a, int M, cudaStream_t st, const int8_t** xq_out, const float** xs_out);
 }  // namespace tc
+namespace wide {  // its bf16 form, gemm_w4a8_wide.cu
+bool preferred(int M, int N, int K);
+cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st);
+size_t scratch_bytes(int M, int N, int K);
+void set_split(int v);
+void set_force(int v);
+}  // namespace wide
 
 // --------------------------------------------------------------------------
 // Plain-load kernel: one warp per output row, lanes stride over k-blocks, up to
@@ -489,7 +497,7 @@ static cudaError_t gemv_dispatch(GemvArgs a, int M, cudaStream_t st) {
                 b.x = static_cast<const float*>(a.x) + (size_t)m0 * a.x_stride;
                 if (a.x2) b.x2 = static_cast<const float*>(a.x2) + (size_t)m0 * a.x_stride;
             }
-            cudaError_t e = tc::launch(b, mc, st);
+            cudaError_t e = wide::preferred(mc, a.N, a.K) ? wide::launch(b, mc, st) : tc::launch(b, mc, st);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -675,7 +683,9 @@ extern "C" int bw_gemv_block_dots(int32_t* dots, const void* x, int a8, const ui
     return cudaPeekAtLastError();
 }
 
-extern "C" size_t bw_gemv_scratch_bytes(int M, int N, int K) { return tc::scratch_bytes(M, N, K); }
+extern "C" size_t bw_gemv_scratch_bytes(int M, int N, int K) {
+    return std::max(tc::scratch_bytes(M, N, K), wide::scratch_bytes(M, N, K));
+}
 extern "C" size_t bw_attention_scratch_bytes(int M, int num_q_heads, int num_kv_heads, int max_context) {
     return attn_scratch_bytes(M, num_q_heads, num_kv_heads, max_context);
 }
@@ -694,7 +704,7 @@ extern "C" int bw_set_tuning(int key, int value) {
         case 3: g_tune_rg = value; return 0;
         case 4: g_tune_threads = value; return 0;
         case 5: g_tune_tc_min = value; return 0;
-        case 6: tc::set_ksplit_override(value); return 0;
+        case 6: tc::set_ksplit_override(value); wide::set_split(value); return 0;
         case 8: set_pdl(value); return 0;
         case 9: set_attn_mma(value); return 0;
         case 10: peer::set_two_step_min_kb(value); return 0;
@@ -710,6 +720,7 @@ extern "C" int bw_set_tuning(int key, int value) {
         case 20: g_tune_prep_min = value; return 0;
         case 21: g_tune_prep_min_swiglu = value; return 0;
         case 22: set_attn_slots_pct(value); return 0;
+        case 24: wide::set_force(value); return 0;
         case 23: lm::set_linear_stream_max(value); return 0;
         default: return cudaErrorInvalidValue;
     }

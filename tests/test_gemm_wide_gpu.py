@@ -1,0 +1,116 @@
+"""The bf16 tcgen05 form of the W4A8 product (17 to 64 sequences) against the double-precision oracle and, where all sums are
+exact integers, bit for bit against the dp4a kernel."""
+import numpy as np
+import pytest
+
+import oracle
+from blackwell_b200 import synth
+from tests.util import max_abs_rel, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def k(cuda):
+    """The kernels with every call of more than 16 sequences on this form."""
+    from blackwell_b200 import kernels
+
+    kernels.set_tuning(24, 1)
+    yield kernels
+    kernels.set_tuning(24, 0)
+
+
+# rows around a tile of 256 and its halves; K of one, a part of one and many chunks of 256, scale rows of 4-, 8- and 16-byte
+# pitch; every number of columns; shares that begin and end inside a tile, clusters (split 2..8), whole tiles (split 1)
+@pytest.mark.parametrize("M,K,N,split", [
+    (17, 32, 1, 0), (32, 256, 128, 0), (33, 288, 255, 0), (48, 544, 257, 9), (49, 4096, 129, 0), (64, 4096, 4096, 0),
+    (40, 10944, 512, 9), (64, 10944, 300, 9), (24, 2080, 40000, 9), (64, 1024, 40000, 1), (32, 4096, 700, 2), (48, 4096, 511, 5),
+    (64, 2048, 256, 8), (65, 1024, 256, 0), (100, 256, 130, 0)])
+def test_matches_the_oracle(k, M, K, N, split):
+    import torch
+
+    W, sc16, _ = synth.int4_weights(N, K, seed=M + K + N, full_range=True)
+    x32 = synth.activations_f16(M, K, 901).astype(np.float32) * 2.0
+    xq, xs = oracle.quantize_int8(x32)
+    args = [to_dev(xq), to_dev(xs), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    y2 = torch.full_like(y, float("nan"))
+    k.set_tuning(6, split)
+    try:
+        k.gemv_w4a8(y, *args)
+        k.gemv_w4a8(y2, *args)
+    finally:
+        k.set_tuning(6, 0)
+    torch.cuda.synchronize()
+    assert k.device_status() == 0
+    assert torch.equal(y, y2)
+    # fp32 sums of K / 16 block terms in K order: K / 16 roundings of 2^-24 at most, far less than the bar
+    assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
+
+
+def test_scales_of_every_kind_are_split_without_rounding(k):
+    """Subnormal, negative, largest and full-mantissa binary16 scales: one k-block per output and an activation scale of 1, so
+    that the output is w_sc * dot, at most 25 bits, to one rounding."""
+    import torch
+
+    M, K, N = 32, 32, 4096
+    r = synth.rng(77)
+    bits = r.integers(0, 1 << 16, size=(N, 2), dtype=np.uint16)
+    bits[(bits & 0x7C00) == 0x7C00] ^= 0x4000            # no infinities or NaN
+    bits[:64, 0] = np.arange(64)                          # subnormals
+    bits[64:68, 0] = [0x7BFF, 0xFBFF, 0x0400, 0x8001]
+    bits[:, 1] = 0
+    W, _, _ = synth.int4_weights(N, K, seed=5, full_range=True)
+    xq = r.integers(-127, 128, size=(M, K), dtype=np.int8)
+    xs = np.ones((M, 2), np.float32)
+    y = torch.empty((M, N), dtype=torch.float32, device="cuda")
+    k.gemv_w4a8(y, to_dev(xq), to_dev(xs), to_dev(W), to_dev(bits), K, N, M)
+    ref = oracle.gemv_w4a8_f64(xq, xs, W, bits.view(np.float16))
+    assert (np.abs(y.cpu().numpy() - ref) <= 2.0 ** -23 * np.abs(ref)).all()
+
+
+def test_integers_match_the_small_batch_kernel(k):
+    import torch
+
+    K, N = 1024, 300
+    W, _, _ = synth.int4_weights(N, K, seed=79, full_range=True)
+    ones16 = np.ones((N, K // 16), np.float16)
+    xq = synth.rng(907).integers(-127, 128, size=(64, K), dtype=np.int8)
+    xs = np.ones((64, K // 16), np.float32)
+    Wd, sd = to_dev(W), to_dev(ones16.view(np.uint16))
+    y4 = torch.empty((4, N), dtype=torch.float32, device="cuda")
+    k.gemv_w4a8(y4, to_dev(xq[:4]), to_dev(xs[:4]), Wd, sd, K, N, 4)
+    for M in (17, 48, 64):
+        y = torch.empty((M, N), dtype=torch.float32, device="cuda")
+        k.gemv_w4a8(y, to_dev(xq[:M]), to_dev(xs[:M]), Wd, sd, K, N, M)
+        assert torch.equal(y[:4], y4), M
+
+
+def test_prologues_strides_and_residual(k):
+    import torch
+
+    M, K, N = 40, 4096, 300
+    W, sc16, _ = synth.int4_weights(N, K, seed=78)
+    x32 = synth.activations_f16(M, K, 903).astype(np.float32)
+    nw = synth.norm_weight(K, 904)
+    res = synth.activations_f16(M, N + 4, 905).astype(np.float32)
+    Wd, sd = to_dev(W), to_dev(sc16.view(np.uint16))
+    y = to_dev(res.copy())
+    k.gemv_w4a8_decode(y, N + 4, y, to_dev(x32), None, 0, to_dev(nw), 1e-6, Wd, sd, K, N, M)
+    xq, xs = oracle.quantize_int8(oracle.rmsnorm(x32, nw))
+    ref = res.copy()
+    ref[:, :N] += oracle.gemv_w4a8_f64(xq, xs, W, sc16)
+    assert max_abs_rel(y.cpu().numpy(), ref) < 1e-3
+    assert np.array_equal(y.cpu().numpy()[:, N:], res[:, N:])
+    gud = to_dev(synth.activations_f16(M, 2 * K, 906).astype(np.float32))
+    y2 = torch.empty((M, N), dtype=torch.float32, device="cuda")
+    k.gemv_w4a8_decode(y2, 0, None, gud, gud[:, K:], 2 * K, None, 0.0, Wd, sd, K, N, M)
+    gu = gud.cpu().numpy()
+    xq, xs = oracle.quantize_int8(oracle.swiglu(np.ascontiguousarray(gu[:, :K]), np.ascontiguousarray(gu[:, K:])))
+    assert max_abs_rel(y2.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 1e-3
+    # binary16 input: the integers of the unfused quantizer
+    x16 = synth.activations_f16(M, K, 907)
+    k.gemv_w4a8_f16in(y2, to_dev(x16.view(np.uint16)), Wd, sd, K, N, M)
+    xq, xs = oracle.quantize_int8(x16.astype(np.float32))
+    assert max_abs_rel(y2.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
+    assert k.device_status() == 0
