@@ -174,42 +174,80 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(A* out, long ldout, con
     }
 }
 
-// The same with one group per head and the gate last: a warp per head.
-template <typename A>
-__global__ void __launch_bounds__(256) gated_norm_heads_kernel(A* out, long ldout, const float* o, long ldo, const A* gate, long ldg,
-                                                               const float* w, int heads, int V, float eps) {
+// The same for groups that are a run of columns in memory (one head each, or heads without padding): a warp per group, `V`
+// columns of it at a pitch of V8 = pad8(V), up to KV * 128 of them in registers, gate and weight in vectors of four where they are
+// aligned (VEC).  HBM bound; 4,096 rows of 8 groups of 512 columns: 36.7 us, 135 with a
+// block per group and scalar accesses.
+template <typename A, int KV, bool GATE_FIRST, bool VEC>
+__global__ void __launch_bounds__(256) gated_norm_runs_kernel(A* out, long ldout, const float* o, long ldo, const A* gate, long ldg,
+                                                              const float* w, int groups, int V, float eps) {
     pdl_trigger();
     pdl_wait();
     const int h = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, V8 = pad8(V);
-    if (h >= heads) return;
+    if (h >= groups) return;
     const long r = blockIdx.y;
-    const float* orow = o + r * ldo + h * V8;
-    const A* grow = gate + r * ldg + h * V8;
-    A* dst = out + r * ldout + h * V8;
-    constexpr int kVec = 4;   // first 512 columns in registers
-    float4 x[kVec];
+    const float* orow = o + r * ldo + (long)h * V8;
+    const A* grow = gate + r * ldg + (long)h * V8;
+    const float* wrow = w ? w + (long)h * V : nullptr;
+    A* dst = out + r * ldout + (long)h * V8;
+    auto gates = [&](int c, float (&g)[4]) {   // silu of four gates
+        if constexpr (VEC && sizeof(A) == 2) {
+            const uint2 u = *reinterpret_cast<const uint2*>(grow + c);
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+            g[0] = lo.x; g[1] = lo.y; g[2] = hi.x; g[3] = hi.y;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) g[e] = c + e < V ? to_f(grow[c + e]) : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[e] = silu_f(g[e]);
+    };
+    auto load = [&](int c) {   // columns V .. V8 of o are zero
+        float4 v = *reinterpret_cast<const float4*>(orow + c);
+        if (GATE_FIRST) {
+            float g[4];
+            gates(c, g);
+            v.x *= g[0]; v.y *= g[1]; v.z *= g[2]; v.w *= g[3];
+        }
+        return v;
+    };
+    float4 x[KV];
     float ss = 0.f;
     auto add = [&](const float4& v) { ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss)))); };
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {   // columns V .. V8 are zero
+    for (int j = 0; j < KV; ++j) {
         const int c = j * 128 + lane * 4;
-        x[j] = c < V8 ? *reinterpret_cast<const float4*>(orow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[j] = c < V8 ? load(c) : make_float4(0.f, 0.f, 0.f, 0.f);
         add(x[j]);
     }
-    for (int c = kVec * 128 + lane * 4; c < V8; c += 128) add(*reinterpret_cast<const float4*>(orow + c));
+    for (int c = KV * 128 + lane * 4; c < V8; c += 128) add(load(c));
     const float rms = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
     auto emit = [&](int c, const float4& v) {
-        const float y[4] = {v.x, v.y, v.z, v.w};
-        float z[4];
+        float z[4] = {v.x, v.y, v.z, v.w}, f[4] = {1.f, 1.f, 1.f, 1.f};
+        if (!GATE_FIRST) {
+            float g[4];
+            gates(c, g);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) z[e] = c + e < V ? y[e] * silu_f(to_f(grow[c + e])) * rms * (w ? w[(long)h * V + c + e] : 1.f) : 0.f;
+            for (int e = 0; e < 4; ++e) z[e] *= g[e];
+        }
+        if (wrow) {
+            if constexpr (VEC) {
+                *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(wrow + c);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f[e] = c + e < V ? wrow[c + e] : 0.f;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z[e] = c + e < V ? z[e] * rms * f[e] : 0.f;
         if constexpr (sizeof(A) == 2) *reinterpret_cast<uint2*>(dst + c) = make_uint2(pack_bf16(z[0], z[1]), pack_bf16(z[2], z[3]));
         else *reinterpret_cast<float4*>(dst + c) = make_float4(z[0], z[1], z[2], z[3]);
     };
 #pragma unroll
-    for (int j = 0; j < kVec; ++j)
+    for (int j = 0; j < KV; ++j)
         if (j * 128 + lane * 4 < V8) emit(j * 128 + lane * 4, x[j]);
-    for (int c = kVec * 128 + lane * 4; c < V8; c += 128) emit(c, *reinterpret_cast<const float4*>(orow + c));
+    for (int c = KV * 128 + lane * 4; c < V8; c += 128) emit(c, load(c));
 }
 
 // Conv channel of a padded column (counted from the start of the convolved part), -1 for padding.
@@ -391,22 +429,34 @@ cudaError_t norm_rows(void* xb, long ldxb, const float* x, const float* w, const
                : by_width(width, Norm<bf16, false>{xm, xb, ldxb, nullptr, w, nullptr, rows, T, width, eps, st});
 }
 
+// A warp per group where a group is a run of columns: heads of their own (what pads them is zero; behind a gate that comes first
+// it need not be), or several heads (or parts of one) without padding.
+template <typename A>
+static cudaError_t gated_norm_as(A* out, long ldout, const float* o, long ldo, const A* gate, long ldg, const float* w, int T, int heads,
+                                 int V, int groups, int gate_first, float eps, cudaStream_t st) {
+    auto aligned = [](const void* p, long ld, size_t elem) { return ((uintptr_t)p | (size_t)ld * elem) % (4 * elem) == 0; };
+    const int part = heads * V / groups;
+    const bool rows = aligned(o, ldo, 4) && aligned(out, ldout, sizeof(A));
+    if (!rows || !((groups == heads && !gate_first) || (V % 8 == 0 && part % 8 == 0)))
+        return launch_pdl(gated_norm_kernel<A>, dim3(groups, T), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, heads, V, groups,
+                          gate_first, eps);
+    const bool vec = part % 8 == 0 && aligned(gate, ldg, sizeof(A)) && (uintptr_t)w % 16 == 0;
+    const bool wide = part > 512;
+    auto kern = gate_first ? (vec ? (wide ? gated_norm_runs_kernel<A, 8, true, true> : gated_norm_runs_kernel<A, 4, true, true>)
+                                  : gated_norm_runs_kernel<A, 4, true, false>)
+                           : (vec ? (wide ? gated_norm_runs_kernel<A, 8, false, true> : gated_norm_runs_kernel<A, 4, false, true>)
+                                  : gated_norm_runs_kernel<A, 4, false, false>);
+    return launch_pdl(kern, dim3((groups + 7) / 8, T), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, groups, part, eps);
+}
+
 cudaError_t gated_norm(void* out, long ldout, const float* o, long ldo, const void* gate, long ldg, const float* w, int T,
                        int heads, int V, int groups, int gate_first, float eps, int f32, cudaStream_t st) {
     if (groups < 1 || (heads * V) % groups != 0) return cudaErrorInvalidValue;
-    const dim3 grid(groups, T), block(256);
     count_launch(1);
-    if (groups == heads && !gate_first) {
-        const dim3 by_heads((heads + 7) / 8, T);
-        return f32 ? launch_pdl(gated_norm_heads_kernel<float>, by_heads, block, 0, st, static_cast<float*>(out), ldout, o, ldo,
-                                static_cast<const float*>(gate), ldg, w, heads, V, eps)
-                   : launch_pdl(gated_norm_heads_kernel<bf16>, by_heads, block, 0, st, static_cast<bf16*>(out), ldout, o, ldo,
-                                static_cast<const bf16*>(gate), ldg, w, heads, V, eps);
-    }
-    return f32 ? launch_pdl(gated_norm_kernel<float>, grid, block, 0, st, static_cast<float*>(out), ldout, o, ldo,
-                            static_cast<const float*>(gate), ldg, w, heads, V, groups, gate_first, eps)
-               : launch_pdl(gated_norm_kernel<bf16>, grid, block, 0, st, static_cast<bf16*>(out), ldout, o, ldo,
-                            static_cast<const bf16*>(gate), ldg, w, heads, V, groups, gate_first, eps);
+    return f32 ? gated_norm_as(static_cast<float*>(out), ldout, o, ldo, static_cast<const float*>(gate), ldg, w, T, heads, V, groups,
+                               gate_first, eps, st)
+               : gated_norm_as(static_cast<bf16*>(out), ldout, o, ldo, static_cast<const bf16*>(gate), ldg, w, T, heads, V, groups,
+                               gate_first, eps, st);
 }
 
 cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st) {
