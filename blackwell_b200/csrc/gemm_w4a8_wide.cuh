@@ -26,8 +26,8 @@
 // A pair is the blocks (p, p + 8) of a chunk, so that a thread's eight blocks are consecutive: its scales are 16 bytes, its
 // nibbles come two blocks per 16-byte load.  Scalar FMAs, not packed ones: the packed form goes to half of the FMA pipe, which
 // the bf16 FMAs of the unpack already fill (708 against 517 us, same case).
-// What bounds it (counters at 8 and 64 columns): issue slots 50-60 % busy with 4.5 warps per scheduler, then the latency chain
-// of a worker's step; HBM 12-20 %, tensor pipe 11 %.
+// What bounds it (75,776 x 4096, 48 / 64 sequences): issue slots 68 % busy with five warps per scheduler, then the latency chain
+// of a worker's step; HBM 12 / 9 %.
 // All waits are bounded; a wait that gives up raises an abort flag.
 #pragma once
 #include <cuda_bf16.h>

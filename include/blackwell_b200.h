@@ -48,7 +48,7 @@ int bw_gemv_int4_warp(float* y_out, const void* x_packed, const float* x_scale, 
  * src/kernels/gemv_int8.cu:937-965 with the int8 operand of :718-748.
  * Any M >= 1.  Batch routing of all bw_gemv_w4a8* entry points (by measurement; bw_set_tuning keys 5, 13, 14 move
  * the borders): up to 4 sequences run in the streaming dp4a kernel, 5 to 16 in the streaming mma.sync kernel, more
- * than 16 (K % 32 == 0, 16-byte aligned W and x) in the tcgen05 kernel, 64 sequences per launch; operands the
+ * than 16 (K % 32 == 0, 16-byte aligned W and x) in one of the tcgen05 kernels, 64 sequences per launch; operands the
  * tensor-core kernel cannot take fall back to passes of 16 through the mma.sync kernel (or 8 through dp4a). */
 int bw_gemv_w4a8(float* y_out, const int8_t* x_q, const float* x_scale, const uint8_t* W_packed,
                  const uint16_t* W_scale_f16, int K, int N, int M, void* stream);
@@ -539,7 +539,9 @@ int bw_reserve_scratch(size_t gemv_bytes, size_t attention_bytes);
  * same for the SwiGLU prologue (0 = default 1), key 22 = decode attention: the earlier split rule with pct % of the SMs
  * as CTA slots (0 = default rule: one wave of two CTAs per SM, at least 224 positions per split),
  * key 23 = bfloat16 linear: up to value - 1 rows (8 at most) take the weight-streaming kernel, more the tcgen05 kernel (0 =
- * automatic). */
+ * automatic), key 24 = products of more than 16 sequences on the tcgen05 kernel's bf16 form (positive: always, negative:
+ * never, 0 = by its estimate of both forms; key 6 there: 1 = whole tiles, 2 to 8 = CTAs of a cluster that share a tile,
+ * more = equal shares of all chunks). */
 int bw_set_tuning(int key, int value);
 /* Number of kernels launched by this library since the last call with reset != 0. */
 long long bw_launch_count(int reset);
