@@ -98,16 +98,23 @@ __device__ __forceinline__ void zero_smem(unsigned char* p, int bytes, int t, in
     for (int i = t * 16; i < bytes; i += threads * 16) *reinterpret_cast<uint4*>(p + i) = make_uint4(0, 0, 0, 0);
 }
 
-// Sum over a block of up to 1024 threads; every thread gets the total.  `buf`: 32 floats of shared memory.
-__device__ __forceinline__ float block_sum(float v, float* buf) {
-    v = warp_sum(v);
-    const int warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if ((threadIdx.x & 31) == 0) buf[warp] = v;
+// Sum over a block of up to 1024 threads; every thread gets the total.  `buf`: 32 floats of shared memory.  With several values per
+// thread (up to 32 in all warps) the sum is that of a block with as many times the threads, value h of thread t belonging to its
+// thread h * blockDim.x + t, in that block's order.
+template <int V>
+__device__ __forceinline__ float block_sum(const float (&v)[V], float* buf) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+    const float s = warp_sum_many(v, lane);
+    if ((lane & (32 / V - 1)) == 0) buf[warp_sum_many_index<V>(lane) * nw + warp] = s;
     __syncthreads();
     float t = 0.f;
-    for (int i = 0; i < nw; ++i) t += buf[i];
+    for (int i = 0; i < nw * V; ++i) t += buf[i];
     __syncthreads();
     return t;
+}
+__device__ __forceinline__ float block_sum(float v, float* buf) {
+    const float one[1] = {v};
+    return block_sum(one, buf);
 }
 
 }  // namespace lm

@@ -15,9 +15,13 @@ namespace {
 
 // Row kernels: a block per row, VEC neighbouring columns per access (4, or 1 for widths that are not a multiple of 4), the
 // first KEEP vectors of a thread in registers.  Weights are fetched before the kernel waits for its predecessor.
-template <int VEC, int KEEP>
+// SHARES: a thread does the work of that many threads of the instance with SHARES times as many (vector j is that of share
+// j % SHARES).  Their sums are kept apart and added in that instance's order, so that a row has the same bits either way and
+// does not depend on how many rows there are.
+template <int VEC, int KEEP, int SHARES>
 struct RowVecs {
-    static constexpr int kKeep = KEEP;
+    static constexpr int kVec = VEC, kKeep = KEEP, kShares = SHARES;
+    static_assert(KEEP % SHARES == 0 && SHARES <= 4, "shares");
     float v[kKeep][VEC];
     static __device__ __forceinline__ int col(int j) { return (j * blockDim.x + threadIdx.x) * VEC; }
     static __device__ __forceinline__ void get(const float* p, float (&x)[VEC]) {
@@ -41,15 +45,20 @@ struct RowVecs {
             if (p && col(j) < width) get(p + col(j), v[j]);
         }
     }
-    __device__ __forceinline__ float squares() const {
-        float s = 0.f;
+    // Sum over the row of the squares of the kept values and of f(column) for the others; every thread gets it.
+    template <typename F>
+    __device__ __forceinline__ float sum_squares(int width, float* buf, F f) const {
+        float s[kShares];
+#pragma unroll
+        for (int h = 0; h < kShares; ++h) s[h] = 0.f;
 #pragma unroll
         for (int j = 0; j < kKeep; ++j)
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) s = fmaf(v[j][e], v[j][e], s);
-        return s;
+            for (int e = 0; e < VEC; ++e) s[j % kShares] = fmaf(v[j][e], v[j][e], s[j % kShares]);
+        beyond(width, [&](int i) { const float x = f(i); s[0] = fmaf(x, x, s[0]); });
+        return block_sum(s, buf);
     }
-    // f(column) for the columns that are not kept
+    // f(column) for the columns that are not kept (none where SHARES > 1)
     template <typename F>
     static __device__ __forceinline__ void beyond(int width, F f) {
         for (int i = kKeep * blockDim.x * VEC + threadIdx.x; i < width; i += blockDim.x) f(i);
@@ -57,16 +66,12 @@ struct RowVecs {
 };
 
 // xb = x / rms(x) * next (next NULL: x) for the block's row x, of which `keep` holds the first values, `gain` those of next.
-template <typename A, int VEC, int KEEP>
-__device__ __forceinline__ void next_input(A* xb, const float* x, const float* next, const RowVecs<VEC, KEEP>& keep,
-                                           const RowVecs<VEC, KEEP>& gain, int width, float eps, float* buf) {
-    typedef RowVecs<VEC, KEEP> R;
+template <typename A, typename R>
+__device__ __forceinline__ void next_input(A* xb, const float* x, const float* next, const R& keep, const R& gain, int width, float eps,
+                                           float* buf) {
+    constexpr int VEC = R::kVec;
     float f = 1.f;
-    if (next) {
-        float ss = keep.squares();
-        R::beyond(width, [&](int i) { ss = fmaf(x[i], x[i], ss); });
-        f = 1.0f / sqrtf(block_sum(ss, buf) / (float)width + eps);
-    }
+    if (next) f = 1.0f / sqrtf(keep.sum_squares(width, buf, [&](int i) { return x[i]; }) / (float)width + eps);
 #pragma unroll
     for (int j = 0; j < R::kKeep; ++j)
         if (R::col(j) < width) {
@@ -78,11 +83,11 @@ __device__ __forceinline__ void next_input(A* xb, const float* x, const float* n
     R::beyond(width, [&](int i) { xb[i] = from_f<A>(x[i] * f * (next ? next[i] : 1.f)); });
 }
 
-template <typename A, int VEC, int KEEP>
+template <typename A, int VEC, int KEEP, int SHARES>
 __global__ void __launch_bounds__(512) embed_kernel(float* x, A* xb, long ldxb, const bf16* table, long ldt, const int* tokens,
                                                     int width, int vocab, float scale, const float* next, float eps) {
     __shared__ float buf[32];
-    typedef RowVecs<VEC, KEEP> R;
+    typedef RowVecs<VEC, KEEP, SHARES> R;
     R gain, keep;
     gain.load(next, width, 1.f);
     pdl_trigger();
@@ -100,15 +105,15 @@ __global__ void __launch_bounds__(512) embed_kernel(float* x, A* xb, long ldxb, 
         if (c < width) R::put(xr + c, keep.v[j]);
     }
     R::beyond(width, [&](int i) { xr[i] = to_f(row[i]) * scale; });   // read again by this thread alone
-    next_input<A, VEC, KEEP>(xb + r * ldxb, xr, next, keep, gain, width, eps, buf);
+    next_input<A, R>(xb + r * ldxb, xr, next, keep, gain, width, eps, buf);
 }
 
 // ADD: x += y / rms(y) * w and xb = the next sublayer's input; otherwise xb = x / rms(x) * w for a listed row.
-template <typename A, int VEC, int KEEP, bool ADD>
+template <typename A, int VEC, int KEEP, int SHARES, bool ADD>
 __global__ void __launch_bounds__(512) norm_kernel(float* x, A* xb, long ldxb, const float* y, const float* w, const float* next,
                                                    const int* rows, int width, float eps) {
     __shared__ float buf[32];
-    typedef RowVecs<VEC, KEEP> R;
+    typedef RowVecs<VEC, KEEP, SHARES> R;
     R weight, gain, keep, sum;
     weight.load(w, width, 0.f);
     if (ADD) gain.load(next, width, 1.f);
@@ -120,9 +125,7 @@ __global__ void __launch_bounds__(512) norm_kernel(float* x, A* xb, long ldxb, c
     const float* src = ADD ? y + r * width : xr;
     keep.load(src, width, 0.f);
     if (ADD) sum.load(xr, width, 0.f);
-    float ss = keep.squares();
-    R::beyond(width, [&](int i) { ss = fmaf(src[i], src[i], ss); });
-    const float rms = 1.0f / sqrtf(block_sum(ss, buf) / (float)width + eps);
+    const float rms = 1.0f / sqrtf(keep.sum_squares(width, buf, [&](int i) { return src[i]; }) / (float)width + eps);
     A* xo = xb + out_row * ldxb;
 #pragma unroll
     for (int j = 0; j < R::kKeep; ++j) {
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(512) norm_kernel(float* x, A* xb, long ldxb, c
         if (ADD) xr[i] += v;
         else xo[i] = from_f<A>(v);
     });
-    if (ADD) next_input<A, VEC, KEEP>(xo, xr, next, keep, gain, width, eps, buf);
+    if (ADD) next_input<A, R>(xo, xr, next, keep, gain, width, eps, buf);
 }
 
 template <typename A>
@@ -376,37 +379,39 @@ __global__ void __launch_bounds__(128) conv_ring_kernel(const ConvArgs c, const 
 
 namespace {
 
-constexpr int kManyRows = 592;   // four blocks for each of 148 SMs
-
-// threads of a row kernel for `vec` columns each, up to 512
+// threads of a row kernel: one access per thread, up to 512
 int row_threads(int width, int vec) { return std::min(512, std::max(64, (width / vec + 31) / 32 * 32)); }
 
-// Calls f<VEC, KEEP>(threads) with the instance for this width.  Few rows: one access per thread, the shortest chain.  Rows for
-// several blocks per SM: four accesses per thread and a quarter of the threads, whose block sums cost a quarter of the warps
-// (4,096 rows of 2,048 columns, norm with residual, under ncu: 21.4 us against 27.8).
+// Calls f<VEC, KEEP, SHARES>(threads) with the instance for this width.  Few rows: one access per thread, the shortest chain.  Rows
+// for more than three quarters of the threads that the SMs hold: the work of four threads in one, whose block sums cost a quarter of
+// the warps.  Measured, norm with residual, us, four in one / one each: 2,048 columns 5.0 / 6.4 at 445 rows, 5.6 / 7.6 at 592, 25.4 /
+// 34.2 at 4,096; 1,024 columns 4.1 / 4.0 at 592, 4.9 / 5.6 at 890; 512 columns 2.7 / 2.4 at 592, 3.5 / 3.4 at 1,000, 4.9 / 5.6 at
+// 1,800.  Two in one beyond 2,048 columns gains nothing (4,096 rows of 4,096: 57.6 / 55.2).
 template <typename F>
 cudaError_t by_width(int width, int T, F f) {
-    if (width % 4 != 0) return f.template operator()<1, 4>(row_threads(width, 1));
-    if (width <= 8192 && width >= 512 && T >= kManyRows) return f.template operator()<4, 4>(row_threads(width, 16));
+    if (width % 4 != 0) return f.template operator()<1, 4, 1>(row_threads(width, 1));
     const int threads = row_threads(width, 4);
-    return width <= 2048 ? f.template operator()<4, 1>(threads) : width <= 4096 ? f.template operator()<4, 2>(threads) : f.template operator()<4, 4>(threads);
+    if (width <= 2048 && threads % 128 == 0 && (long)T * threads > 1536l * sm_count(current_device()))
+        return f.template operator()<4, 4, 4>(threads / 4);
+    return width <= 2048 ? f.template operator()<4, 1, 1>(threads) : width <= 4096 ? f.template operator()<4, 2, 1>(threads)
+                                                                                  : f.template operator()<4, 4, 1>(threads);
 }
 template <typename A>
 struct Embed {
     float* x; void* xb; long ldxb; const bf16* table; long ldt; const int* tokens; int T, width, vocab; float scale; const float* next;
     float eps; cudaStream_t st;
-    template <int VEC, int KEEP>
+    template <int VEC, int KEEP, int SHARES>
     cudaError_t operator()(int threads) const {
-        return launch_pdl(embed_kernel<A, VEC, KEEP>, dim3(T), dim3(threads), 0, st, x, static_cast<A*>(xb), ldxb, table, ldt,
+        return launch_pdl(embed_kernel<A, VEC, KEEP, SHARES>, dim3(T), dim3(threads), 0, st, x, static_cast<A*>(xb), ldxb, table, ldt,
                           tokens, width, vocab, scale, next, eps);
     }
 };
 template <typename A, bool ADD>
 struct Norm {
     float* x; void* xb; long ldxb; const float *y, *w, *next; const int* rows; int T, width; float eps; cudaStream_t st;
-    template <int VEC, int KEEP>
+    template <int VEC, int KEEP, int SHARES>
     cudaError_t operator()(int threads) const {
-        return launch_pdl(norm_kernel<A, VEC, KEEP, ADD>, dim3(T), dim3(threads), 0, st, x, static_cast<A*>(xb), ldxb, y, w, next,
+        return launch_pdl(norm_kernel<A, VEC, KEEP, SHARES, ADD>, dim3(T), dim3(threads), 0, st, x, static_cast<A*>(xb), ldxb, y, w, next,
                           rows, width, eps);
     }
 };
