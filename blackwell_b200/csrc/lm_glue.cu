@@ -177,18 +177,19 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(A* out, long ldout, con
     }
 }
 
-// The same for groups that are a run of columns in memory (one head each, or heads without padding): a warp per group, `V`
-// columns of it at a pitch of V8 = pad8(V), up to KV * 128 of them in registers, gate and weight in vectors of four where they are
-// aligned (VEC).  HBM bound; 4,096 rows of 8 groups of 512 columns: 36.7 us, 135 with a
-// block per group and scalar accesses.
+// The same for groups that are a run of columns in memory (one head each with the gate last, or heads without padding with the gate
+// first): a warp per group, `V` columns of it at a pitch of V8 = pad8(V), up to KV * 128 of them in registers, gate and weight in
+// vectors of four where they are aligned (VEC).  GATE_FIRST sums in the order of the 256 threads of gated_norm_kernel, so that a
+// group has the same bits there and here; it takes up to KV * 128 columns.
 template <typename A, int KV, bool GATE_FIRST, bool VEC>
 __global__ void __launch_bounds__(256) gated_norm_runs_kernel(A* out, long ldout, const float* o, long ldo, const A* gate, long ldg,
-                                                              const float* w, int groups, int V, float eps) {
+                                                              const float* w, int T, int groups, int V, float eps) {
     pdl_trigger();
     pdl_wait();
-    const int h = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, V8 = pad8(V);
-    if (h >= groups) return;
-    const long r = blockIdx.y;
+    const int g = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, V8 = pad8(V);
+    const int row = g / groups, h = g - row * groups;
+    if (row >= T) return;
+    const long r = row;
     const float* orow = o + r * ldo + (long)h * V8;
     const A* grow = gate + r * ldg + (long)h * V8;
     const float* wrow = w ? w + (long)h * V : nullptr;
@@ -216,16 +217,48 @@ __global__ void __launch_bounds__(256) gated_norm_runs_kernel(A* out, long ldout
         return v;
     };
     float4 x[KV];
-    float ss = 0.f;
-    auto add = [&](const float4& v) { ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss)))); };
 #pragma unroll
     for (int j = 0; j < KV; ++j) {
         const int c = j * 128 + lane * 4;
         x[j] = c < V8 ? load(c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        add(x[j]);
     }
-    for (int c = KV * 128 + lane * 4; c < V8; c += 128) add(load(c));
-    const float rms = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
+    float ss;
+    if constexpr (GATE_FIRST) {
+        // column c is thread c % 256's: vector j of a lane is that of warp 4 (j % 2) + lane / 8 there, its element e of lane
+        // 4 (lane % 8) + e
+        float a[8] = {};
+#pragma unroll
+        for (int j = 0; j < KV; ++j) {
+            const float v[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[4 * (j & 1) + e] = fmaf(v[e], v[e], a[4 * (j & 1) + e]);
+        }
+        // a warp's tree: its lane bits 4, 3, 2 are lane bits 2, 1, 0 here, handing over half of the values at each; then e
+        auto halve = [&](int bit, int n) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                const float keep = upper ? a[i + n] : a[i], send = upper ? a[i] : a[i + n];
+                a[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            }
+        };
+        halve(4, 4);
+        halve(2, 2);
+        halve(1, 1);
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+        ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss += __shfl_sync(0xffffffffu, a[0], (i & 3) * 8 + (i >> 2) * 4);   // the warps in turn
+    } else {
+        ss = 0.f;
+        auto add = [&](const float4& v) { ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss)))); };
+#pragma unroll
+        for (int j = 0; j < KV; ++j) add(x[j]);
+        for (int c = KV * 128 + lane * 4; c < V8; c += 128) add(load(c));
+        ss = warp_sum(ss);
+    }
+    const float rms = 1.0f / sqrtf(ss / (float)V + eps);
     auto emit = [&](int c, const float4& v) {
         float z[4] = {v.x, v.y, v.z, v.w}, f[4] = {1.f, 1.f, 1.f, 1.f};
         if (!GATE_FIRST) {
@@ -250,7 +283,8 @@ __global__ void __launch_bounds__(256) gated_norm_runs_kernel(A* out, long ldout
 #pragma unroll
     for (int j = 0; j < KV; ++j)
         if (j * 128 + lane * 4 < V8) emit(j * 128 + lane * 4, x[j]);
-    for (int c = KV * 128 + lane * 4; c < V8; c += 128) emit(c, load(c));
+    if constexpr (!GATE_FIRST)
+        for (int c = KV * 128 + lane * 4; c < V8; c += 128) emit(c, load(c));
 }
 
 // Conv channel of a padded column (counted from the start of the convolved part), -1 for padding.
@@ -440,24 +474,30 @@ cudaError_t norm_rows(void* xb, long ldxb, const float* x, const float* w, const
                : by_width(width, T, Norm<bf16, false>{xm, xb, ldxb, nullptr, w, nullptr, rows, T, width, eps, st});
 }
 
-// A warp per group where a group is a run of columns: heads of their own (what pads them is zero; behind a gate that comes first
-// it need not be), or several heads (or parts of one) without padding.
+// A warp per group where a group is a run of columns and the warps in flight make up for its serial chain, otherwise a block per
+// group.  Measured with the gate first, us, a warp / a block: groups of 128 columns 2.0 / 2.2 at 32 groups in all, 50 / 249 at
+// 131,072; of 512 columns 3.6 / 3.0 at 8, 3.8 / 3.8 at 256, 6.3 / 11.8 at 2,368, 33 / 130 at 32,768; of 520 to 1,024 columns
+// 7.2 / 6.5 (1,024) and 4.5 / 4.4 (520) at 592, 8.8 / 10.8 (1,024) and 4.6 / 6.8 (520) at 800, 37 / 111 at 16,384.  Longer groups
+// lie beyond a warp's registers.
 template <typename A>
 static cudaError_t gated_norm_as(A* out, long ldout, const float* o, long ldo, const A* gate, long ldg, const float* w, int T, int heads,
                                  int V, int groups, int gate_first, float eps, cudaStream_t st) {
     auto aligned = [](const void* p, long ld, size_t elem) { return ((uintptr_t)p | (size_t)ld * elem) % (4 * elem) == 0; };
     const int part = heads * V / groups;
+    const long all = (long)T * groups;
     const bool rows = aligned(o, ldo, 4) && aligned(out, ldout, sizeof(A));
-    if (!rows || !((groups == heads && !gate_first) || (V % 8 == 0 && part % 8 == 0)))
+    const bool vec = part % 8 == 0 && aligned(gate, ldg, sizeof(A)) && (uintptr_t)w % 16 == 0;
+    const int sms = sm_count(current_device());
+    const bool runs = gate_first ? V % 8 == 0 && vec && (part <= 128 || (part <= 512 && all >= 2 * sms) || (part <= 1024 && all > 4 * sms))
+                                 : groups == heads;
+    if (!rows || !runs || all > 0x7ffffff0)
         return launch_pdl(gated_norm_kernel<A>, dim3(groups, T), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, heads, V, groups,
                           gate_first, eps);
-    const bool vec = part % 8 == 0 && aligned(gate, ldg, sizeof(A)) && (uintptr_t)w % 16 == 0;
     const bool wide = part > 512;
-    auto kern = gate_first ? (vec ? (wide ? gated_norm_runs_kernel<A, 8, true, true> : gated_norm_runs_kernel<A, 4, true, true>)
-                                  : gated_norm_runs_kernel<A, 4, true, false>)
+    auto kern = gate_first ? (wide ? gated_norm_runs_kernel<A, 8, true, true> : gated_norm_runs_kernel<A, 4, true, true>)
                            : (vec ? (wide ? gated_norm_runs_kernel<A, 8, false, true> : gated_norm_runs_kernel<A, 4, false, true>)
                                   : gated_norm_runs_kernel<A, 4, false, false>);
-    return launch_pdl(kern, dim3((groups + 7) / 8, T), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, groups, part, eps);
+    return launch_pdl(kern, dim3((unsigned)(all + 7) / 8), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, T, groups, part, eps);
 }
 
 cudaError_t gated_norm(void* out, long ldout, const float* o, long ldo, const void* gate, long ldg, const float* w, int T,
