@@ -217,6 +217,7 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
         const bool elected = elect_one();
         bool ok = true;
         uint32_t ph = 0;   // phase of the A slots
+        pdl_wait();        // see the workers' first wait for activations
         Stage st;
         for (int n = 0; n < total && ok; ++n) {
             const int s = n % S;
@@ -328,7 +329,7 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
                 }
                 return true;
             }
-            pdl_wait();   // y may still be read, the partial tiles still be summed by the kernels before
+            // (y may still be read, the partial tiles still be summed by the kernels before: past the dependency wait since chunk 0)
             if (begin == first && wlast == first + a.nchunks - 1) {
 #pragma unroll
                 for (int j = 0; j < CW; ++j) {
@@ -469,6 +470,9 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
                         if ((n == total || (w0 + n) % a.nchunks == 0) && !(ok = finish(w0 + n - 1))) break;
                     }
                     if (n == total) break;
+                    // The limit of a wait counts this kernel's own progress, not the time until the activations' producers are done
+                    // (an exchange before them may wait longer for a late rank).
+                    if (n == 0) pdl_wait();
                     if (!(ok = wait(Sh::kFullX + s, (n / S) & 1))) break;
                     xs = reinterpret_cast<const float*>(ring + s * Sh::BYTES + kWBytes + xop_bytes(NP)) + cg * CW;
                 }
@@ -479,7 +483,6 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
         if (a.csize > 1) {
             __syncwarp();
             cluster_sync_all();   // every CTA's share of the tile is in its shared memory
-            pdl_wait();
             const int tile = w0 / a.nchunks, rank = blockIdx.x % a.csize;
             const int r0 = kRows * rank / a.csize, nr = kRows * (rank + 1) / a.csize - r0;
             const uint32_t base = smem_u32(ring);

@@ -122,6 +122,45 @@ def test_peer_wait_runs_out_and_the_next_call_works():
         c1.close()
 
 
+@pytest.mark.parametrize("M", [32])
+def test_a_product_waits_as_long_as_the_exchange_before_it(M):
+    """A product that starts early behind an exchange whose peer is late must not count that time against its own waits, which
+    give up after 2.5e9 cycles: here the peer never signals and the exchange gives up after 2.9e9 (1.4 s on the key's scale).  Only
+    rank 0 launches; the exchange's wait is bounded."""
+
+    import oracle
+    from blackwell_b200 import kernels as k
+    from blackwell_b200 import synth
+    from blackwell_b200.peer import PeerComm
+    from tests.util import max_abs_rel, to_dev
+
+    dev = torch.device("cuda", 0)
+    K, N, n = 4096, 512, 4096
+    W, sc16, _ = synth.int4_weights(N, K, seed=78)
+    x16 = synth.activations_f16(M, K, 907)
+    args = [to_dev(x16.view(np.uint16)), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
+    y = torch.empty((M, N), dtype=torch.float32, device=dev)
+    out = torch.empty((n,), dtype=torch.float32, device=dev)
+    k.gemv_w4a8_f16in(y, *args)   # sizes the scratch: no allocation between the two calls below
+    y.fill_(float("nan"))
+    c0, c1 = PeerComm(2, 0, n, dev), PeerComm(2, 1, n, dev)
+    k.set_tuning(11, 1400)
+    try:
+        c0.attach(c1)
+        torch.cuda.synchronize()
+        c0.allreduce(0, out, n)   # rank 1 never signals
+        k.gemv_w4a8_f16in(y, *args)
+        torch.cuda.synchronize()
+        assert c0.status() == 3
+        assert k.device_status() == 0
+        assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(*oracle.quantize_int8(x16.astype(np.float32)), W, sc16)) < 2e-5
+    finally:
+        k.set_tuning(11, 0)
+        torch.cuda.synchronize()
+        c0.close()
+        c1.close()
+
+
 def test_peer_allreduce_rejects_bad_arguments():
     from blackwell_b200.kernels import KernelError
     from blackwell_b200.peer import PeerComm
