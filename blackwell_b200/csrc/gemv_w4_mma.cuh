@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_w4_mma_kernel(const GemvArgs
                     const int cols = min(p.slab_cols, wc1 - c0);
                     const int s = item % S;
                     if (item >= S) {
+                        if (item == S) pdl_wait();   // as the consumers: the limit below counts this kernel's own progress
                         if (!mbar_wait(smem_u32(&empty[s]), ((item / S) & 1) ^ 1)) { *abort_flag = 1; ok = false; break; }
                     }
                     if (*abort_flag) { ok = false; break; }

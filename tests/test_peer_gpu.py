@@ -122,8 +122,8 @@ def test_peer_wait_runs_out_and_the_next_call_works():
         c1.close()
 
 
-@pytest.mark.parametrize("M", [32])
-def test_a_product_waits_as_long_as_the_exchange_before_it(M):
+@pytest.mark.parametrize("M,N", [(32, 512), (8, 40000)])
+def test_a_product_waits_as_long_as_the_exchange_before_it(M, N):
     """A product that starts early behind an exchange whose peer is late must not count that time against its own waits, which
     give up after 2.5e9 cycles: here the peer never signals and the exchange gives up after 2.9e9 (1.4 s on the key's scale).  Only
     rank 0 launches; the exchange's wait is bounded."""
@@ -135,7 +135,7 @@ def test_a_product_waits_as_long_as_the_exchange_before_it(M):
     from tests.util import max_abs_rel, to_dev
 
     dev = torch.device("cuda", 0)
-    K, N, n = 4096, 512, 4096
+    K, n = 4096, 4096
     W, sc16, _ = synth.int4_weights(N, K, seed=78)
     x16 = synth.activations_f16(M, K, 907)
     args = [to_dev(x16.view(np.uint16)), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
