@@ -5,6 +5,12 @@
 
 namespace bw {
 
+// The arrival counters of the product that follows start at zero whatever became of earlier calls (a product that gave up in a
+// wait leaves tiles half counted).  Every thread of a prep kernel of 256 threads a block, after its dependency wait.
+__device__ __forceinline__ void zero_counters(unsigned int* counters, int n) {
+    const int step = gridDim.x * gridDim.y * 256;
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x; i < n; i += step) counters[i] = 0;
+}
 // Sum of squares of one row by 256 threads -> 1 / rms, the same on every thread.
 __device__ __forceinline__ float row_rstd(const GemvArgs& a, int m, int t, float* part) {
     float ss = 0.f;

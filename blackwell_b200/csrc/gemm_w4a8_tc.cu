@@ -25,11 +25,13 @@ namespace tc {
 // streaming kernel's prologue: plain / RMSNorm / SwiGLU, int8 rule) and stores it in the layout the MMA's B
 // operand wants, chunk by chunk:
 //   chunk c: [block 0..15][Mpad rows x 16 B]   then   [block 0..15][Mpad] float scales / 16 * 2^39
-// Rows >= M and k-blocks >= K/16 are zero with scale 0.  Grid (ceil(nkb_pad / 256), Mpad), 256 threads.
+// Rows >= M and k-blocks >= K/16 are zero with scale 0.  Zeroes the arrival counters of a K split (`ncounters`, or 0).  Grid
+// (ceil(nkb_pad / 256), Mpad), 256 threads.
 // ----------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int M, int Mpad,
-                                                     int nchunks) {
+                                                     int nchunks, unsigned int* counters, int ncounters) {
     __shared__ float part[8];
+    zero_counters(counters, ncounters);
     const int m = blockIdx.y, t = threadIdx.x;
     const int nkb = a.K / 16;
     const float rstd = a.xkind == kXFloatNorm && m < M ? row_rstd(a, m, t, part) : 1.f;
@@ -484,7 +486,6 @@ gemm_w4a8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const TcArgs a) {
                         }
                     }
                     asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-                    if (t == 128) a.tickets[tile] = 0;
                 }
             }
         }
@@ -521,7 +522,7 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// Per-device scratch: activation chunks, K-split partials, tickets (kept zero between calls).
+// Per-device scratch: activation chunks, K-split partials, tickets (zeroed by the prep kernel of a call that splits K).
 static GrowScratch g_tc_scratch;
 // The block of the tensor-core kernels (gemm_w4a8_wide.cu works in it too): arrival counters first.
 cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p) { return g_tc_scratch.get(bytes, (size_t)16 << 20, st, p); }
@@ -598,9 +599,8 @@ static TcLayout tc_layout(int M, int N, int K) {
     l.ksplit = ksplit;
     const size_t xb_bytes = (size_t)l.nchunks * xb_chunk_bytes(l.Mpad);
     l.part_bytes = ksplit > 1 ? (size_t)l.tiles * ksplit * l.Mpad * kRows * sizeof(float) : 0;
-    // The arrival counters own a region of fixed size at the front of the block: they must read zero at the start of
-    // every call, and a region sized by the problem would let one call's activations lie where a later, larger call
-    // expects its counters.
+    // The arrival counters own a region of fixed size at the front of the block, which no call's activations or partial
+    // tiles share.
     if ((size_t)l.tiles * sizeof(unsigned int) > kTicketBytes) { l.ksplit = 1; l.part_bytes = 0; }
     l.xb_off = kTicketBytes;
     l.part_off = (l.xb_off + xb_bytes + 255) & ~(size_t)255;
@@ -637,7 +637,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
 
     const dim3 pgrid((nchunks * kBlocksPerChunk + 255) / 256, Mpad);
-    prep_x_kernel<<<pgrid, 256, 0, st>>>(scratch + xb_off, a, M, Mpad, nchunks);
+    prep_x_kernel<<<pgrid, 256, 0, st>>>(scratch + xb_off, a, M, Mpad, nchunks, reinterpret_cast<unsigned int*>(scratch), ksplit > 1 ? tiles : 0);
     count_launch(1);
     e = cudaPeekAtLastError();
     if (e != cudaSuccess) return e;

@@ -64,7 +64,7 @@ struct TcArgs {
     const __half* Wsc;        // [N][nkb] weight scales
     int nkb;                  // K / 16
     float* partial;           // [tiles][ksplit][Mpad][128] when ksplit > 1
-    unsigned int* tickets;    // [tiles], zero before and after the call
+    unsigned int* tickets;    // [tiles], zero at the start (see the prep kernel)
     int* status;              // device status word
     int N, M, Mpad;           // Mpad = MMA N in {16, 32, 64}
     int nchunks;              // ceil(K / 256)

@@ -26,13 +26,15 @@ namespace wide {
 //   chunk c: [block 0..15][k half][NP rows x 16 B: eight bf16]   then   [block 0..15][NP] fp32 scales
 // The eight elements of a half are in the order in which the unpack takes the nibbles of a word: 0 4 1 5 2 6 3 7.
 // k-blocks >= K/16 of the last chunk are zero (their weights multiply as zero too); rows >= M are left as they are: an
-// accumulator column is one sequence.  Grid (ceil(chunks / 8), M), 256 threads of eight elements; starts early under
-// programmatic dependent launch.
+// accumulator column is one sequence.  Zeroes the arrival counters of equal shares (`ncounters`, or 0).  Grid (ceil(chunks / 8), M),
+// 256 threads of eight elements; starts early under programmatic dependent launch.
 // ----------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int NP, int nchunks) {
+__global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int NP, int nchunks,
+                                                     unsigned int* counters, int ncounters) {
     __shared__ float part[8];
     pdl_trigger();
     pdl_wait();   // the activations come from the kernel before
+    zero_counters(counters, ncounters);
     const int m = blockIdx.y, t = threadIdx.x;
     const float rstd = a.xkind == kXFloatNorm ? row_rstd(a, m, t, part) : 1.f;
     const int e0 = (blockIdx.x * 256 + t) * 8;
@@ -379,7 +381,6 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
                             if (row0 < a.N) store(cg * CW + j, row0, acc[0][j]);
                             if (row0 + 128 < a.N) store(cg * CW + j, row0 + 128, acc[1][j]);
                         }
-                    if (wt == 0) a.tickets[tile] = 0;
                 }
                 if (!team_sync()) return false;   // `last` is written again
             }
@@ -580,9 +581,7 @@ static WideLayout layout_of(int M, int N, int K) {
     if (force > 8) l.csize = 1;
     else if (force > 1 && force <= l.nchunks) l.csize = force;
     else if (force == 1) l.csize = 0;
-    // The arrival counters own a region of fixed size at the front of the block: they must read zero at the start of
-    // every call, and a region sized by the problem would let one call's activations lie where a later, larger call
-    // expects its counters.  Matrices with more tiles than counters are dealt out by whole tiles.
+    // The arrival counters own a region of fixed size at the front of the block.  Matrices with more tiles than counters are dealt out by whole tiles.
     if (l.csize == 1 && (size_t)l.tiles * sizeof(unsigned int) > tc::kTicketBytes) l.csize = 0;
     if (l.csize == 0) l.grid = l.tiles < sms ? l.tiles : sms;
     if (l.csize > 1) l.grid = l.tiles * l.csize;
@@ -669,7 +668,8 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
 
-    e = launch_pdl(prep_x_kernel, dim3((lay.nchunks + 7) / 8, M), dim3(256), 0, st, scratch + lay.xb_off, a, lay.NE, lay.nchunks);
+    e = launch_pdl(prep_x_kernel, dim3((lay.nchunks + 7) / 8, M), dim3(256), 0, st, scratch + lay.xb_off, a, lay.NE, lay.nchunks,
+                   reinterpret_cast<unsigned int*>(scratch), lay.csize == 1 ? lay.tiles : 0);
     count_launch(1);
     if (e != cudaSuccess) return e;
 

@@ -69,7 +69,7 @@ struct WideArgs {
     int nkb;                  // K / 16
     int sc_gran;              // largest of 16, 8, 4 bytes that divides scale base and row pitch
     float* partial;           // [CTA][2][sequences][256] partial tiles of K ranges that begin or end inside a tile
-    unsigned int* tickets;    // [tiles], zero before and after the call
+    unsigned int* tickets;    // [tiles], zero at the start (see the prep kernel)
     int* status;              // device status word
     int N, M;
     int nchunks;              // ceil(K / 256)

@@ -114,3 +114,40 @@ def test_prologues_strides_and_residual(k):
     xq, xs = oracle.quantize_int8(x16.astype(np.float32))
     assert max_abs_rel(y2.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
     assert k.device_status() == 0
+
+
+# (form, key 6): equal shares of the bf16 form, K split of the int8 form
+@pytest.mark.parametrize("form,split", [(1, 9), (-1, 5)])
+def test_counters_of_a_call_that_gave_up_do_not_reach_the_next(k, form, split):
+    """A product that gives up in a wait leaves tiles half counted in the block that both forms share."""
+    import ctypes as C
+
+    import torch
+
+    from blackwell_b200 import _lib
+
+    M, K, N = 40, 4096, 700
+    W, sc16, _ = synth.int4_weights(N, K, seed=91)
+    xq, xs = oracle.quantize_int8(synth.activations_f16(M, K, 92).astype(np.float32))
+    args = [to_dev(xq), to_dev(xs), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    block = C.c_void_p()
+    L = _lib.load()
+    assert L["_ZN2bw2tc7scratchEmP11CUstream_stPPh"](C.c_size_t(1), None, C.byref(block)) == 0
+    k.set_tuning(24, form)
+    k.set_tuning(6, split)
+    try:
+        k.gemv_w4a8(y, *args)
+        torch.cuda.synchronize()
+        half = type("_View", (), {"__cuda_array_interface__": {"shape": (16384,), "typestr": "<i4", "data": (block.value, False), "version": 2}})()
+        torch.as_tensor(half, device="cuda").fill_(1)
+        want = y.clone()
+        y.fill_(float("nan"))
+        k.gemv_w4a8(y, *args)
+        torch.cuda.synchronize()
+    finally:
+        k.set_tuning(6, 0)
+        k.set_tuning(24, 1)
+    assert k.device_status() == 0
+    assert torch.equal(y, want)
+    assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
