@@ -524,14 +524,11 @@ static EncodeTiledFn encode_fn() {
 
 // Per-device scratch: activation chunks, K-split partials, tickets (zeroed by the prep kernel of a call that splits K).
 static GrowScratch g_tc_scratch;
-// The block of the tensor-core kernels (gemm_w4a8_wide.cu works in it too): arrival counters first.
 cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p) { return g_tc_scratch.get(bytes, (size_t)16 << 20, st, p); }
 cudaError_t reserve_scratch(size_t bytes) {
     unsigned char* p = nullptr;
     return bytes ? g_tc_scratch.get(bytes, (size_t)16 << 20, nullptr, &p) : cudaSuccess;
 }
-
-constexpr size_t kTicketBytes = 65536;  // arrival counters: 16,384 row tiles; larger matrices are not K-split
 
 // Quantizes the activations of a streaming-kernel call once (see prep_plain_kernel) into the scratch block and returns
 // the pre-quantized operand.  Calls that go on to the tensor-core kernel do not use this (its own prep writes the same

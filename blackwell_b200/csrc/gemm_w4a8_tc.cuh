@@ -56,6 +56,11 @@ constexpr int kAStageBytes = kBlocksPerChunk * kABlockStride;    // 33024
 constexpr int kEpiWarps = 8;     // epilogue warps: two per TMEM lane quarter, each half of the sequences
 constexpr int kThreads = (4 + kEpiWarps + 4) * 32;   // + producer, MMA issuer, two scale-loader and four unpack warps
 
+// The scratch block in which both tcgen05 forms work (this one and gemm_w4a8_wide.cu): arrival counters of 16,384 row tiles first
+// (larger matrices are not split inside a tile), then what a call lays out.
+constexpr size_t kTicketBytes = 65536;
+cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p);
+
 struct TcArgs {
     float* y;                 // [M][y_stride]
     const float* residual;    // optional, same layout as y

@@ -14,10 +14,6 @@
 #include "tensor_map.h"
 
 namespace bw {
-namespace tc {  // gemm_w4a8_tc.cu
-constexpr size_t kTicketBytes = 65536;
-cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p);
-}  // namespace tc
 namespace wide {
 
 // ----------------------------------------------------------------------------------------------------------
