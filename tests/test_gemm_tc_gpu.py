@@ -12,13 +12,15 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def k(cuda):
-    """The kernels with the mma.sync kernel switched off, so that every batch from 8 sequences up takes the tcgen05
-    kernel as it does by default above 16."""
+    """The kernels with the mma.sync kernel and the bf16 tcgen05 form switched off, so that every batch from 8 sequences up takes
+    the int8 form."""
     from blackwell_b200 import kernels
 
     kernels.set_tuning(13, 99)
+    kernels.set_tuning(24, -1)
     yield kernels
     kernels.set_tuning(13, 0)
+    kernels.set_tuning(24, 0)
 
 
 CASES = [(16, 256, 128), (9, 4096, 128), (16, 4096, 300), (17, 512, 129), (32, 4096, 1024), (33, 2048, 640),

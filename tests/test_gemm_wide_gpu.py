@@ -48,12 +48,13 @@ def test_matches_the_oracle(k, M, K, N, split):
     assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
 
 
-def test_scales_of_every_kind_are_split_without_rounding(k):
+@pytest.mark.parametrize("M", [32, 48, 64])
+def test_scales_of_every_kind_are_split_without_rounding(k, M):
     """Subnormal, negative, largest and full-mantissa binary16 scales: one k-block per output and an activation scale of 1, so
     that the output is w_sc * dot, at most 25 bits, to one rounding."""
     import torch
 
-    M, K, N = 32, 32, 4096
+    K, N = 32, 4096
     r = synth.rng(77)
     bits = r.integers(0, 1 << 16, size=(N, 2), dtype=np.uint16)
     bits[(bits & 0x7C00) == 0x7C00] ^= 0x4000            # no infinities or NaN
@@ -114,6 +115,27 @@ def test_prologues_strides_and_residual(k):
     xq, xs = oracle.quantize_int8(x16.astype(np.float32))
     assert max_abs_rel(y2.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
     assert k.device_status() == 0
+
+
+def test_both_forms_in_turn_on_the_block_they_share(k):
+    """K split of the int8 form (-1) and equal shares of the bf16 form (1), with few tiles and with many."""
+    import torch
+
+    K = 2048
+    try:
+        for form, M, N in [(-1, 32, 256), (1, 48, 9000), (-1, 64, 384), (1, 17, 12800), (-1, 64, 1100), (1, 64, 700), (-1, 20, 130)]:
+            W, sc16, _ = synth.int4_weights(N, K, seed=N)
+            xq, xs = oracle.quantize_int8(synth.activations_f16(M, K, N + 1).astype(np.float32))
+            y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+            k.set_tuning(24, form)
+            k.set_tuning(6, 9 if form > 0 else 0)
+            k.gemv_w4a8(y, to_dev(xq), to_dev(xs), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M)
+            torch.cuda.synchronize()
+            assert k.device_status() == 0
+            assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5, (form, M, N)
+    finally:
+        k.set_tuning(6, 0)
+        k.set_tuning(24, 1)
 
 
 # (form, key 6): equal shares of the bf16 form, K split of the int8 form
