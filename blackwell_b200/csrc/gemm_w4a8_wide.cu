@@ -523,6 +523,24 @@ void set_split(int v) { g_split = v; }
 // Sequences an instantiation handles: those of M rounded up.
 static int cols_of(int M) { return M <= 32 ? 32 : M <= 48 ? 48 : 64; }
 
+// Makes an instance launchable on the current device, once.  The roles' register shares are drawn from what the launch allocates.
+template <int NE>
+static cudaError_t prepare() {
+    static std::once_flag once[kMaxDevices];
+    static cudaError_t usable[kMaxDevices];
+    const int dev = current_device();
+    std::call_once(once[dev], [&] {
+        cudaFuncAttributes fa;
+        cudaError_t e = cudaFuncSetAttribute(gemm_w4a8_wide_kernel<NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<NE>::kSmem);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, gemm_w4a8_wide_kernel<NE>);
+        if (e == cudaSuccess && fa.numRegs < 96) e = cudaErrorInvalidConfiguration;
+        if (e != cudaSuccess) cudaGetLastError();
+        usable[dev] = e;
+    });
+    return usable[dev];
+}
+static bool usable(int NE) { return (NE == 32 ? prepare<32>() : NE == 48 ? prepare<48>() : prepare<64>()) == cudaSuccess; }
+
 // Clusters of `csize` CTAs that are resident at once on the current device, at most (the SMs of a cluster share a GPC).
 static int max_clusters(int csize) {
     static std::atomic<int> cached[kMaxDevices][9];
@@ -539,8 +557,7 @@ static int max_clusters(int csize) {
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(gemm_w4a8_wide_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<64>::kSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_w4a8_wide_kernel<64>, &cfg) != cudaSuccess || n < 1) {
+    if (prepare<64>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_w4a8_wide_kernel<64>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
         n = 1;
     }
@@ -594,7 +611,7 @@ void set_force(int v) { g_force = v; }
 // 26 / 30 at 32 sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 73 / 114, 103 / 115; 3072 x 2048 11 / 26,
 // 13 / 42, 16 / 42; the other way round 4096 x 10944 42 / 40 at 32, 68 / 59 at 64, 151643 x 4096 331 / 327, 530 / 480.
 bool preferred(int M, int N, int K) {
-    if (M <= 16) return false;
+    if (M <= 16 || !usable(cols_of(M))) return false;   // the int8 form takes the same operands
     if (g_force.load() != 0) return g_force.load() > 0;
     const int sms = sm_count(current_device()), tiles = (N + 127) / 128, nchunks = (K + kKc - 1) / kKc;
     const int ks = std::max(1, std::min(sms / tiles, nchunks));
@@ -617,17 +634,8 @@ size_t scratch_bytes(int M, int N, int K) {
 template <int NE>
 static cudaError_t launch_n(const CUtensorMap& map_w, const WideArgs& t, int grid, cudaStream_t st) {
     auto kern = gemm_w4a8_wide_kernel<NE>;
-    static std::once_flag once[kMaxDevices];
-    const int dev = current_device();
-    static cudaError_t usable[kMaxDevices];
-    std::call_once(once[dev], [&] {
-        usable[dev] = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<NE>::kSmem);
-        cudaFuncAttributes fa;
-        if (usable[dev] == cudaSuccess) usable[dev] = cudaFuncGetAttributes(&fa, kern);
-        // the roles' register shares are drawn from what the launch allocates
-        if (usable[dev] == cudaSuccess && fa.numRegs < 96) usable[dev] = cudaErrorInvalidConfiguration;
-    });
-    if (usable[dev] != cudaSuccess) return usable[dev];
+    const cudaError_t e0 = prepare<NE>();
+    if (e0 != cudaSuccess) return e0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreads);

@@ -2,6 +2,7 @@
 declares and the reference's C++ symbols for the decode path, and the
 reference's own consumers link against it unchanged (where their sources are
 present)."""
+import ctypes as C
 import os
 import re
 import shutil
@@ -61,6 +62,17 @@ def test_argument_checks_need_no_gpu(so_path):
     assert lib.bw_quantize_int8(None, None, None, 15, None) == 1
     assert lib.bw_gemv_w4a8(None, None, None, None, None, 4096, 16, 0, None) == 1
     assert lib.bw_set_tuning(99, 0) == 1
+
+
+def test_a_product_form_that_cannot_run_is_not_chosen(so_path):
+    """Where the bf16 tcgen05 form cannot be launched (here: no device) the routing leaves its calls to the int8 form."""
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("this machine can run it")
+    preferred = _lib.load()["_ZN2bw4wide9preferredEiii"]
+    preferred.restype = C.c_bool
+    assert not preferred(32, 21888, 4096)
 
 
 def test_cxx_dropin_symbols_exported(so_path):
