@@ -160,11 +160,11 @@ __global__ void __launch_bounds__(256) argmax_batched_kernel(const float* logits
     // rows of 151,643 under ncu).  Indices rise within a thread, so a strict comparison keeps the lowest of equal values.
     unsigned int key = fkey(-1e38f);
     int at = 0;
-    const int step = gridDim.x * blockDim.x;
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < vocab; i0 += 8 * step) {
+    const unsigned int step = gridDim.x * blockDim.x, n = vocab;   // unsigned: the last indices may pass 2^31
+    for (unsigned int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 8 * step) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = i0 + (long)j * step < vocab ? row[i0 + (long)j * step] : -INFINITY;
+        for (int j = 0; j < 8; ++j) v[j] = i0 + j * step < n ? row[i0 + j * step] : -INFINITY;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const unsigned int k = fkey(v[j]);

@@ -232,6 +232,21 @@ def test_fused_norm_rope_kv_attention_equals_the_two_launches(cuda, nq, nkv):
     assert k.device_status() == 0
 
 
+def test_argmax_of_a_row_that_ends_just_below_2_to_the_31(cuda):
+    """The last round of eight loads per thread passes 2^31."""
+    import torch
+    from blackwell_b200 import kernels as k
+
+    V = 2 ** 31 - 40000
+    if torch.cuda.mem_get_info()[0] < 4 * V + (1 << 30):
+        pytest.skip("needs 9 GB")
+    logits = torch.zeros(V, dtype=torch.float32, device="cuda")
+    logits[V - 1] = 1.0
+    ids = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    k.sample_argmax_batched(logits, V, V, 1, ids)
+    assert int(ids.cpu()[0]) == V - 1
+
+
 def test_tensor_parallel_argmax_candidates_and_merge(cuda):
     """The vocabulary cut into three ranks' slices: per-slice candidates + merge give the ids of the full argmax
     (ties to the lowest global index) and advance the positions once."""
