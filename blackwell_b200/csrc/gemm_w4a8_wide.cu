@@ -607,7 +607,10 @@ static std::atomic<int> g_force{0};
 void set_force(int v) { g_force = v; }
 // Whether a call of 17 to 64 sequences is faster here than in the int8 form (gemm_w4a8_tc.cu), by the estimates of both.  That
 // one takes 2.27 us for a chunk of 128 rows up to 32 sequences and 3.33 above (it computes 64 columns then), its tiles come in
-// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  Measured, this form / that one: 6144 x 4096
+// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  And whether no sum is a longer chain of chunks than there: a
+// narrow matrix of very long rows is split finer by the int8 form (300 x 32768, 64 chunks: 4 against 16 in a cluster of eight), and
+// its error against 64 bits was 1.8e-7 where this form had 2.9e-7; where the chains here are no longer it is 0.6 to 1.01 of that
+// form's (2048 to 21888 rows of 2048 to 12288, 17 to 64 sequences).  Measured, this form / that one: 6144 x 4096
 // 26 / 30 at 32 sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 73 / 114, 103 / 115; 3072 x 2048 11 / 26,
 // 13 / 42, 16 / 42; the other way round 4096 x 10944 42 / 40 at 32, 68 / 59 at 64, 151643 x 4096 331 / 327, 530 / 480.
 bool preferred(int M, int N, int K) {
@@ -618,7 +621,10 @@ bool preferred(int M, int N, int K) {
     const int boxes = ((nchunks + 1) / 2 + ks - 1) / ks, rounds = (tiles * ks + sms - 1) / sms;
     const float chunks = (float)(std::min(2 * boxes, nchunks) * rounds);
     const float us = M <= 32 ? 2.27f * chunks + (ks > 1 ? 8.f + 2.2f * ks : 6.f) : 3.33f * chunks + (ks > 1 ? 10.f + 3.6f * ks : 6.f);
-    return layout_of(M, N, K).us < us;
+    const WideLayout l = layout_of(M, N, K);
+    const int share = (int)(((long long)l.tiles * l.nchunks + l.grid - 1) / l.grid);
+    const int chain = l.csize == 0 ? nchunks : std::min(share, nchunks);
+    return l.us < us && chain <= std::min(2 * boxes, nchunks);
 }
 // Enough for every batch up to M.
 size_t scratch_bytes(int M, int N, int K) {

@@ -138,6 +138,25 @@ def test_both_forms_in_turn_on_the_block_they_share(k):
         k.set_tuning(24, 1)
 
 
+def test_a_form_with_longer_chains_of_sums_is_not_chosen(k):
+    """A narrow matrix of long rows, which the int8 form splits finer."""
+    import torch
+
+    M, K, N = 32, 32768, 300
+    W, sc16, _ = synth.int4_weights(N, K, seed=93)
+    xq, xs = oracle.quantize_int8(synth.activations_f16(M, K, 94).astype(np.float32))
+    args = [to_dev(xq), to_dev(xs), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
+    out = []
+    try:
+        for form in (-1, 0):
+            k.set_tuning(24, form)
+            out.append(torch.empty((M, N), dtype=torch.float32, device="cuda"))
+            k.gemv_w4a8(out[-1], *args)
+    finally:
+        k.set_tuning(24, 1)
+    assert torch.equal(*out)
+
+
 # (form, key 6): equal shares of the bf16 form, K split of the int8 form
 @pytest.mark.parametrize("form,split", [(1, 9), (-1, 5)])
 def test_counters_of_a_call_that_gave_up_do_not_reach_the_next(k, form, split):
