@@ -488,12 +488,9 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
                     const int m = i / nr, r = r0 + i - m * nr, n = tile * kRows + r;
                     float p[8];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        if (c < a.csize) p[c] = ld_dsmem(base + (m * kRows + r) * 4, c);
-                    float sum = p[0];
-#pragma unroll
-                    for (int c = 1; c < 8; ++c)
-                        if (c < a.csize) sum += p[c];
+                    for (int c = 0; c < 8; ++c) p[c] = c < a.csize ? ld_dsmem(base + (m * kRows + r) * 4, c) : 0.f;
+                    // neighbours first: eight sums in a row had 2 % more error (2048 x 5632, against 64 bits)
+                    const float sum = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
                     if (n < a.N) store(m, n, sum);
                 }
             __syncwarp();
@@ -573,7 +570,8 @@ struct WideLayout {
 };
 // Equal shares of all chunks, or a cluster per tile: whichever the estimate says.  Measured (us, prep included; 4096 x 4096,
 // 6144 x 4096, 21888 x 4096, 4096 x 10944): a chunk of a tile takes 5.1 / 5.9 / 8.2 at 32 / 48 / 64 sequences; a cluster adds 6
-// to its longest share, equal shares add 10 and about 0.9 (at 32) for every share that the last CTA of a tile adds up.
+// to its longest share, equal shares add 10 and about 0.9 (at 32) for every share that the last CTA of a tile adds up.  Clusters of
+// 2 to 8 resident at once on a B200: 74, 45, 33, 26, 22, 15, 15.
 static WideLayout layout_of(int M, int N, int K) {
     WideLayout l;
     l.NE = cols_of(M);
@@ -607,12 +605,13 @@ static std::atomic<int> g_force{0};
 void set_force(int v) { g_force = v; }
 // Whether a call of 17 to 64 sequences is faster here than in the int8 form (gemm_w4a8_tc.cu), by the estimates of both.  That
 // one takes 2.27 us for a chunk of 128 rows up to 32 sequences and 3.33 above (it computes 64 columns then), its tiles come in
-// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  And whether no sum is a longer chain of chunks than there: a
+// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  And whether every sum is a shorter chain of chunks than there (or neither splits K): a
 // narrow matrix of very long rows is split finer by the int8 form (300 x 32768, 64 chunks: 4 against 16 in a cluster of eight), and
-// its error against 64 bits was 1.8e-7 where this form had 2.9e-7; where the chains here are no longer it is 0.6 to 1.01 of that
-// form's (2048 to 21888 rows of 2048 to 12288, 17 to 64 sequences).  Measured, this form / that one: 6144 x 4096
-// 26 / 30 at 32 sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 73 / 114, 103 / 115; 3072 x 2048 11 / 26,
-// 13 / 42, 16 / 42; the other way round 4096 x 10944 42 / 40 at 32, 68 / 59 at 64, 151643 x 4096 331 / 327, 530 / 480.
+// its error against 64 bits was 1.8e-7 where this form had 2.9e-7; where the chains here are shorter it is 0.6 to 0.99 of that
+// form's (2048 to 24576 rows of 2048 to 12288, 17 to 64 sequences; 1.02 at most over 60 random sizes, 1.15 where they are equal).  Measured, this form / that one: 6144 x 4096
+// 26 / 31 at 32 sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 72 / 115, 95 / 115; 3072 x 2048 11 / 26, 13 / 42,
+// 16 / 42; 4096 x 10944 42 / 41, 48 / 58, 65 / 59; 4096 x 12288 46 / 42, 54 / 60, 72 / 60; 32768 x 2048 47 / 45, 55 / 64, 71 / 64;
+// 151643 x 4096 327 / 329, 383 / 480, 526 / 482: the rule takes the faster one in each but the last at 32, where they are level.
 bool preferred(int M, int N, int K) {
     if (M <= 16 || !usable(cols_of(M))) return false;   // the int8 form takes the same operands
     if (g_force.load() != 0) return g_force.load() > 0;
@@ -624,7 +623,8 @@ bool preferred(int M, int N, int K) {
     const WideLayout l = layout_of(M, N, K);
     const int share = (int)(((long long)l.tiles * l.nchunks + l.grid - 1) / l.grid);
     const int chain = l.csize == 0 ? nchunks : std::min(share, nchunks);
-    return l.us < us && chain <= std::min(2 * boxes, nchunks);
+    const int theirs = std::min(2 * boxes, nchunks);
+    return l.us < us && (chain < theirs || theirs == nchunks);
 }
 // Enough for every batch up to M.
 size_t scratch_bytes(int M, int N, int K) {

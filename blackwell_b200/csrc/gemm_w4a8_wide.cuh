@@ -26,8 +26,9 @@
 // A pair is the blocks (p, p + 8) of a chunk, so that a thread's eight blocks are consecutive: its scales are 16 bytes, its
 // nibbles come two blocks per 16-byte load.  Scalar FMAs, not packed ones: the packed form goes to half of the FMA pipe, which
 // the bf16 FMAs of the unpack already fill (708 against 517 us, same case).
-// What bounds it (75,776 x 4096, 48 / 64 sequences): issue slots 68 % busy with five warps per scheduler, then the latency chain
-// of a worker's step; HBM 12 / 9 %.
+// What bounds it (75,776 x 4096, 32 / 48 / 64 sequences): issue slots 63 / 68 / 68 % busy with five warps per scheduler, then the
+// latency chain of a worker's step; HBM 15 / 13 / 10 %, tensor pipe 11 / 14 / 14 % active.  Spilled by ptxas at 32 / 48 columns:
+// 12 / 56 bytes stored, 56 loaded; none at 64.
 // All waits are bounded; a wait that gives up raises an abort flag.
 #pragma once
 #include <cuda_bf16.h>
