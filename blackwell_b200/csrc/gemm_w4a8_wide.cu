@@ -605,13 +605,14 @@ static std::atomic<int> g_force{0};
 void set_force(int v) { g_force = v; }
 // Whether a call of 17 to 64 sequences is faster here than in the int8 form (gemm_w4a8_tc.cu), by the estimates of both.  That
 // one takes 2.27 us for a chunk of 128 rows up to 32 sequences and 3.33 above (it computes 64 columns then), its tiles come in
-// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  And whether every sum is a shorter chain of chunks than there (or neither splits K): a
-// narrow matrix of very long rows is split finer by the int8 form (300 x 32768, 64 chunks: 4 against 16 in a cluster of eight), and
-// its error against 64 bits was 1.8e-7 where this form had 2.9e-7; where the chains here are shorter it is 0.6 to 0.99 of that
-// form's (2048 to 24576 rows of 2048 to 12288, 17 to 64 sequences; 1.02 at most over 60 random sizes, 1.15 where they are equal).  Measured, this form / that one: 6144 x 4096
-// 26 / 31 at 32 sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 72 / 115, 95 / 115; 3072 x 2048 11 / 26, 13 / 42,
-// 16 / 42; 4096 x 10944 42 / 41, 48 / 58, 65 / 59; 4096 x 12288 46 / 42, 54 / 60, 72 / 60; 32768 x 2048 47 / 45, 55 / 64, 71 / 64;
+// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  Measured, this form / that one: 6144 x 4096 26 / 31 at 32
+// sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 72 / 115, 95 / 115; 3072 x 2048 11 / 26, 13 / 42, 16 / 42;
+// 4096 x 10944 42 / 41, 48 / 58, 65 / 59; 4096 x 12288 46 / 42, 54 / 60, 72 / 60; 32768 x 2048 47 / 45, 55 / 64, 71 / 64;
 // 151643 x 4096 327 / 329, 383 / 480, 526 / 482: the rule takes the faster one in each but the last at 32, where they are level.
+// And whether every sum is a shorter chain of chunks than there, or neither splits K: a narrow matrix of very long rows is split
+// finer by the int8 form (300 x 32768, 64 chunks: 4 against 16 in a cluster of eight), and its error against 64 bits was 1.8e-7
+// where this form had 2.9e-7.  With the shorter chains here it is 0.6 to 0.99 of that form's (2048 to 24576 rows of 2048 to 12288,
+// 17 to 64 sequences; 1.02 at most over 60 random sizes, 1.15 where the chains were equal).
 bool preferred(int M, int N, int K) {
     if (M <= 16 || !usable(cols_of(M))) return false;   // the int8 form takes the same operands
     if (g_force.load() != 0) return g_force.load() > 0;
