@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <mutex>
 
@@ -18,12 +19,13 @@ namespace wide {
 
 // ----------------------------------------------------------------------------------------------------------
 // Activation prep of the tensor-core kernel: quantizes every sequence once (int8 rule; plain / RMSNorm / SwiGLU, or int8 as
-// it comes) and stores it in the layout of the MMA's B operand, chunk by chunk:
-//   chunk c: [block 0..15][k half][NP rows x 16 B: eight bf16]   then   [block 0..15][NP] fp32 scales
-// The eight elements of a half are in the order in which the unpack takes the nibbles of a word: 0 4 1 5 2 6 3 7.
-// k-blocks >= K/16 of the last chunk are zero (their weights multiply as zero too); rows >= M are left as they are: an
-// accumulator column is one sequence.  Zeroes the arrival counters of equal shares (`ncounters`, or 0).  Grid (ceil(chunks / 8), M),
-// 256 threads of eight elements; starts early under programmatic dependent launch.
+// it comes) and stores x = xq x_sc as three bf16 parts in units of u (gemm_w4a8_wide.cuh) in the layout of the MMA's B operand:
+//   chunk c: [half 0..1][block 0..7][k half][x1, x2, x3][NP rows x 16 B: eight bf16]   then   [NP] units u
+// Half h holds the chunk's blocks whose index has bit 2 equal to h, in order.  The eight elements of a k half are in the order in
+// which the unpack takes the nibbles of a word: 0 4 1 5 2 6 3 7.  k-blocks >= K/16 of the last chunk are zero (their weights
+// multiply as zero too); rows >= M are left as they are: an accumulator column is one sequence.  An infinite or NaN scale makes its
+// sequence's results non-finite.  Zeroes the arrival counters of equal shares (`ncounters`, or 0).  Grid (ceil(chunks / 8), M), 256
+// threads of eight elements, a warp per chunk; starts early under programmatic dependent launch.
 // ----------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int NP, int nchunks,
                                                      unsigned int* counters, int ncounters) {
@@ -31,7 +33,7 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
     pdl_trigger();
     pdl_wait();   // the activations come from the kernel before
     zero_counters(counters, ncounters);
-    const int m = blockIdx.y, t = threadIdx.x;
+    const int m = blockIdx.y, t = threadIdx.x, lane = t & 31;
     const float rstd = a.xkind == kXFloatNorm ? row_rstd(a, m, t, part) : 1.f;
     const int e0 = (blockIdx.x * 256 + t) * 8;
     const bool valid = e0 < a.K;   // K % 16 == 0: the two threads of a block are valid or not together
@@ -42,7 +44,7 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
             const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const int8_t*>(a.x) + (size_t)m * a.K + e0));
 #pragma unroll
             for (int i = 0; i < 8; ++i) q[i] = (i < 4 ? u.x : u.y) >> (8 * (i & 3));
-            if ((t & 1) == 0) sc = __ldg(a.xsc + (size_t)m * (a.K / 16) + (e0 >> 4));
+            sc = __ldg(a.xsc + (size_t)m * (a.K / 16) + (e0 >> 4));
         }
     } else {
         float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -56,17 +58,45 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
             round_elements<8>(v, am, sc, q);
         }
     }
-    const int kb = e0 >> 4, c = kb / kBlocksPerChunk, b = kb % kBlocksPerChunk;
+    // u = 2^e with e the exponent of the chunk's largest |x| / 128 (so |x| < 256 u), within what has a normal reciprocal or 2^-127
+    float f[8], big = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        f[i] = (float)(int8_t)q[i];
+        big = fmaxf(big, fabsf(f[i]));
+    }
+    if (big == 0.f && fabsf(sc) < INFINITY) sc = 0.f;   // (0 times a scale far above the chunk's)
+    float top = big * (fabsf(sc) * 0.0078125f);
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, i));
+    const uint32_t eb = min(max(__float_as_uint(top) & 0x7F800000u, 0x00800000u), 0x7F000000u);
+    const float rs = sc * __uint_as_float(eb == 0x7F000000u ? 0x00400000u : 0x7F000000u - eb);   // x_sc / u: exact
+    const int c = e0 / kKc, b = (e0 >> 4) % kBlocksPerChunk;
     if (c >= nchunks) return;
-    uint32_t o[4];
+    uint32_t o[3][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn((float)(int8_t)q[i], (float)(int8_t)q[i + 4]);
-        o[i] = *reinterpret_cast<const uint32_t*>(&p);
+        float p[3][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float v = f[i + 4 * j];
+            p[0][j] = rintf(v * rs);
+            const float r = fmaf(v, rs, -p[0][j]);   // exact: the product's upper bits are gone
+            p[1][j] = __bfloat162float(__float2bfloat16_rn(r));
+            p[2][j] = r - p[1][j];
+        }
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(p[n][0], p[n][1]);
+            o[n][i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
     }
     unsigned char* chunk = xb + (size_t)c * xchunk_bytes(NP);
-    *reinterpret_cast<uint4*>(chunk + ((size_t)(2 * b + (t & 1)) * NP + m) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-    if ((t & 1) == 0) reinterpret_cast<float*>(chunk + xop_bytes(NP))[b * NP + m] = sc;
+    const int half = (b >> 2) & 1, at = (b >> 3) * 4 + (b & 3);
+    unsigned char* row = chunk + half * xhalf_bytes(NP) + ((size_t)(2 * at + (t & 1)) * 3 * NP + m) * 16;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) *reinterpret_cast<uint4*>(row + n * NP * 16) = make_uint4(o[n][0], o[n][1], o[n][2], o[n][3]);
+    if (lane == 0) reinterpret_cast<float*>(chunk + 2 * xhalf_bytes(NP))[m] = __uint_as_float(eb) * 0.125f;   // the operand A is eight times the weights
 }
 
 // ----------------------------------------------------------------------------------------------------------
@@ -74,36 +104,40 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
 // ----------------------------------------------------------------------------------------------------------
 template <int NE>
 struct WideShape {
-    static constexpr int NP = NE;                        // MMA N
-    static constexpr int CW = NE / 4;                    // sequences per worker thread, for each of its two rows
-    static constexpr bool kTight = NE > 48;              // two pairs of accumulators do not fit beside the A operand
-    static constexpr int DB = kTight ? 1 : 2;            // k-blocks per accumulator stage
-    static constexpr int DS = kTight ? 3 : 2;            // accumulator stages, of a pair or (kTight) of a block
-    static constexpr int kDCols = DB * 2 * NP;           // tensor-memory columns of a stage: [block][row group][NP]
-    static constexpr int kACol = DS * kDCols;            // first column of the two A slots: [row group][block of the pair][q sh, q sl][8]
-    static constexpr int BYTES = kWBytes + xchunk_bytes(NP);
-    static constexpr int S = (kMaxDynSmem - 2048) / BYTES < 5 ? (kMaxDynSmem - 2048) / BYTES : 5;
-    static constexpr int kSmem = 2048 + S * BYTES;       // up to 1023 bytes of alignment, 1 KB of barriers and flags
-    static_assert(BYTES % 1024 == 0 && kACol + 2 * 64 <= 512 && S >= 2, "shape");
-    static_assert(NE * kRows * 4 <= S * BYTES, "the tile for the cluster reduction takes the place of the operand ring");
+    static constexpr int NP = NE;                        // columns of an MMA
+    static constexpr int CW = NE / 2;                    // sequences per worker thread
+    static constexpr int LD = NE == 32 ? 16 : 8;         // of them read from tensor memory together
+    static constexpr bool kTwice = NE <= 32;             // two sets of accumulators
+    static constexpr int kDCols = 4 * NP;                // tensor memory: sets of [row group][sum of q sh x1, sum of the rest][NP], then
+    static constexpr int kACol = (kTwice ? 2 : 1) * kDCols;   // A: [row group][slot][half of its workers][two blocks][q sh, q sl][8]
+    // stages of weights (of a chunk) and of activations (of half a chunk): with few sequences the weights in flight matter, with many
+    // the tensor pipe takes its time over a chunk
+    static constexpr int SW = NE == 32 ? 3 : 2;
+    static constexpr int SX = NE == 64 ? 3 : 4;
+    static constexpr int kSmem = 1024 + 2048 + SW * kStageBytes + SX * xhalf_bytes(NP);   // alignment; barriers, flags, units; the rings
+    static_assert(kACol + 2 * kSlots * 64 <= 512 && kSmem <= kMaxDynSmem, "shape");
+    static_assert(NE * kRows * 4 <= SW * kStageBytes, "the tile for the cluster reduction takes the place of the weights");
+    static_assert(kScaleSlots * NP * 4 <= 1024 && SX <= 6, "units");   // see the activation producer
     // barriers
-    static constexpr int kFullW = 0;             // + stage: nibbles landed
-    static constexpr int kFullX = kFullW + S;    // + stage: activations and their scales landed
-    static constexpr int kEmpty = kFullX + S;    // + stage: used up by the workers (and so by the MMAs before them)
-    static constexpr int kFullA = kEmpty + S;    // + A slot: stored by the workers
-    static constexpr int kFullD = kFullA + 2;    // + accumulator stage: its MMAs have completed
-    static constexpr int kRead = kFullD + DS;    // kTight: the first block of a pair has been read
-    static constexpr int kTeam = kRead + 1;      // all workers together, at the end of a tile
+    static constexpr int kFullW = 0;             // + stage: nibbles and scales landed
+    static constexpr int kEmptyW = kFullW + SW;  // + stage: unpacked
+    static constexpr int kFullX = kEmptyW + SW;  // + stage: activations landed
+    static constexpr int kEmptyX = kFullX + SX;  // + stage: multiplied
+    static constexpr int kFullU = kEmptyX + SX;  // + slot: units of a chunk landed
+    static constexpr int kFullA = kFullU + kScaleSlots;   // + A slot: stored by the row group's workers, who have read what its unit will overwrite
+    static constexpr int kDone = kFullA + 2 * kSlots;     // + A slot: its MMAs have completed
+    static constexpr int kTeam = kDone + 2 * kSlots;      // all workers have left the ring, at the end of a cluster's tile
     static constexpr int kDrain = kTeam + 1;
-    static constexpr int kNumBars = kDrain + 1;
+    static constexpr int kNumBars = kDrain + 2;
     static_assert(kNumBars * 8 <= 512, "barriers");
 };
 
-// Place in a ring of three stages.
-struct Stage {
+// Place in a ring.
+template <int N>
+struct Ring {
     uint32_t at = 0, phase = 0;
     __device__ __forceinline__ void step() {
-        if (++at == 3) { at = 0; phase ^= 1; }
+        if (++at == N) { at = 0; phase ^= 1; }
     }
 };
 
@@ -128,38 +162,60 @@ __device__ __forceinline__ int chunk_owner(const WideArgs& a, int w, int grid) {
     return (int)((((long long)w + 1) * grid - 1) / all);
 }
 
+// The scales of chunk c of a tile's rows, B bytes a copy, by one warp: neighbouring lanes take neighbouring pieces of a row.  One
+// addition and one copy per 32 pieces: a loop with a product per row was the slowest part of the kernel (44 against 36 us, 16 tiles
+// of 16 chunks on a CTA each, 32 sequences).
+template <int B>
+__device__ __forceinline__ void copy_scales(const WideArgs& a, uint32_t to, int tile, int c, int lane) {
+    constexpr int kStep = B / 2, kPer = kBlocksPerChunk / kStep, kAtOnce = 32 / kPer;   // blocks a piece, pieces a row, rows at once
+    const int piece = lane % kPer, r0 = lane / kPer, at = c * kBlocksPerChunk + piece * kStep, row0 = tile * kRows + r0;
+    const uint32_t dst = to + (piece * kStep >> 3) * kRows * 16 + (piece * kStep & 7) * 2 + r0 * 16, src = at < a.nkb ? B : 0;
+    const char* p = reinterpret_cast<const char*>(a.Wsc + min(at, a.nkb - kStep));
+    const size_t pitch = (size_t)a.nkb * 2;
+    if (tile * kRows + kRows <= a.N) {
+        p += row0 * pitch;
+#pragma unroll
+        for (int i = 0; i < kRows / kAtOnce; ++i, p += kAtOnce * pitch) cp_async<B>(dst + i * kAtOnce * 16, p, src);
+    } else {   // the last tile: rows past the end take the last one's scales, nothing reads what comes of them
+#pragma unroll 1
+        for (int i = 0; i < kRows / kAtOnce; ++i) cp_async<B>(dst + i * kAtOnce * 16, p + min(row0 + i * kAtOnce, a.N - 1) * pitch, src);
+    }
+}
+
 template <int NE>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs a) {
     using Sh = WideShape<NE>;
-    constexpr int NP = Sh::NP, CW = Sh::CW, DB = Sh::DB, DS = Sh::DS, S = Sh::S;
-    constexpr bool kTight = Sh::kTight;
+    constexpr int NP = Sh::NP, CW = Sh::CW, SW = Sh::SW, SX = Sh::SX;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* ring = smem + 1024;
+    float* units = reinterpret_cast<float*>(smem + 1024);   // [slot][NP]
+    unsigned char* ring = smem + 2048;                      // nibbles and scales
+    unsigned char* xring = ring + SW * kStageBytes;         // activations
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(smem + 512);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 516);
-    volatile int* last = reinterpret_cast<volatile int*>(smem + 520);
     const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31;   // the warp index is uniform
     const uint32_t bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8 * i; };
-    auto wait = [&](int i, uint32_t parity) {   // by a whole warp (whose lanes see the same) or by one lane
-        if (mbar_wait_quick(bar(i), parity)) return true;
-        *abort_flag = 1;
-        return false;
-    };
+    const uint32_t flag = smem_u32(const_cast<int*>(abort_flag));
+    auto wait = [&](int i, uint32_t parity) { mbar_wait_or_abort(bar(i), parity, flag); };   // by a converged warp or by one lane
     if (t == 0) {
-        for (int i = 0; i < S; ++i) {
-            mbar_init(bar(Sh::kFullW + i), 1);
-            mbar_init(bar(Sh::kFullX + i), 1);
-            mbar_init(bar(Sh::kEmpty + i), kWorkers);
+        for (int i = 0; i < SW; ++i) {
+            mbar_init(bar(Sh::kFullW + i), 1 + 32);
+            mbar_init(bar(Sh::kEmptyW + i), kWorkers);
         }
-        for (int i = 0; i < 2; ++i) mbar_init(bar(Sh::kFullA + i), kWorkers);
-        for (int i = 0; i < DS; ++i) mbar_init(bar(Sh::kFullD + i), 1);
-        mbar_init(bar(Sh::kRead), kWorkers);
+        for (int i = 0; i < SX; ++i) {
+            mbar_init(bar(Sh::kFullX + i), 1);
+            mbar_init(bar(Sh::kEmptyX + i), 2);
+        }
+        for (int i = 0; i < kScaleSlots; ++i) mbar_init(bar(Sh::kFullU + i), 1);
+        for (int i = 0; i < 2 * kSlots; ++i) {
+            mbar_init(bar(Sh::kFullA + i), kWorkers / 2);
+            mbar_init(bar(Sh::kDone + i), 1);
+        }
         mbar_init(bar(Sh::kTeam), kWorkers);
-        mbar_init(bar(Sh::kDrain), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(bar(Sh::kDrain + i), 1);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -178,180 +234,149 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
     const int total = w1 - w0;
 
     if (warp < 4) regs_fewer<kRegsFew>();
-    if (warp == 0) {
-        if (lane == 0) {
-            // -------------------------------------------------------------------------------- producer
-            auto load_w = [&](int n) {
-                const int w = w0 + n, tile = w / a.nchunks, s = n % S;
+    if (warp == 3) {
+        // ------------------------------------------------------------------------------------ weights
+        // Nibbles by TMA, scales (32 bytes of a row and chunk, zeros past the end of the row) in the largest copies that the row pitch
+        // allows.  Loaded into registers by the workers a chunk ahead, the scales held up every wait for shared memory behind them (12 %
+        // of the time at 32 sequences, 19 % at 64).
+        bool waited = false;
+        int n = 0;
+        for (; n < total; ++n) {
+            const int w = w0 + n, tile = w / a.nchunks, c = w - tile * a.nchunks, s = n % SW;
+            if (n >= SW) {
+                if (!waited) pdl_wait();   // the weights do not depend on the kernel before; see the workers' first wait
+                waited = true;
+                wait(Sh::kEmptyW + s, ((n / SW) & 1) ^ 1);
+                if (*abort_flag) break;
+            }
+            const uint32_t stage = smem_u32(ring + s * kStageBytes);
+            if (lane == 0) {
                 mbar_expect_tx(bar(Sh::kFullW + s), kWBytes);
-                tma_load_2d(smem_u32(ring + s * Sh::BYTES), &map_w, (w - tile * a.nchunks) * (kKc / 2), tile * kRows, bar(Sh::kFullW + s));
-            };
-            const int ahead = min(total, S);
-            for (int n = 0; n < ahead; ++n) load_w(n);   // the weights do not depend on the kernel before
+                tma_load_2d(stage, &map_w, c * (kKc / 2), tile * kRows, bar(Sh::kFullW + s));
+            }
+            if (a.sc_gran == 16) copy_scales<16>(a, stage + kWBytes, tile, c, lane);
+            else if (a.sc_gran == 8) copy_scales<8>(a, stage + kWBytes, tile, c, lane);
+            else copy_scales<4>(a, stage + kWBytes, tile, c, lane);
+            tc::cp_async_arrive(bar(Sh::kFullW + s));
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (*abort_flag && lane == 0)   // gave up: the copies in flight end before the block does
+            for (int i = max(0, n - SW); i < n; ++i) mbar_wait(bar(Sh::kFullW + i % SW), (i / SW) & 1);
+    } else if (warp == 2) {
+        if (lane == 0) {
+            // -------------------------------------------------------------------------------- activations
+            // The units of chunk n take the slot of chunk n - 4.  They follow the chunk's second half, which is let in by the MMAs of half
+            // 2 n + 1 - SX: of chunk n - 3 or later, and the workers read the sums (and units) of chunk n - 4 before they store the operands of
+            // that one's second half.
             pdl_wait();
-            int n = 0;
-            for (; n < total; ++n) {
-                const int s = n % S, c = (w0 + n) % a.nchunks;
-                if (n >= S) {
-                    if (!wait(Sh::kEmpty + s, ((n / S) & 1) ^ 1)) break;
-                    load_w(n);
+            int h = 0;
+            for (; h < 2 * total; ++h) {
+                const int s = h % SX, n = h >> 1;
+                wait(Sh::kEmptyX + s, ((h / SX) & 1) ^ 1);   // (at once the first time round)
+                if (*abort_flag) break;
+                const unsigned char* chunk = a.xb + (size_t)((w0 + n) % a.nchunks) * xchunk_bytes(NP);
+                mbar_expect_tx(bar(Sh::kFullX + s), xhalf_bytes(NP));
+                bulk_g2s_plain(smem_u32(xring + s * xhalf_bytes(NP)), chunk + (h & 1) * xhalf_bytes(NP), xhalf_bytes(NP), bar(Sh::kFullX + s));
+                if (h & 1) {
+                    const int u = n % kScaleSlots;
+                    mbar_expect_tx(bar(Sh::kFullU + u), NP * 4);
+                    bulk_g2s_plain(smem_u32(units + u * NP), chunk + 2 * xhalf_bytes(NP), NP * 4, bar(Sh::kFullU + u));
                 }
-                mbar_expect_tx(bar(Sh::kFullX + s), xchunk_bytes(NP));
-                bulk_g2s_plain(smem_u32(ring + s * Sh::BYTES + kWBytes), a.xb + (size_t)c * xchunk_bytes(NP), xchunk_bytes(NP), bar(Sh::kFullX + s));
             }
-            if (n < total)   // gave up: the copies in flight end before the block does
-                for (int i = max(0, n - S); i < n; ++i) {
-                    mbar_wait(bar(Sh::kFullW + i % S), (i / S) & 1);
-                    mbar_wait(bar(Sh::kFullX + i % S), (i / S) & 1);
-                }
+            if (*abort_flag) {   // gave up
+                for (int i = max(0, h - SX); i < h; ++i) mbar_wait(bar(Sh::kFullX + i % SX), (i / SX) & 1);
+                for (int n = max(0, h / 2 - kScaleSlots); n < h / 2; ++n) mbar_wait(bar(Sh::kFullU + n % kScaleSlots), (n / kScaleSlots) & 1);
+            }
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------------------------ MMA issuer
-        // The whole warp walks the loop, one elected lane issues (see elect_one).  Stored A operands of a pair also say that
-        // every worker has read the accumulators of the pair before the last, whose stage this pair takes over; of three
-        // single-block stages the second block of a pair takes over that of the first block of the pair before, whose reading it
-        // waits for (before the first block's commit, so that the phase waited for cannot be followed by another unseen).
+    } else if (warp < 2) {
+        // ------------------------------------------------------------------------------------ MMA issuers, one for each row group
+        // The whole warp walks the loop, one elected lane issues (see elect_one).
         constexpr uint32_t idesc = idesc_bf16(NP);
-        const bool elected = elect_one();
-        bool ok = true;
-        uint32_t ph = 0;   // phase of the A slots
-        pdl_wait();        // see the workers' first wait for activations
-        Stage st;
-        for (int n = 0; n < total && ok; ++n) {
-            const int s = n % S;
-            if (!(ok = wait(Sh::kFullX + s, (n / S) & 1))) break;
-            const uint32_t xop = smem_u32(ring + s * Sh::BYTES + kWBytes);
+        const int g = warp;
+        const bool elected = elect_one(), six = a.six;
+        pdl_wait();        // see the workers' first wait
+        Ring<SX> xs;
+        for (int n = 0; n < total && !*abort_flag; ++n) {
+            const uint32_t d1 = tmem + (Sh::kTwice ? (n & 1) * Sh::kDCols : 0) + g * 2 * NP, d2 = d1 + NP;
 #pragma unroll 1
-            for (int p = 0; p < kPairs && ok; p += 2, ph ^= 1) {
+            for (int h = 0; h < 2; ++h, xs.step()) {
+                wait(Sh::kFullX + xs.at, xs.phase);
+                const uint64_t db0 = smem_desc(smem_u32(xring) + xs.at * xhalf_bytes(NP), 3 * NP * 16, 128);
 #pragma unroll
-                for (int as = 0; as < 2; ++as) {   // pair p + as
-                    if (!(ok = wait(Sh::kFullA + as, ph))) break;
+                for (int z = 0; z < kSlots; ++z) {
+                    const int slot = g * kSlots + z;
+                    wait(Sh::kFullA + slot, h);
                     tc_fence_after();
+                    if (elected) {
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint32_t dst = kTight ? st.at : as;
-                        if (elected) {
-                            const uint64_t db = smem_desc(xop + (p + as + 8 * j) * NP * 32, NP * 16, 128);
-#pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                const uint32_t d = tmem + dst * Sh::kDCols + ((DB == 2 ? 2 * j : 0) + g) * NP;
-                                const uint32_t av = tmem + Sh::kACol + as * 64 + g * 32 + j * 16;
-                                tc_mma_bf16_ta(d, av, db, idesc, 0u);
-                                tc_mma_bf16_ta(d, av + 8, db, idesc, 1u);
-                            }
+                        for (int b = 0; b < 4; ++b) {   // blocks 2 z, 2 z + 1 of a thread's four, of either half of the workers
+                            const uint32_t hi = tmem + Sh::kACol + slot * 64 + b * 16, lo = hi + 8, more = z + b > 0 ? 1u : (uint32_t)h;
+                            const uint64_t x1 = db0 + (b / 2 * 4 + z * 2 + b % 2) * (2 * 3 * NP), x2 = x1 + NP, x3 = x2 + NP;   // (in 16 bytes)
+                            tc_mma_bf16_ta(d2, hi, x3, idesc, more);
+                            if (six) tc_mma_bf16_ta(d2, lo, x3, idesc, 1u);
+                            tc_mma_bf16_ta(d2, lo, x2, idesc, 1u);
+                            tc_mma_bf16_ta(d2, hi, x2, idesc, 1u);
+                            tc_mma_bf16_ta(d2, lo, x1, idesc, 1u);
+                            tc_mma_bf16_ta(d1, hi, x1, idesc, more);
                         }
-                        __syncwarp();
-                        if (kTight && j == 0 && (as > 0 || n + p > 0)) {
-                            if (!(ok = wait(Sh::kRead, as ^ 1))) break;   // the pair before
-                            tc_fence_after();
-                        }
-                        if (elected && (kTight || j == 1)) tc_commit(bar(Sh::kFullD + dst));
-                        st.step();
-                        __syncwarp();
+                        tc_commit(bar(Sh::kDone + slot));
+                        if (z == 1) tc_commit(bar(Sh::kEmptyX + xs.at));
                     }
-                    if (!ok) break;
+                    __syncwarp();
                 }
             }
         }
-        if (!ok) {   // gave up: the MMAs in flight end before the tensor memory is freed
-            if (elected) tc_commit(bar(Sh::kDrain));
-            __syncwarp();
-            mbar_wait(bar(Sh::kDrain), 0);
-        }
+        if (elected) tc_commit(bar(Sh::kDrain + g));   // whatever became of the others: no MMA in flight when the tensor memory is freed
+        __syncwarp();
+        mbar_wait(bar(Sh::kDrain + g), 0);
     } else if (warp >= 4) {
         // ------------------------------------------------------------------------------------ workers
         regs_more<kRegsWork>();
-        const int wt = t - 128, q = warp & 3, cg = (warp - 4) >> 2;   // TMEM lanes 32 q ..; one of four warps on them
-        // unpack: row group `ug`, block p + 8 uj of the pair; scaling: rows `row` and `row + 128`, sequences [cg CW, cg CW + CW)
-        const int ug = cg & 1, uj = cg >> 1, urow = ug * 128 + q * 32 + lane, row = q * 32 + lane;
+        // Row group g; TMEM lanes 32 q ..; blocks 8 cg .. 8 cg + 7 of a chunk to unpack, sequences [cg CW, cg CW + CW) to add up.
+        const int wt = t - 128, g = (warp - 4) >> 3, cg = ((warp - 4) >> 2) & 1, q = warp & 3, row = g * 128 + q * 32 + lane;
         const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
-        const uint32_t a_addr = lanes + Sh::kACol + ug * 32 + uj * 16, d_addr = lanes + cg * CW;
-        // This row's eight scales of a chunk (blocks 8 uj ..), in the largest accesses that the row pitch allows; zero past the
-        // end of the row.
-        auto load_scales = [&](int w, uint32_t (&v)[4]) {
-            const int tile = w / a.nchunks, b0 = (w - tile * a.nchunks) * kBlocksPerChunk + 8 * uj, left = a.nkb - b0;
-            const __half* p = a.Wsc + (size_t)min(tile * kRows + urow, a.N - 1) * a.nkb + b0;
+        const uint32_t a_addr = lanes + Sh::kACol + g * 128 + cg * 32, d_addr = lanes + g * 2 * NP + cg * CW;
+        float acc[CW];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = 0;
-            if (a.sc_gran == 16) {
-                if (left > 0)
-                    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
-            } else if (a.sc_gran == 8) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-                    if (left > 4 * i) asm volatile("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(v[2 * i]), "=r"(v[2 * i + 1]) : "l"(p + 4 * i));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (left > 2 * i) asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(v[i]) : "l"(p + 2 * i));
-            }
-        };
-        float acc[2][CW];
-#pragma unroll
-        for (int g = 0; g < 2; ++g)
-#pragma unroll
-            for (int j = 0; j < CW; ++j) acc[g][j] = 0.f;
+        for (int j = 0; j < CW; ++j) acc[j] = 0.f;
         auto store = [&](int m, int n, float v) {
             const size_t yi = (size_t)m * a.y_stride + n;
             a.y[yi] = a.residual ? v + a.residual[yi] : v;
         };
-        // acc += accumulators of a block whose scales are at x
-        auto scale = [&](const uint32_t (&v)[2][CW], const float* x) {
-#pragma unroll
-            for (int i = 0; i < CW; i += 4) {
-                float xv[4];
-                *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(x + i);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int g = 0; g < 2; ++g) acc[g][i + j] = fmaf(__uint_as_float(v[g][i + j]), xv[j], acc[g][i + j]);
-            }
-        };
-        int team = 0;
-        auto team_sync = [&]() {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(Sh::kTeam));
-            return wait(Sh::kTeam, team++ & 1);
-        };
         // The tile of chunk `wlast` is finished (or this CTA's share of it): results out, accumulators back to zero.
-        auto finish = [&](int wlast) -> bool {
+        auto finish = [&](int wlast) {
             const int tile = wlast / a.nchunks, first = tile * a.nchunks, begin = max(w0, first);
             const int row0 = tile * kRows + row;
             if (a.csize > 1) {   // one tile per cluster: this CTA's share goes where the ring was, once all have left it
-                if (!team_sync()) return false;
+                __syncwarp();
+                mbar_arrive_by(lane == 0, bar(Sh::kTeam));
+                wait(Sh::kTeam, 0);
                 float* sm = reinterpret_cast<float*>(ring) + row;
 #pragma unroll
-                for (int j = 0; j < CW; ++j) {
-                    sm[(cg * CW + j) * kRows] = acc[0][j];
-                    sm[(cg * CW + j) * kRows + 128] = acc[1][j];
-                }
-                return true;
+                for (int j = 0; j < CW; ++j) sm[(cg * CW + j) * kRows] = acc[j];
+                return;
             }
+            if (*abort_flag) return;
             // (y may still be read, the partial tiles still be summed by the kernels before: past the dependency wait since chunk 0)
             if (begin == first && wlast == first + a.nchunks - 1) {
 #pragma unroll
-                for (int j = 0; j < CW; ++j) {
-                    const int m = cg * CW + j;
-                    if (m < a.M) {
-                        if (row0 < a.N) store(m, row0, acc[0][j]);
-                        if (row0 + 128 < a.N) store(m, row0 + 128, acc[1][j]);
-                    }
-                }
+                for (int j = 0; j < CW; ++j)
+                    if (cg * CW + j < a.M && row0 < a.N) store(cg * CW + j, row0, acc[j]);
             } else {
-                // a share that begins or ends inside the tile: the last CTA to arrive adds all shares in the order of K
+                // A share that begins or ends inside the tile: every warp leaves its part of it (32 rows x CW sequences), and the last
+                // CTA's warp to arrive there adds all shares in the order of K.  (One counter per tile, with the workers in step: 34.2
+                // against 32.3 us, 2,048 x 5,632 at 64 sequences in equal shares.)
                 float* mine = a.partial + (size_t)(2 * blockIdx.x + (begin == w0 ? 0 : 1)) * NE * kRows + row;
 #pragma unroll
                 for (int j = 0; j < CW; ++j)
-                    if (cg * CW + j < a.M) {
-                        mine[(cg * CW + j) * kRows] = acc[0][j];
-                        mine[(cg * CW + j) * kRows + 128] = acc[1][j];
-                    }
+                    if (cg * CW + j < a.M) mine[(cg * CW + j) * kRows] = acc[j];
                 __threadfence();
-                if (!team_sync()) return false;
+                __syncwarp();
                 const int grid = gridDim.x, i0 = chunk_owner(a, first, grid), i1 = chunk_owner(a, first + a.nchunks - 1, grid);
-                if (wt == 0) *last = (atomicAdd(&a.tickets[tile], 1u) == (unsigned)(i1 - i0)) ? 1 : 0;
-                if (!team_sync()) return false;
-                if (*last) {
+                unsigned int before = 0;
+                if (lane == 0) before = atomicAdd(&a.tickets[tile * kWorkers + warp - 4], 1u);
+                before = __shfl_sync(0xffffffffu, before, 0);
+                if (before == (unsigned)(i1 - i0)) {
                     __threadfence();
                     int b0, b1;
                     chunk_range(a, i0, grid, b0, b1);
@@ -361,122 +386,87 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
                     // share by share, every column's load of a share in flight together
                     auto add = [&](const float* p, bool first_share) {
 #pragma unroll
-                        for (int j = 0; j < CW; ++j)
-#pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                const float v = cg * CW + j < a.M ? __ldcg(p + (cg * CW + j) * kRows + 128 * g) : 0.f;
-                                acc[g][j] = first_share ? v : acc[g][j] + v;
-                            }
+                        for (int j = 0; j < CW; ++j) {
+                            const float v = cg * CW + j < a.M ? __ldcg(p + (cg * CW + j) * kRows) : 0.f;
+                            acc[j] = first_share ? v : acc[j] + v;
+                        }
                     };
                     add(p0, true);
 #pragma unroll 1
                     for (int i = 0; i < i1 - i0; ++i) add(p1 + (size_t)i * 2 * NE * kRows, false);
 #pragma unroll
                     for (int j = 0; j < CW; ++j)
-                        if (cg * CW + j < a.M) {
-                            if (row0 < a.N) store(cg * CW + j, row0, acc[0][j]);
-                            if (row0 + 128 < a.N) store(cg * CW + j, row0 + 128, acc[1][j]);
-                        }
+                        if (cg * CW + j < a.M && row0 < a.N) store(cg * CW + j, row0, acc[j]);
                 }
-                if (!team_sync()) return false;   // `last` is written again
             }
 #pragma unroll
-            for (int g = 0; g < 2; ++g)
-#pragma unroll
-                for (int j = 0; j < CW; ++j) acc[g][j] = 0.f;
-            return true;
+            for (int j = 0; j < CW; ++j) acc[j] = 0.f;
         };
 
-        uint32_t cur[4], next[4];
-        load_scales(w0, next);
-        bool ok = true;
-        Stage st;
-        const float* xs = nullptr;   // scales of the chunk whose accumulators are being read
-        // Unpack this thread's block of a pair into A slot `as` and hand it to the MMA issuer.  The MMAs that read the slot
-        // before are those of the pair before the last, whose accumulators this warp has seen.
-        auto unpack = [&](int as, uint32_t wlo, uint32_t whi, float sc) {
-            const ScaleParts sp = split_scale(sc);
-            uint32_t v[16];
-            unpack_word(wlo, sp, v, v + 8);
-            unpack_word(whi, sp, v + 4, v + 12);
-            tmem_st16(a_addr + as * 64, v);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(Sh::kFullA + as));
-        };
-        // Scale the accumulators of a pair (slot `as`, phase ph): blocks at xs + x and 8 blocks further.
-        auto take = [&](int as, uint32_t ph, const float* x) -> bool {
-            if constexpr (DB == 2) {
-                if (!wait(Sh::kFullD + as, ph)) return false;
-                tc_fence_after();
-                uint32_t v0[2][CW], v1[2][CW];
+        // acc += the sums over chunk n, which have been waited for
+        auto take = [&](int n) {
+            wait(Sh::kFullU + n % kScaleSlots, (n / kScaleSlots) & 1);
+            const float* u = units + n % kScaleSlots * NP + cg * CW;
+            const uint32_t d = d_addr + (Sh::kTwice ? (n & 1) * Sh::kDCols : 0);
 #pragma unroll
-                for (int g = 0; g < 2; ++g) tmem_ld<CW>(d_addr + as * Sh::kDCols + g * NP, v0[g]);
-#pragma unroll
-                for (int g = 0; g < 2; ++g) tmem_ld<CW>(d_addr + as * Sh::kDCols + (2 + g) * NP, v1[g]);
+            for (int j0 = 0; j0 < CW; j0 += Sh::LD) {
+                uint32_t d1[Sh::LD], d2[Sh::LD];
+                tmem_ld<Sh::LD>(d + j0, d1);
+                tmem_ld<Sh::LD>(d + NP + j0, d2);
                 tmem_wait_ld();
-                scale(v0, x);
-                scale(v1, x + 8 * NP);
-            } else {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    if (!wait(Sh::kFullD + st.at, st.phase)) return false;
-                    tc_fence_after();
-                    uint32_t v0[2][CW];
-#pragma unroll
-                    for (int g = 0; g < 2; ++g) tmem_ld<CW>(d_addr + st.at * Sh::kDCols + g * NP, v0[g]);
-                    st.step();
-                    tmem_wait_ld();
-                    if (j == 0) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(Sh::kRead));
-                    }
-                    scale(v0, x + 8 * j * NP);
-                }
+                for (int j = 0; j < Sh::LD; ++j)
+                    acc[j0 + j] = fmaf(__uint_as_float(d1[j]) + __uint_as_float(d2[j]), u[j0 + j], acc[j0 + j]);
             }
-            tc_fence_before();   // read before the next pair's arrival lets the MMAs write there
-            return true;
         };
-        uint32_t ph = 0;   // phase of the pairs of this loop iteration
-        for (int n = 0; n <= total && ok; ++n) {
-            const int s = n % S;
-            const unsigned char* src = ring + s * Sh::BYTES + urow * 128;
-            if (n < total) {
+        Ring<SW> ws;
+        const uint32_t row_off = row * 128, sc_off = kWBytes + cg * kRows * 16 + row * 16;
+        int left = a.nchunks - w0 % a.nchunks;   // chunks of the tile, from chunk n on
+        for (int n = 0; n < total && !*abort_flag; ++n) {
+            const unsigned char* stage = ring + ws.at * kStageBytes;
+            wait(Sh::kFullW + ws.at, ws.phase);
+            uint32_t sc[4];
+            *reinterpret_cast<uint4*>(sc) = *reinterpret_cast<const uint4*>(stage + sc_off);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) cur[i] = next[i];
-                if (n + 1 < total) load_scales(w0 + n + 1, next);
-                if (!(ok = wait(Sh::kFullW + s, (n / S) & 1))) break;
-            }
-#pragma unroll 1
-            for (int p = 0; p < kPairs; p += 2, ph ^= 1) {
-                uint4 w4;
-                float2 f;
-                if (n < total) {
-                    w4 = *reinterpret_cast<const uint4*>(src + (((4 * uj + p / 2) ^ (urow & 7)) << 4));
-                    f = __half22float2(*reinterpret_cast<const __half2*>(&cur[0]));
-                    cur[0] = cur[1]; cur[1] = cur[2]; cur[2] = cur[3];
-                    unpack(0, w4.x, w4.y, f.x);
+            for (int j = 0; j < 4; ++j) {   // blocks 2 j, 2 j + 1 of the thread's eight: half j / 2, slot j % 2
+                const int slot = g * kSlots + j % 2;
+                uint32_t v[32];
+                const uint4 w4 = *reinterpret_cast<const uint4*>(stage + row_off + (((4 * cg + j) ^ (row & 7)) << 4));
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&sc[j]));
+                const ScaleParts s0 = split_scale(f.x), s1 = split_scale(f.y);
+                unpack_word(w4.x, s0, v, v + 8);
+                unpack_word(w4.y, s0, v + 4, v + 12);
+                unpack_word(w4.z, s1, v + 16, v + 24);
+                unpack_word(w4.w, s1, v + 20, v + 28);
+                // The limit of a wait counts this kernel's own progress, not the time until the activations' producers are done (an
+                // exchange before them may wait longer for a late rank).
+                if (n == 0 && j == 2) pdl_wait();
+                wait(Sh::kDone + slot, j < 2);   // the slot's last MMAs (at once the first time)
+                tc_fence_after();
+                tmem_st16(a_addr + j % 2 * 64, v);
+                tmem_st16(a_addr + j % 2 * 64 + 16, v + 16);
+                if (!Sh::kTwice && j == 0 && n > 0) {   // the next MMAs take the place of the sums over the chunk before
+                    wait(Sh::kDone + g * kSlots + 1, 1);
+                    tc_fence_after();
+                    take(n - 1);
                 }
-                if (n + p > 0 && !(ok = take(1, ph ^ 1, xs + (p == 0 ? kPairs - 1 : p - 1) * NP))) break;
-                if (p == 0) {
-                    if (n > 0) {   // that was the last pair of chunk n - 1
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(Sh::kEmpty + (n - 1) % S));
-                        if ((n == total || (w0 + n) % a.nchunks == 0) && !(ok = finish(w0 + n - 1))) break;
-                    }
-                    if (n == total) break;
-                    // The limit of a wait counts this kernel's own progress, not the time until the activations' producers are done
-                    // (an exchange before them may wait longer for a late rank).
-                    if (n == 0) pdl_wait();
-                    if (!(ok = wait(Sh::kFullX + s, (n / S) & 1))) break;
-                    xs = reinterpret_cast<const float*>(ring + s * Sh::BYTES + kWBytes + xop_bytes(NP)) + cg * CW;
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                mbar_arrive_by(lane == 0, bar(Sh::kFullA + slot));
+                if (j == 3) mbar_arrive_by(lane == 0, bar(Sh::kEmptyW + ws.at));
+                if (j == (Sh::kTwice ? 1 : 0) && n > 0) {
+                    if (Sh::kTwice) take(n - 1);   // (complete: its last MMAs read the slot that was waited for)
+                    if (left == a.nchunks) finish(w0 + n - 1);
                 }
-                unpack(1, w4.z, w4.w, f.y);
-                if (!(ok = take(0, ph, xs + p * NP))) break;
             }
+            ws.step();
+            if (--left == 0) left = a.nchunks;
         }
+        wait(Sh::kDone + g * kSlots + 1, 1);
+        tc_fence_after();
+        take(total - 1);
+        finish(w0 + total - 1);
         if (a.csize > 1) {
             __syncwarp();
             cluster_sync_all();   // every CTA's share of the tile is in its shared memory
@@ -565,35 +555,36 @@ static int max_clusters(int csize) {
 // Launch geometry and scratch layout of one call: [tickets][activation chunks][partial tiles].
 struct WideLayout {
     int NE, nchunks, tiles, csize, grid;
-    float us;   // estimate of the call's time
     size_t xb_off, part_off, part_bytes;
 };
-// Equal shares of all chunks, or a cluster per tile: whichever the estimate says.  Measured (us, prep included; 4096 x 4096,
-// 6144 x 4096, 21888 x 4096, 4096 x 10944): a chunk of a tile takes 5.1 / 5.9 / 8.2 at 32 / 48 / 64 sequences; a cluster adds 6
-// to its longest share, equal shares add 10 and about 0.9 (at 32) for every share that the last CTA of a tile adds up.  Clusters of
-// 2 to 8 resident at once on a B200: 74, 45, 33, 26, 22, 15, 15.
+// A cluster per tile, equal shares of all chunks or whole tiles: whichever the estimate says.  Measured (us, prep included; 21
+// geometries of the matrices of three models, one CTA to 148): a chunk takes 2.3 / 3.1 / 4.0 at 32 / 48 / 64 sequences; a
+// cluster adds 6 to 8 to its longest share; whole tiles 6; equal shares 12 and 0.5 to 0.9 for every share of a tile.  4096 x 4096,
+// cluster of six / equal shares / whole tiles: 14.1 / 21.3 / 34.0 at 32 sequences; 21888 x 4096 (six, equal, whole): 56 / 36 / 36;
+// 32768 x 2048: 68 / 30 / 23.  Clusters of 2 to 8 resident at once on a B200: 74, 45, 33, 26, 22, 15, 15.
 static WideLayout layout_of(int M, int N, int K) {
     WideLayout l;
     l.NE = cols_of(M);
     l.nchunks = (K + kKc - 1) / kKc;
     l.tiles = (N + kRows - 1) / kRows;
-    const int sms = sm_count(current_device()), force = g_split.load();
+    const int sms = sm_count(current_device()), force = g_split.load(), at = l.NE / 16 - 2;
     const long long all = (long long)l.tiles * l.nchunks;
-    const float chunk = l.NE == 32 ? 5.1f : l.NE == 48 ? 5.9f : 8.2f;
+    const float chunk = std::array<float, 3>{2.3f, 3.1f, 4.0f}[at], share = std::array<float, 3>{0.5f, 0.7f, 0.9f}[at];
     l.csize = 1;
     l.grid = (int)(all < sms ? all : sms);
-    l.us = chunk * (float)((all + l.grid - 1) / l.grid) + 10.f + 0.9f * (float)l.NE / 32.f * (float)(l.grid / l.tiles + 1);
+    float best = chunk * (float)((all + l.grid - 1) / l.grid) + 12.f + share * (float)(l.grid / l.tiles + 1);
+    const float whole = chunk * (float)l.nchunks * (float)((l.tiles + sms - 1) / sms) + 5.5f;
+    if (whole < best) { best = whole; l.csize = 0; }
     for (int cs = 8; cs > 1; --cs)
         if (cs <= l.nchunks && l.tiles <= max_clusters(cs)) {   // the largest that is resident at once
-            const float us = 6.f + chunk * (float)((l.nchunks + cs - 1) / cs);
-            if (us < l.us) { l.us = us; l.csize = cs; }
+            if (6.6f + 0.6f * (float)at + chunk * (float)((l.nchunks + cs - 1) / cs) < best) l.csize = cs;
             break;
         }
     if (force > 8) l.csize = 1;
     else if (force > 1 && force <= l.nchunks) l.csize = force;
     else if (force == 1) l.csize = 0;
     // The arrival counters own a region of fixed size at the front of the block.  Matrices with more tiles than counters are dealt out by whole tiles.
-    if (l.csize == 1 && (size_t)l.tiles * sizeof(unsigned int) > tc::kTicketBytes) l.csize = 0;
+    if (l.csize == 1 && (size_t)l.tiles * kWorkers * sizeof(unsigned int) > tc::kTicketBytes) l.csize = 0;
     if (l.csize == 0) l.grid = l.tiles < sms ? l.tiles : sms;
     if (l.csize > 1) l.grid = l.tiles * l.csize;
     l.part_bytes = l.csize == 1 ? (size_t)l.grid * 2 * l.NE * kRows * sizeof(float) : 0;
@@ -603,29 +594,27 @@ static WideLayout layout_of(int M, int N, int K) {
 }
 static std::atomic<int> g_force{0};
 void set_force(int v) { g_force = v; }
-// Whether a call of 17 to 64 sequences is faster here than in the int8 form (gemm_w4a8_tc.cu), by the estimates of both.  That
-// one takes 2.27 us for a chunk of 128 rows up to 32 sequences and 3.33 above (it computes 64 columns then), its tiles come in
-// whole rounds of one per SM, and a K split adds 2.2 / 3.6 us per part.  Measured, this form / that one: 6144 x 4096 26 / 31 at 32
-// sequences, 31 / 46 at 48, 40 / 47 at 64; 21888 x 4096 62 / 80, 72 / 115, 95 / 115; 3072 x 2048 11 / 26, 13 / 42, 16 / 42;
-// 4096 x 10944 42 / 41, 48 / 58, 65 / 59; 4096 x 12288 46 / 42, 54 / 60, 72 / 60; 32768 x 2048 47 / 45, 55 / 64, 71 / 64;
-// 151643 x 4096 327 / 329, 383 / 480, 526 / 482: the rule takes the faster one in each but the last at 32, where they are level.
-// And whether every sum is a shorter chain of chunks than there, or neither splits K: a narrow matrix of very long rows is split
-// finer by the int8 form (300 x 32768, 64 chunks: 4 against 16 in a cluster of eight), and its error against 64 bits was 1.8e-7
-// where this form had 2.9e-7.  With the shorter chains here it is 0.6 to 0.99 of that form's (2048 to 24576 rows of 2048 to 12288,
-// 17 to 64 sequences; 1.02 at most over 60 random sizes, 1.15 where the chains were equal).
+// Whether a call of 17 to 64 sequences comes here; the int8 form (gemm_w4a8_tc.cu) takes the same operands.  Measured (us, prep
+// included, this form / that one at 17, 32, 48 and 64 sequences): 6144 x 4096 17 / 32, 18 / 33, 23 / 48, 28 / 48; 21888 x 4096
+// 37 / 81, 38 / 81, 46 / 116, 55 / 117; 4096 x 12288 25 / 42, 28 / 43, 35 / 61, 41 / 61; 2048 x 2048 9.7 / 22, 10 / 22, 12 / 32,
+// 13 / 33; 633 x 64 7.4 / 8.9, 7.4 / 8.8, 8.7 / 11, 10 / 12: this one is faster at every one of 24 shapes, by 0.16 to 0.9.
+// It does not come here where its chains of chunks would be longer than that form's, unless neither splits K: a narrow matrix of very
+// long rows (300 x 32768), which that form splits finer.
+// Error against 64 bits (2-norm, three seeds; five products / six / the forms that these calls took before): 633 x 64
+// 8.9e-8 / 2.8e-8 / 4.0e-8, 2481 x 1024 1.0e-7 / 4.9e-8 / 8.3e-8, 3072 x 2048 1.04e-7 / 5.6e-8 / 8.8e-8, 2048 x 5632 1.09e-7 / 6.6e-8 /
+// 1.30e-7, 4096 x 4096 1.08e-7 / 6.4e-8 / 1.28e-7, 21888 x 4096 1.12e-7 / 7.1e-8 / 2.0e-7, 4096 x 12288 1.17e-7 / 7.8e-8 / 2.1e-7 to
+// 2.5e-7.  Hence six products up to kSixK, where five would lose more than those did; above, the sixth costs 5 to 10 % of the time.
+constexpr int kSixK = 3072;
 bool preferred(int M, int N, int K) {
-    if (M <= 16 || !usable(cols_of(M))) return false;   // the int8 form takes the same operands
+    if (M <= 16 || !usable(cols_of(M))) return false;
     if (g_force.load() != 0) return g_force.load() > 0;
     const int sms = sm_count(current_device()), tiles = (N + 127) / 128, nchunks = (K + kKc - 1) / kKc;
     const int ks = std::max(1, std::min(sms / tiles, nchunks));
-    const int boxes = ((nchunks + 1) / 2 + ks - 1) / ks, rounds = (tiles * ks + sms - 1) / sms;
-    const float chunks = (float)(std::min(2 * boxes, nchunks) * rounds);
-    const float us = M <= 32 ? 2.27f * chunks + (ks > 1 ? 8.f + 2.2f * ks : 6.f) : 3.33f * chunks + (ks > 1 ? 10.f + 3.6f * ks : 6.f);
+    const int theirs = std::min(2 * (((nchunks + 1) / 2 + ks - 1) / ks), nchunks);
     const WideLayout l = layout_of(M, N, K);
     const int share = (int)(((long long)l.tiles * l.nchunks + l.grid - 1) / l.grid);
     const int chain = l.csize == 0 ? nchunks : std::min(share, nchunks);
-    const int theirs = std::min(2 * boxes, nchunks);
-    return l.us < us && (chain < theirs || theirs == nchunks);
+    return chain < theirs || theirs == nchunks;
 }
 // Enough for every batch up to M.
 size_t scratch_bytes(int M, int N, int K) {
@@ -680,7 +669,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
 
     e = launch_pdl(prep_x_kernel, dim3((lay.nchunks + 7) / 8, M), dim3(256), 0, st, scratch + lay.xb_off, a, lay.NE, lay.nchunks,
-                   reinterpret_cast<unsigned int*>(scratch), lay.csize == 1 ? lay.tiles : 0);
+                   reinterpret_cast<unsigned int*>(scratch), lay.csize == 1 ? lay.tiles * kWorkers : 0);
     count_launch(1);
     if (e != cudaSuccess) return e;
 
@@ -694,7 +683,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     t.partial = reinterpret_cast<float*>(scratch + lay.part_off);
     t.tickets = reinterpret_cast<unsigned int*>(scratch);
     t.status = a.status;
-    t.N = a.N; t.M = M; t.nchunks = lay.nchunks; t.tiles = lay.tiles; t.csize = lay.csize;
+    t.N = a.N; t.M = M; t.nchunks = lay.nchunks; t.tiles = lay.tiles; t.csize = lay.csize; t.six = a.K <= kSixK;
     switch (lay.NE) {
         case 32: return launch_n<32>(map_w, t, lay.grid, st);
         case 48: return launch_n<48>(map_w, t, lay.grid, st);

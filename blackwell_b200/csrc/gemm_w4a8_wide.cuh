@@ -3,32 +3,41 @@
 //
 //   y[m][n] = sum_kb (sum_{k in kb} W[n,k] * w_sc[n,kb] * xq[m,k]) * x_sc[m,kb]
 //
-// The weight scale goes into the MMA's A operand without rounding: a binary16 scale s (11 significant bits) is the sum of
-// two bf16 numbers of five significant bits each, s = sh + sl (sh = s rounded to five bits, |s - sh| <= 32 units of s's last
-// place), a nibble q in [-8, 7] has three, so q * sh and q * sl are bf16 numbers exactly.  An int8 activation is a bf16 number
-// exactly.  One k-block is the K = 16 of one MMA: two MMAs (q sh, then += q sl) leave w_sc * dot16 in the accumulator.  All
-// products of an MMA are integer multiples of one unit with sums below 2^19, and w_sc * dot16 has 25 bits at the most
-// (11 + 14), so what the accumulator holds is exact but for its last bit in extreme blocks.  What remains per (row, sequence,
-// block) is ONE fp32 FMA with the activation scale.
+// Both block scales go into the MMA's operands, as sums of bf16 numbers, so that an accumulator runs over a whole chunk of 256 k
+// and one fp32 FMA per (row, sequence, chunk) is left of the scaling.
+//   Weights: a binary16 scale s (11 significant bits) is sh + sl, two numbers of five significant bits each (sh = s rounded to
+//   five bits, |s - sh| <= 32 units of s's last place); a nibble q in [-8, 7] has three, so q sh and q sl are bf16 numbers: exact.
+//   Activations: x = xq x_sc is cut into x1 + x2 + x3 in units of a power of two u per (sequence, chunk), u the place of the eighth
+//   bit of the chunk's largest |x|: x1 = x rounded to whole units (|x1| <= 256), x2 the rest as a bf16 number, x3 what is still
+//   left as another: 2^-27 of the chunk's largest |x| or less is lost (an fp32 number loses 2^-25 of itself).
+// Products: q sh x1 | q sh x2, q sh x3, q sl x1, q sl x2, and q sl x3 where the chains of sums are short (WideArgs::six): without
+// it 8e-8 of a result is lost, whatever its length.
+// The first product has an accumulator of its own: x1 and, where the scales of a row's chunk share an exponent, q sh are whole
+// numbers of one unit below 2^8 in magnitude, so its sum over 256 k stays below 2^24 units and is exact -- the tensor core cuts off
+// what an addition shifts out, which in one accumulator would cost up to a unit of the last place at every step, always towards
+// zero.  The others are 2^-5 to 2^-22 of the first; what is cut off there does not count.  The sum of both times u joins the fp32
+// result.  Errors against 64 bits: beside preferred() in the .cu file.
 //
-// Against the int8 form (gemm_w4a8_tc.cuh: exact int32 dots, two FMAs per value in the epilogue) this moves half of the scaling
-// to the operand, where it is done once per weight and not once per weight and sequence.
+// Against the int8 form (gemm_w4a8_tc.cuh: exact int32 dots, two FMAs per row, sequence and block in the epilogue) and an earlier
+// bf16 form (weight scale in A, activation scale by one FMA per row, sequence and block) this trades CUDA-core work and
+// tensor-memory reads for 2.5 to 3 times the MMAs; the tensor pipe had been 11 to 14 % busy.  151,643 x 4096 at 32 / 48 / 64 sequences,
+// prep included: int8 form 329 / 480 / 482 us, earlier bf16 form 327 / 383 / 526, this one 170 / 225 / 280.
 //
-// A tile is 256 weight rows: two MMA row groups that share the activations and their scales.  Roles in a CTA of 20 warps:
-//   warp 0       producer: TMA boxes of 256 rows x 128 bytes of nibbles, bulk copies of activations and their scales
-//   warp 1       MMA issuer
-//   warps 4-19   workers, all alike: a worker unpacks one k-block of one row per thread and pair of blocks (nibbles -> q sh, q sl
-//                by packed bf16 FMAs, stored straight to tensor memory: through shared memory the A operand alone would take a
-//                third of its bandwidth), then scales the accumulators of the pair before, two rows x a quarter of the sequences
-//                per thread.  Unpack and scaling in the same warps: four independent warps per scheduler hide each other's
-//                tensor-memory and barrier latencies (eight unpack and eight epilogue warps measured 594 us where this takes
-//                530: 151,643 x 4096, 64 sequences).
-// A pair is the blocks (p, p + 8) of a chunk, so that a thread's eight blocks are consecutive: its scales are 16 bytes, its
-// nibbles come two blocks per 16-byte load.  Scalar FMAs, not packed ones: the packed form goes to half of the FMA pipe, which
-// the bf16 FMAs of the unpack already fill (708 against 517 us, same case).
-// What bounds it (75,776 x 4096, 32 / 48 / 64 sequences): issue slots 63 / 68 / 68 % busy with five warps per scheduler, then the
-// latency chain of a worker's step; HBM 15 / 13 / 10 %, tensor pipe 11 / 14 / 14 % active.  Spilled by ptxas at 32 / 48 columns:
-// 12 / 56 bytes stored, 56 loaded; none at 64.
+// A tile is 256 weight rows: two MMA row groups that share the activations.  Roles in a CTA of 20 warps:
+//   warps 0, 1   MMA issuers, one for each row group: between two A slots an issuer needs some 150 cycles, which the other's MMAs
+//                fill (65,536 x 4096 at 32 / 64 sequences: 101 / 139 us with one issuer for both, 94 / 131 with two)
+//   warp 2       activations: bulk copies of half a chunk's operand
+//   warp 3       nibbles: TMA boxes of 256 rows x 128 bytes; weight scales: 32 bytes of a row and chunk by cp.async
+//   warps 4-19   workers: a worker thread unpacks k-blocks of one row (nibbles -> q sh, q sl by packed bf16 FMAs, stored straight to
+//                tensor memory: through shared memory the A operand alone would take its whole bandwidth) and, once per chunk,
+//                adds up the accumulators of that row x half of the sequences.
+// Eight workers serve each row group, so that one group's waiting falls into the other's unpacking and MMAs.  A thread's eight blocks
+// of a chunk are consecutive, four to each half: half h of a chunk is the blocks whose index has bit 2 equal to h, and the
+// activations are laid out the same way.
+// What bounds it (65,536 x 4096): at 64 sequences the tensor pipe, 81 % busy at the 1.55 GHz that the power limit leaves (five products
+// of 64 columns take 161 cycles per k-block and group; 48 / 32 columns 121 / 83, measured); at 32 the workers' issue
+// slots (63 % used; bf16 FMAs, shifts and logic operations take two cycles of their pipes each): with one MMA in five the same
+// kernel takes 74 us of 80 there, with two thirds of the activation traffic left out 79.
 // All waits are bounded; a wait that gives up raises an abort flag.
 #pragma once
 #include <cuda_bf16.h>
@@ -52,11 +61,13 @@ using tc::tmem_wait_ld;
 
 constexpr int kKc = 256;          // k per chunk = 16 k-blocks
 constexpr int kBlocksPerChunk = 16;
-constexpr int kPairs = 8;         // block pairs (p, p + 8) of a chunk
 constexpr int kRows = 256;        // weight rows per tile: two MMA row groups of 128
 constexpr int kWBytes = kRows * (kKc / 2);           // nibbles of a tile's chunk: 128 bytes a row, 128-byte swizzle
 constexpr int kWorkers = 16;                         // worker warps
-constexpr int kThreads = 128 + kWorkers * 32;        // warp 0 producer, warp 1 MMA issuer, two idle warps, workers
+constexpr int kStageBytes = kWBytes + kRows * 32;    // and the scales: [blocks 0-7, 8-15][row][16 bytes]
+constexpr int kThreads = 128 + kWorkers * 32;        // two MMA issuers, activations, weights, workers
+constexpr int kScaleSlots = 4;    // chunks whose units u are in shared memory
+constexpr int kSlots = 2;         // A slots of a row group, four k-blocks each (eight in one slot, at 32 sequences: 86 against 78 us)
 // Registers by role: the launch gives every thread 96; the first four warps keep 32, the workers take 112.
 constexpr int kRegsFew = 32, kRegsWork = 112;
 static_assert(4 * kRegsFew + kWorkers * kRegsWork <= (4 + kWorkers) * 96, "register shares above the launch's total wait forever");
@@ -65,33 +76,43 @@ struct WideArgs {
     float* y;                 // [M][y_stride]
     const float* residual;    // optional, same layout as y
     long y_stride;
-    const unsigned char* xb;  // activations in chunk layout (see prep kernel)
+    const unsigned char* xb;  // activations in chunk layout (see the prep kernel)
     const __half* Wsc;        // [N][nkb] weight scales
     int nkb;                  // K / 16
     int sc_gran;              // largest of 16, 8, 4 bytes that divides scale base and row pitch
     float* partial;           // [CTA][2][sequences][256] partial tiles of K ranges that begin or end inside a tile
-    unsigned int* tickets;    // [tiles], zero at the start (see the prep kernel)
+    unsigned int* tickets;    // [tiles][worker warps], zero at the start (see the prep kernel)
     int* status;              // device status word
     int N, M;
     int nchunks;              // ceil(K / 256)
     int tiles;                // ceil(N / 256)
     int csize;                // > 1: the CTAs of a cluster share one tile's K range; 1: chunks of all tiles dealt out
                               // evenly; 0: whole tiles dealt out
+    int six;                  // all six products, not five
 };
 
-// bytes of one activation chunk: [block 0..15][k half][NP sequences x 16 B bf16], then 16 x NP fp32 block scales
-__host__ __device__ constexpr int xop_bytes(int NP) { return kBlocksPerChunk * NP * 32; }
-__host__ __device__ constexpr int xchunk_bytes(int NP) { return xop_bytes(NP) + kBlocksPerChunk * NP * 4; }
+// bytes of half an activation chunk: [block 0..7][k half][x1, x2, x3][NP sequences x 16 B bf16]; of a chunk: two halves, then NP units u
+__host__ __device__ constexpr int xhalf_bytes(int NP) { return 8 * 2 * 3 * NP * 16; }
+__host__ __device__ constexpr int xchunk_bytes(int NP) { return 2 * xhalf_bytes(NP) + NP * 4; }
 
-// Bounded wait of a converged warp whose common case is a probe and a branch; false after about a second.
-__device__ __forceinline__ bool mbar_wait_quick(uint32_t bar, uint32_t parity) {
-    uint32_t tries;
+// Bounded wait that is a probe and a branch in the common case.  After more than a second, or once another has given up (a non-zero
+// word of shared memory at `flag`), it sets that word and returns; the caller looks at it now and then.  What is computed in between
+// is never stored.
+__device__ __forceinline__ void mbar_wait_or_abort(uint32_t bar, uint32_t parity, uint32_t flag) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmov.u32 %0, 0;\n"
-        "W%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra D%=;\n\t"
-        "add.u32 %0, %0, 1;\n\tsetp.lt.u32 p, %0, 64;\n\t@p bra W%=;\nD%=:\n\t}"
-        : "=&r"(tries) : "r"(bar), "r"(parity) : "memory");
-    return tries < 64 || mbar_wait(bar, parity);
+        "{\n\t.reg .pred p;\n\t.reg .b32 f;\n\t.reg .b64 t0, t1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra D%=;\n\t"
+        "mov.u64 t0, %%clock64;\n"
+        "W%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra D%=;\n\t"
+        "ld.volatile.shared.u32 f, [%2];\n\tsetp.ne.u32 p, f, 0;\n\t@p bra D%=;\n\t"
+        "mov.u64 t1, %%clock64;\n\tsub.s64 t1, t1, t0;\n\tsetp.lt.s64 p, t1, 2500000000;\n\t@p bra W%=;\n\t"
+        "st.volatile.shared.u32 [%2], 1;\nD%=:\n\t}"
+        ::"r"(bar), "r"(parity), "r"(flag) : "memory");
+}
+// Arrival of the lanes for which `yes` holds, without a branch around it (94 against 85 us, 65,536 x 4096 at 32 sequences).
+__device__ __forceinline__ void mbar_arrive_by(bool yes, uint32_t bar) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+                 ::"r"(bar), "r"((uint32_t)yes) : "memory");
 }
 // D = A * B (accumulate == 0) or D += A * B; A (bf16, row = lane, two k per column) in tensor memory, B in shared memory.
 __device__ __forceinline__ void tc_mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -115,12 +136,18 @@ __device__ __forceinline__ void tmem_ld<12>(uint32_t addr, uint32_t* v) {
     tmem_ld<8>(addr, v);
     tmem_ld<4>(addr + 8, v + 8);
 }
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
         ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
           "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(addr)
         : "memory");
+}
+// Asynchronous copy of B bytes global -> shared; src_bytes 0 writes zeros.
+template <int B>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, uint32_t src_bytes) {
+    if constexpr (B == 16) asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+    else asm volatile("cp.async.ca.shared.global.L2::256B [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(src_bytes), "n"(B) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -137,7 +164,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
 // ------------------------------------------------------------------ weight unpack
 // What the unpack of one k-block needs of its scale s = sh + sl, each as a bf16 number in both halves of a word.
 struct ScaleParts {
-    uint32_t sh8, sh24, sl8, sl24;   // sh / 8, -24 sh, sl / 8, -24 sl: exact (24 has two significant bits)
+    uint32_t sh, sh192, sl, sl192;   // sh, -192 sh, sl, -192 sl: exact (192 has two significant bits)
 };
 // In the fp32 form of a binary16 number mantissa bits 12..0 are zero: bits 22..19 stay in sh (rounded), what is left is a
 // multiple of bit 13 of magnitude at most 2^5 such units.  Both parts and their multiples end above bit 16 of the word.
@@ -151,23 +178,23 @@ __device__ __forceinline__ ScaleParts split_scale(float s) {
         asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(by));
         return r;
     };
-    return ScaleParts{mul(sh, 0x3E003E00u), mul(sh, 0xC1C0C1C0u), mul(sl, 0x3E003E00u), mul(sl, 0xC1C0C1C0u)};
+    return ScaleParts{sh, mul(sh, 0xC340C340u), sl, mul(sl, 0xC340C340u)};
 }
 __device__ __forceinline__ uint32_t bfma2(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t r;
     asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
     return r;
 }
-// Four words of A: nibbles (i, i + 4) of w, i = 0..3, as bf16 pairs q sh (hi) and q sl (lo).  A nibble n at bits 6..3 under
-// the exponent of 128 is 8 (16 + n) in bf16, and 8 (16 + n) * s / 8 - 24 s = (n - 8) s: one FMA, exact.
+// Four words of A: nibbles (i, i + 4) of w, i = 0..3, as bf16 pairs 8 q sh (hi) and 8 q sl (lo).  A nibble n at bits 6..3 under
+// the exponent of 128 is 128 + 8 n in bf16, and (128 + 8 n) s - 192 s = 8 (n - 8) s: one FMA, exact.  (The eight is in u.)
 __device__ __forceinline__ void unpack_word(uint32_t w, const ScaleParts& s, uint32_t* hi, uint32_t* lo) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         uint32_t n;
         const uint32_t sft = i == 0 ? w << 3 : w >> (4 * i - 3);
         asm("lop3.b32 %0, %1, 0x00780078, 0x43004300, 0xEA;" : "=r"(n) : "r"(sft));   // (a & b) | c
-        hi[i] = bfma2(n, s.sh8, s.sh24);
-        lo[i] = bfma2(n, s.sl8, s.sl24);
+        hi[i] = bfma2(n, s.sh, s.sh192);
+        lo[i] = bfma2(n, s.sl, s.sl192);
     }
 }
 

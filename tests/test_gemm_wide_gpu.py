@@ -192,3 +192,27 @@ def test_counters_of_a_call_that_gave_up_do_not_reach_the_next(k, form, split):
     assert k.device_status() == 0
     assert torch.equal(y, want)
     assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
+
+
+# Halves of a chunk that K ends in, six products (K up to 3,072) and five, one and many chunks, whole tiles and shares.
+@pytest.mark.parametrize("M,K,N,split", [(17, 96, 40, 0), (48, 128, 513, 0), (64, 160, 256, 0), (33, 3072, 300, 0), (32, 3104, 300, 0),
+                                         (64, 4096, 2000, 0), (20, 4128, 2000, 9), (48, 2080, 700, 1)])
+def test_error_against_64_bits(k, M, K, N, split):
+    """Neighbouring blocks and weights of very different size.  What is lost beside the fp32 sums: sl x3, 8e-8 (2-norm) where it is
+    left out, and the fp32 additions, at most K / 256 + 2 roundings of 2^-24.  Without any other of the products: 6e-6 or more."""
+    import torch
+
+    r = synth.rng(K + N)
+    W, sc16, _ = synth.int4_weights(N, K, seed=K, full_range=True)
+    sc16 = (sc16.astype(np.float32) * 2.0 ** r.integers(-6, 7, size=sc16.shape)).astype(np.float16)
+    x = synth.activations_f16(M, K, 95).astype(np.float32) * np.repeat(2.0 ** r.integers(-6, 7, size=(M, K // 16)), 16, 1).astype(np.float32)
+    xq, xs = oracle.quantize_int8(x)
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    k.set_tuning(6, split)
+    try:
+        k.gemv_w4a8(y, to_dev(xq), to_dev(xs), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M)
+    finally:
+        k.set_tuning(6, 0)
+    ref = oracle.gemv_w4a8_f64(xq, xs, W, sc16)
+    err = np.linalg.norm(y.cpu().numpy() - ref) / np.linalg.norm(ref)
+    assert err < (1e-7 if K <= 3072 else 2e-7) + (K // 256 + 2) ** 0.5 * 2.0 ** -25
