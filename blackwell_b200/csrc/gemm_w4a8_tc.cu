@@ -525,6 +525,7 @@ static EncodeTiledFn encode_fn() {
 // Per-device scratch: activation chunks, K-split partials, tickets (zeroed by the prep kernel of a call that splits K).
 static GrowScratch g_tc_scratch;
 cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p) { return g_tc_scratch.get(bytes, (size_t)16 << 20, st, p); }
+bool scratch_at_hand(size_t bytes, cudaStream_t st) { return g_tc_scratch.at_hand(bytes, st); }
 cudaError_t reserve_scratch(size_t bytes) {
     unsigned char* p = nullptr;
     return bytes ? g_tc_scratch.get(bytes, (size_t)16 << 20, nullptr, &p) : cudaSuccess;

@@ -60,6 +60,7 @@ constexpr int kThreads = (4 + kEpiWarps + 4) * 32;   // + producer, MMA issuer, 
 // (larger matrices are not split inside a tile), then what a call lays out.
 constexpr size_t kTicketBytes = 65536;
 cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p);
+bool scratch_at_hand(size_t bytes, cudaStream_t st);   // whether that would not have to grow under capture
 
 struct TcArgs {
     float* y;                 // [M][y_stride]

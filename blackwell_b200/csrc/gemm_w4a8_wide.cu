@@ -112,8 +112,8 @@ struct WideShape {
     static constexpr int kACol = (kTwice ? 2 : 1) * kDCols;   // A: [row group][slot][half of its workers][two blocks][q sh, q sl][8]
     // stages of weights (of a chunk) and of activations (of half a chunk): with few sequences the weights in flight matter, with many
     // the tensor pipe takes its time over a chunk
-    static constexpr int SW = NE == 32 ? 3 : 2;
-    static constexpr int SX = NE == 64 ? 3 : 4;
+    static constexpr int SW = NE == 16 ? 4 : NE == 32 ? 3 : 2;
+    static constexpr int SX = NE == 16 ? 5 : NE == 64 ? 3 : 4;
     static constexpr int kSmem = 1024 + 2048 + SW * kStageBytes + SX * xhalf_bytes(NP);   // alignment; barriers, flags, units; the rings
     static_assert(kACol + 2 * kSlots * 64 <= 512 && kSmem <= kMaxDynSmem, "shape");
     static_assert(NE * kRows * 4 <= SW * kStageBytes, "the tile for the cluster reduction takes the place of the weights");
@@ -293,7 +293,7 @@ gemm_w4a8_wide_kernel(const __grid_constant__ CUtensorMap map_w, const WideArgs 
         // The whole warp walks the loop, one elected lane issues (see elect_one).
         constexpr uint32_t idesc = idesc_bf16(NP);
         const int g = warp;
-        const bool elected = elect_one(), six = a.six;
+        const bool elected = elect_one(), six = NE == 16 || a.six;
         pdl_wait();        // see the workers' first wait
         Ring<SX> xs;
         for (int n = 0; n < total && !*abort_flag; ++n) {
@@ -508,7 +508,7 @@ static std::atomic<int> g_split{0};
 void set_split(int v) { g_split = v; }
 
 // Sequences an instantiation handles: those of M rounded up.
-static int cols_of(int M) { return M <= 32 ? 32 : M <= 48 ? 48 : 64; }
+static int cols_of(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 48 ? 48 : 64; }
 
 // Makes an instance launchable on the current device, once.  The roles' register shares are drawn from what the launch allocates.
 template <int NE>
@@ -526,7 +526,9 @@ static cudaError_t prepare() {
     });
     return usable[dev];
 }
-static bool usable(int NE) { return (NE == 32 ? prepare<32>() : NE == 48 ? prepare<48>() : prepare<64>()) == cudaSuccess; }
+static bool usable(int NE) {
+    return (NE == 16 ? prepare<16>() : NE == 32 ? prepare<32>() : NE == 48 ? prepare<48>() : prepare<64>()) == cudaSuccess;
+}
 
 // Clusters of `csize` CTAs that are resident at once on the current device, at most (the SMs of a cluster share a GPC).
 static int max_clusters(int csize) {
@@ -558,7 +560,7 @@ struct WideLayout {
     size_t xb_off, part_off, part_bytes;
 };
 // A cluster per tile, equal shares of all chunks or whole tiles: whichever the estimate says.  Measured (us, prep included; 21
-// geometries of the matrices of three models, one CTA to 148): a chunk takes 2.3 / 3.1 / 4.0 at 32 / 48 / 64 sequences; a
+// geometries of the matrices of three models, one CTA to 148): a chunk takes 2.0 / 2.3 / 3.1 / 4.0 at 16 / 32 / 48 / 64 sequences; a
 // cluster adds 6 to 8 to its longest share; whole tiles 6; equal shares 12 and 0.5 to 0.9 for every share of a tile.  4096 x 4096,
 // cluster of six / equal shares / whole tiles: 14.1 / 21.3 / 34.0 at 32 sequences; 21888 x 4096 (six, equal, whole): 56 / 36 / 36;
 // 32768 x 2048: 68 / 30 / 23.  Clusters of 2 to 8 resident at once on a B200: 74, 45, 33, 26, 22, 15, 15.
@@ -567,9 +569,9 @@ static WideLayout layout_of(int M, int N, int K) {
     l.NE = cols_of(M);
     l.nchunks = (K + kKc - 1) / kKc;
     l.tiles = (N + kRows - 1) / kRows;
-    const int sms = sm_count(current_device()), force = g_split.load(), at = l.NE / 16 - 2;
+    const int sms = sm_count(current_device()), force = g_split.load(), at = l.NE / 16 - 1;
     const long long all = (long long)l.tiles * l.nchunks;
-    const float chunk = std::array<float, 3>{2.3f, 3.1f, 4.0f}[at], share = std::array<float, 3>{0.5f, 0.7f, 0.9f}[at];
+    const float chunk = std::array<float, 4>{2.0f, 2.3f, 3.1f, 4.0f}[at], share = std::array<float, 4>{0.4f, 0.5f, 0.7f, 0.9f}[at];
     l.csize = 1;
     l.grid = (int)(all < sms ? all : sms);
     float best = chunk * (float)((all + l.grid - 1) / l.grid) + 12.f + share * (float)(l.grid / l.tiles + 1);
@@ -577,7 +579,7 @@ static WideLayout layout_of(int M, int N, int K) {
     if (whole < best) { best = whole; l.csize = 0; }
     for (int cs = 8; cs > 1; --cs)
         if (cs <= l.nchunks && l.tiles <= max_clusters(cs)) {   // the largest that is resident at once
-            if (6.6f + 0.6f * (float)at + chunk * (float)((l.nchunks + cs - 1) / cs) < best) l.csize = cs;
+            if (6.f + 0.6f * (float)at + chunk * (float)((l.nchunks + cs - 1) / cs) < best) l.csize = cs;
             break;
         }
     if (force > 8) l.csize = 1;
@@ -594,7 +596,7 @@ static WideLayout layout_of(int M, int N, int K) {
 }
 static std::atomic<int> g_force{0};
 void set_force(int v) { g_force = v; }
-// Whether a call of 17 to 64 sequences comes here; the int8 form (gemm_w4a8_tc.cu) takes the same operands.  Measured (us, prep
+// Whether a call of 9 to 64 sequences comes here.  From 17 on the int8 form (gemm_w4a8_tc.cu) takes the same operands.  Measured (us, prep
 // included, this form / that one at 17, 32, 48 and 64 sequences): 6144 x 4096 17 / 32, 18 / 33, 23 / 48, 28 / 48; 21888 x 4096
 // 37 / 81, 38 / 81, 46 / 116, 55 / 117; 4096 x 12288 25 / 42, 28 / 43, 35 / 61, 41 / 61; 2048 x 2048 9.7 / 22, 10 / 22, 12 / 32,
 // 13 / 33; 633 x 64 7.4 / 8.9, 7.4 / 8.8, 8.7 / 11, 10 / 12: this one is faster at every one of 24 shapes, by 0.16 to 0.9.
@@ -604,10 +606,17 @@ void set_force(int v) { g_force = v; }
 // 8.9e-8 / 2.8e-8 / 4.0e-8, 2481 x 1024 1.0e-7 / 4.9e-8 / 8.3e-8, 3072 x 2048 1.04e-7 / 5.6e-8 / 8.8e-8, 2048 x 5632 1.09e-7 / 6.6e-8 /
 // 1.30e-7, 4096 x 4096 1.08e-7 / 6.4e-8 / 1.28e-7, 21888 x 4096 1.12e-7 / 7.1e-8 / 2.0e-7, 4096 x 12288 1.17e-7 / 7.8e-8 / 2.1e-7 to
 // 2.5e-7.  Hence six products up to kSixK, where five would lose more than those did; above, the sixth costs 5 to 10 % of the time.
+// At 9 to 16 sequences the other form is the mma.sync kernel.  Measured (us, binary16 input, this form / that one at 9 and at 16
+// sequences): 6144 x 4096 14.6 / 18.4, 15.2 / 20.6; 21888 x 4096 32.3 / 33.2, 32.8 / 35.7; 4096 x 10944 21 / 32, 22 / 32; 2048 x 5632 12 / 24,
+// 12 / 24; 32768 x 2048 21 / 26, 21 / 28; 2048 x 2048 8.4 / 8.7, 8.8 / 10.2; 28683 x 704 11 / 18, 11 / 18; 5558 x 736 8.4 / 8.7, 9.0 / 8.8;
+// 2481 x 1024 7.9 / 6.9, 8.4 / 7.6; 700 x 256 5.9 / 4.8, 6.1 / 5.4: the line lies at rows of 2,048 or 8 million weights.  Always six
+// products (1 to 3 % of the time), error 0.32 to 0.68 of that kernel's.  Up to eight sequences that one is faster (151,643 x 4096:
+// 114 against 127).
 constexpr int kSixK = 3072;
 bool preferred(int M, int N, int K) {
-    if (M <= 16 || !usable(cols_of(M))) return false;
+    if (M <= 8 || !usable(cols_of(M))) return false;
     if (g_force.load() != 0) return g_force.load() > 0;
+    if (M <= 16) return K >= 2048 || (long long)N * K >= 8000000;
     const int sms = sm_count(current_device()), tiles = (N + 127) / 128, nchunks = (K + kKc - 1) / kKc;
     const int ks = std::max(1, std::min(sms / tiles, nchunks));
     const int theirs = std::min(2 * (((nchunks + 1) / 2 + ks - 1) / ks), nchunks);
@@ -616,11 +625,16 @@ bool preferred(int M, int N, int K) {
     const int chain = l.csize == 0 ? nchunks : std::min(share, nchunks);
     return chain < theirs || theirs == nchunks;
 }
+// Whether a call can have its scratch: unless it would have to grow while the stream is captured.
+bool scratch_at_hand(int M, int N, int K, cudaStream_t st) {
+    const WideLayout l = layout_of(M, N, K);
+    return tc::scratch_at_hand(l.part_off + l.part_bytes, st);
+}
 // Enough for every batch up to M.
 size_t scratch_bytes(int M, int N, int K) {
-    if (M <= 16 || N < 1 || K < 32) return 0;
+    if (M <= 8 || N < 1 || K < 32) return 0;
     size_t most = 0;
-    for (int m = 32; m <= cols_of(std::min(M, 64)); m += 16) {
+    for (int m = 16; m <= cols_of(std::min(M, 64)); m += 16) {
         const WideLayout l = layout_of(m, N, K);
         most = std::max(most, l.part_off + l.part_bytes);
     }
@@ -685,6 +699,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     t.status = a.status;
     t.N = a.N; t.M = M; t.nchunks = lay.nchunks; t.tiles = lay.tiles; t.csize = lay.csize; t.six = a.K <= kSixK;
     switch (lay.NE) {
+        case 16: return launch_n<16>(map_w, t, lay.grid, st);
         case 32: return launch_n<32>(map_w, t, lay.grid, st);
         case 48: return launch_n<48>(map_w, t, lay.grid, st);
         default: return launch_n<64>(map_w, t, lay.grid, st);

@@ -35,8 +35,8 @@
 // of a chunk are consecutive, four to each half: half h of a chunk is the blocks whose index has bit 2 equal to h, and the
 // activations are laid out the same way.
 // What bounds it (65,536 x 4096): at 64 sequences the tensor pipe, 81 % busy at the 1.55 GHz that the power limit leaves (five products
-// of 64 columns take 161 cycles per k-block and group; 48 / 32 columns 121 / 83, measured); at 32 the workers' issue
-// slots (63 % used; bf16 FMAs, shifts and logic operations take two cycles of their pipes each): with one MMA in five the same
+// of 64 columns take 161 cycles per k-block and group; 48 / 32 / 16 columns 121 / 83 / 53, measured); at 32 and 16 the workers' issue
+// slots (63 % used at 32; bf16 FMAs, shifts and logic operations take two cycles of their pipes each): with one MMA in five the same
 // kernel takes 74 us of 80 there, with two thirds of the activation traffic left out 79.
 // All waits are bounded; a wait that gives up raises an abort flag.
 #pragma once

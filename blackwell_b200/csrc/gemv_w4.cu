@@ -37,6 +37,7 @@ namespace wide {  // its bf16 form, gemm_w4a8_wide.cu
 bool preferred(int M, int N, int K);
 cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st);
 size_t scratch_bytes(int M, int N, int K);
+bool scratch_at_hand(int M, int N, int K, cudaStream_t st);
 void set_split(int v);
 void set_force(int v);
 }  // namespace wide
@@ -444,6 +445,11 @@ static cudaError_t gemv_dispatch(GemvArgs a, int M, cudaStream_t st) {
         const bool forced = g_tune_mma_min.load() > 0;  // an explicit range (tests, experiments) takes the kernel as it is
         use_mma = forced || !(windows && tc_can);
     }
+    // 9 to 16 sequences of a matrix that is not small: the bf16 tcgen05 kernel (wide::preferred).  Pre-quantized input that the mma.sync
+    // kernel takes stays there, which needs no scratch memory, and so does a call that would have to grow the scratch under capture.
+    if (sizeof(WS) == 2 && M > 8 && M <= 16 && g_tune_mma_min.load() <= 0 && !a.next_q && !a.x_sumsq && (a.xkind != kXInt8 || !use_mma) &&
+        tc::eligible(a, M) && wide::preferred(M, a.N, a.K) && wide::scratch_at_hand(M, a.N, a.K, st))
+        return wide::launch(a, M, st);
     const bool use_tc = !use_mma && sizeof(WS) == 2 && M >= tc_min && tc::eligible(a, M < 64 ? M : 64);
     // From 2 sequences on, a call of a streaming kernel with an int8 prologue (f16 / f32 / RMSNorm / SwiGLU input) has
     // its activations quantized once by a small kernel instead of once per CTA; the GEMV then runs on the result as on
@@ -497,7 +503,9 @@ static cudaError_t gemv_dispatch(GemvArgs a, int M, cudaStream_t st) {
                 b.x = static_cast<const float*>(a.x) + (size_t)m0 * a.x_stride;
                 if (a.x2) b.x2 = static_cast<const float*>(a.x2) + (size_t)m0 * a.x_stride;
             }
-            cudaError_t e = wide::preferred(mc, a.N, a.K) ? wide::launch(b, mc, st) : tc::launch(b, mc, st);
+            // (the int8 form needs about half the scratch)
+            const bool bf16 = wide::preferred(std::max(mc, 9), a.N, a.K) && wide::scratch_at_hand(mc, a.N, a.K, st);
+            cudaError_t e = bf16 ? wide::launch(b, mc, st) : tc::launch(b, mc, st);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;

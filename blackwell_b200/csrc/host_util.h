@@ -83,6 +83,14 @@ public:
         return cudaSuccess;
     }
 
+    // Whether get() would hand out `bytes`, unless the allocation itself fails.
+    bool at_hand(size_t bytes, cudaStream_t st) {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (cur_[current_device()].bytes >= bytes) return true;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        return !(cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone);
+    }
+
 private:
     struct Block { unsigned char* ptr = nullptr; size_t bytes = 0; };
     Block cur_[kMaxDevices];

@@ -47,8 +47,9 @@ int bw_gemv_int4_warp(float* y_out, const void* x_packed, const float* x_scale, 
  * (passed as uint16_t bit patterns).  Extension; arithmetic follows
  * src/kernels/gemv_int8.cu:937-965 with the int8 operand of :718-748.
  * Any M >= 1.  Batch routing of all bw_gemv_w4a8* entry points (by measurement; bw_set_tuning keys 5, 13, 14 move
- * the borders): up to 4 sequences run in the streaming dp4a kernel, 5 to 16 in the streaming mma.sync kernel, more
- * than 16 (K % 32 == 0, 16-byte aligned W and x) in one of the tcgen05 kernels, 64 sequences per launch; operands the
+ * the borders): up to 4 sequences run in the streaming dp4a kernel, 5 to 8 in the streaming mma.sync kernel, 9 to 16 there
+ * too where the matrix is small (K < 2048 and K * N < 8,000,000) or the input pre-quantized, everything else from 9 sequences on
+ * (K % 32 == 0, 16-byte aligned W and x) in one of the tcgen05 kernels, 64 sequences per launch; operands the
  * tensor-core kernel cannot take fall back to passes of 16 through the mma.sync kernel (or 8 through dp4a). */
 int bw_gemv_w4a8(float* y_out, const int8_t* x_q, const float* x_scale, const uint8_t* W_packed,
                  const uint16_t* W_scale_f16, int K, int N, int M, void* stream);
@@ -507,7 +508,7 @@ int bw_peer_comm_status(void* comm, int* status_out);
 int bw_peer_comm_destroy(void* comm);
 
 /* Library-owned scratch memory.  Two kernel families keep a per-device, grow-only scratch block: the tensor-core
- * GEMV (float-input calls from 2 sequences on: activations quantized once; more than 16 sequences: prepared activations, K-split partial sums, arrival
+ * GEMV (float-input calls from 2 sequences on: activations quantized once; on the tcgen05 kernels: prepared activations, K-split partial sums, arrival
  * counters) and the allocating attention entry points (split partials, arrival counters).  A block is shared by all
  * streams of the device -- two calls of the same family must not overlap on one GPU -- and grows (cudaMalloc +
  * cudaMemset, synchronising) when a larger problem arrives; an outgrown block stays allocated until the library is

@@ -216,3 +216,46 @@ def test_error_against_64_bits(k, M, K, N, split):
     ref = oracle.gemv_w4a8_f64(xq, xs, W, sc16)
     err = np.linalg.norm(y.cpu().numpy() - ref) / np.linalg.norm(ref)
     assert err < (1e-7 if K <= 3072 else 2e-7) + (K // 256 + 2) ** 0.5 * 2.0 ** -25
+
+
+# whole tiles, clusters and shares; rows that end in either half of a chunk; scale rows of every pitch
+@pytest.mark.parametrize("M,K,N,split", [(9, 2048, 300, 0), (16, 4096, 257, 0), (12, 10944, 512, 9), (10, 5632, 2000, 2), (13, 2080, 40000, 1),
+                                         (16, 2208, 700, 9), (11, 704, 12000, 0), (75, 2048, 256, 0)])
+def test_nine_to_sixteen_sequences(k, M, K, N, split):
+    import torch
+
+    W, sc16, _ = synth.int4_weights(N, K, seed=K, full_range=True)
+    x16 = synth.activations_f16(M, K, 96)
+    xq, xs = oracle.quantize_int8(x16.astype(np.float32))
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    k.set_tuning(6, split)
+    try:
+        k.gemv_w4a8_f16in(y, to_dev(x16.view(np.uint16)), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M)
+    finally:
+        k.set_tuning(6, 0)
+    torch.cuda.synchronize()
+    assert k.device_status() == 0
+    ref = oracle.gemv_w4a8_f64(xq, xs, W, sc16)
+    # six products: the fp32 additions are all that is lost (see above)
+    assert np.linalg.norm(y.cpu().numpy() - ref) / np.linalg.norm(ref) < (K // 256 + 2) ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("M,K", [(16, 499968), (40, 119968)])
+def test_a_call_that_may_not_grow_the_scratch_is_still_taken(k, M, K):
+    """Under capture, 48 / 34 MB of prepared activations against 10 MB of quantized ones."""
+    import torch
+
+    N = 32
+    W, sc16, _ = synth.int4_weights(N, K, seed=97)
+    x16 = synth.activations_f16(M, K, 98)
+    args = [to_dev(x16.view(np.uint16)), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M]
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    k.gemv_w4a8_f16in(torch.empty((2, N), dtype=torch.float32, device="cuda"), *args[:5], 2)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        k.gemv_w4a8_f16in(y, *args)
+    g.replay()
+    torch.cuda.synchronize()
+    xq, xs = oracle.quantize_int8(x16.astype(np.float32))
+    assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
