@@ -66,7 +66,7 @@ int alloc_driver(bw_decode* d) {
     BW_TRY(zeroed(&d->gen, M * (size_t)d->max_new));
     d->at.assign(M, 0);
     if (d->model->max_portion() > 0) {
-        BW_TRY(zeroed(&d->p_tokens, d->model->max_portion()));
+        BW_TRY(zeroed(&d->p_tokens, d->model->max_group_rows()));
         BW_TRY(zeroed(&d->p_want, d->model->max_portion()));
         BW_TRY(zeroed(&d->p_one, 2));
         BW_TRY(c.alloc(&d->p_logits, (size_t)kWantRows * c.cfg.vocab));
@@ -74,13 +74,32 @@ int alloc_driver(bw_decode* d) {
     return 0;
 }
 
-// Tokens of one slot, `tokens` in device memory: portions of at most max_portion.
-int feed(bw_decode* d, int slot, const int* tokens, int n, cudaStream_t st) {
-    for (int i = 0; i < n;) {
-        const int len = std::min(n - i, d->model->max_portion());
-        BW_TRY(d->model->enqueue_portion(d->ctx, slot, d->at[slot], len, tokens + i, 0, nullptr, nullptr, st));
-        d->at[slot] += len;
-        i += len;
+// The first prompt_len[m] - 1 tokens of every slot, in passes of portions of different slots: as many rows as a pass holds, so that
+// its products fill the SMs and read the weights once.  (Two portions of one slot in a pass would not do: a layer that reads an
+// earlier layer's ring comes after that one has written both.)  `ids` holds the tokens of all passes and must outlive the copies.
+int feed_prompts(bw_decode* d, const int* prompt_ids, const int* prompt_len, int max_prompt, std::vector<int>* ids, cudaStream_t st) {
+    const int M = d->ctx.cfg.batch, cap = d->model->max_group_rows();
+    size_t total = 0;
+    for (int m = 0; m < M; ++m) total += prompt_len[m] - 1;
+    ids->reserve(total);   // the copies below read it in place
+    for (bool more = true; more;) {
+        more = false;
+        for (int m = 0; m < M;) {
+            std::vector<bw::Portion> pass;
+            const size_t first = ids->size();
+            for (; m < M; ++m) {
+                const int at = d->at[m], n = std::min(prompt_len[m] - 1 - at, d->model->max_portion());
+                if (n < 1) continue;
+                if ((int)(ids->size() - first) + n > cap) break;
+                pass.push_back({m, at, n});
+                ids->insert(ids->end(), prompt_ids + (size_t)m * max_prompt + at, prompt_ids + (size_t)m * max_prompt + at + n);
+                d->at[m] += n;
+                more |= d->at[m] < prompt_len[m] - 1;
+            }
+            if (pass.empty()) continue;
+            BW_TRY(cudaMemcpyAsync(d->p_tokens, ids->data() + first, (ids->size() - first) * 4, cudaMemcpyHostToDevice, st));
+            BW_TRY(d->model->enqueue_group(d->ctx, pass, d->p_tokens, st));
+        }
     }
     return 0;
 }
@@ -147,8 +166,8 @@ extern "C" int bw_decode_begin(bw_decode* d, const int* prompt_ids, const int* p
     BW_TRY(cudaMemcpyAsync(d->prompt_len, prompt_len, (size_t)M * 4, cudaMemcpyHostToDevice, st));
     BW_TRY(cudaMemsetAsync(d->gen, 0xFF, (size_t)M * d->max_new * 4, st));  // -1 = not generated
     d->at.assign(M, 0);
-    if (portions)   // everything but the last prompt token, which the first step takes
-        for (int m = 0; m < M; ++m) BW_TRY(feed(d, m, d->prompt + (size_t)m * d->max_prompt, prompt_len[m] - 1, st));
+    std::vector<int> ids;
+    if (portions) BW_TRY(feed_prompts(d, prompt_ids, prompt_len, max_prompt, &ids, st));   // all but the last, which the first step takes
     BW_TRY(cudaMemcpyAsync(d->ctx.pos, d->at.data(), (size_t)M * 4, cudaMemcpyHostToDevice, st));
     return (int)cudaStreamSynchronize(st);  // the pageable host buffers above must outlive the copies
 }

@@ -44,6 +44,11 @@ struct DecodeContext {
     }
 };
 
+// Consecutive tokens of the sequence in `slot`, from position pos0 on.
+struct Portion {
+    int slot, pos0, n;
+};
+
 class DecodeModel {
 public:
     virtual ~DecodeModel() {}
@@ -61,6 +66,9 @@ public:
     virtual int enqueue_portion(DecodeContext&, int, int, int, const int*, int, const int*, float*, cudaStream_t) {
         return cudaErrorNotSupported;
     }
+    // Portions of different slots in one pass, max_group_rows() tokens at the most; tokens: theirs one after the other.
+    virtual int max_group_rows() const { return max_portion(); }
+    virtual int enqueue_group(DecodeContext&, const std::vector<Portion>&, const int*, cudaStream_t) { return cudaErrorNotSupported; }
     virtual void caches(uint16_t** k, uint16_t** v) { *k = *v = nullptr; }
 };
 

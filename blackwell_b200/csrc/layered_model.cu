@@ -118,8 +118,15 @@ struct Work {
     long ldx = 0;
 };
 
+// Rows of one sequence (or one row of each, a token step) among the rows of a pass, from row0 on.  Products and norms take all
+// rows of a pass at once, what runs along a sequence takes a span.
+struct Span {
+    int row0;
+    lm::Rows r;
+};
+
 struct Env {   // fixed properties of an engine
-    int f32 = 0, slots = 0, max_seq = 0, max_rows = 0, width = 0, sms = 148;
+    int f32 = 0, slots = 0, max_seq = 0, max_rows = 0, pass_rows = 0, width = 0, sms = 148;   // rows: of a span, of a pass
     float eps = 0;
     int elem() const { return f32 ? 4 : 2; }
     char* at(void* base, long elems) const { return static_cast<char*>(base) + elems * elem(); }
@@ -139,7 +146,7 @@ public:
     virtual ~Mixer() {}
     virtual int load(Loader& l, const std::string& p, int width) = 0;
     virtual int alloc(DecodeContext& ctx, const Env& e, Work* w) = 0;   // per-slot state; raises the work sizes
-    virtual int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) = 0;   // w.xb -> w.mixed_b
+    virtual int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) = 0;   // w.xb -> w.mixed_b
     int mixed_ld() const { return s_.heads * pad8(s_.vdim); }
     const Mat& out() const { return o_; }
     const MixerSpec& spec() const { return s_; }
@@ -147,6 +154,18 @@ public:
     void set_rotation(const float2* cs) { cs_ = cs; }
 
 protected:
+    // The buffers from a span's first row on; row lengths of the projection, its fp32 part and the convolved part.
+    Work from(const Env& e, const Work& w, int row, long proj, long proj32, long conv) const {
+        Work v = w;
+        v.proj_b = e.at(w.proj_b, row * proj);
+        v.proj32_b = w.proj32_b + row * proj32;
+        v.conv_b = e.at(w.conv_b, row * conv);
+        v.mixed_b = e.at(w.mixed_b, (long)row * mixed_ld());
+        v.o32_b = w.o32_b + (long)row * mixed_ld();
+        v.log_decay = w.log_decay + (long)row * s_.heads;
+        v.weight = w.weight + (long)row * s_.heads;
+        return v;
+    }
     MixerSpec s_;
     Mat in_, o_;
     const float2* cs_ = nullptr;
@@ -212,30 +231,31 @@ public:
         BW_TRY(ctx.alloc(&ring_, (size_t)e.slots * s_.conv * (s_.heads * s_.vdim + 2 * s_.groups * s_.state)));
         return alloc_recurrent(ctx, e, w);
     }
-    int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) override {
+    int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
+        const int inner8 = mixed_ld();
+        BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, split_, w.proj32_b, s_.heads, split_, st));
+        for (const Span& s : spans) BW_TRY(mix(e, from(e, w, s.row0, split_, s_.heads, split_ - inner8), s.r, st));
+        return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, T, s_.heads, s_.vdim, s_.norm_groups, 1, e.eps,
+                              e.f32, st);
+    }
+
+private:
+    int mix(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) const {
         const int inner8 = mixed_ld(), bc = s_.groups * pad8(s_.state);
-        BW_TRY(project(e, w, in_, w.xb, w.ldx, r.T, w.proj_b, split_, w.proj32_b, s_.heads, split_, st));
         lm::ConvArgs c{};
         c.u = w.proj_b; c.ldu = split_; c.w = conv_w_; c.bias = conv_b_; c.ring = ring_; c.taps = s_.conv; c.heads = s_.heads;
         c.V = s_.vdim; c.N = s_.state; c.groups = s_.groups; c.off = inner8; c.out = w.conv_b; c.ldo = split_ - inner8;
         c.dt_raw = w.proj32_b; c.ld_dt = s_.heads; c.dt_bias = dt_bias_; c.A_log = A_log_; c.log_decay = w.log_decay; c.weight = w.weight;
         lm::RecurrenceArgs a = recurrence(w);
         a.groups = s_.groups; a.D = D_;
-        if (r.row_slot) {
-            BW_TRY(lm::recurrence_step(a, &c, r, e.f32, st));
-        } else {
-            BW_TRY(lm::conv_silu(c, r, e.f32, st));
-            BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
-            a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + bc);
-            a.ldq = a.ldk = a.ldv = c.ldo;
-            a.log_decay = w.log_decay; a.weight = w.weight;
-            BW_TRY(recur(e, a, r, st));
-        }
-        return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, r.T, s_.heads, s_.vdim, s_.norm_groups, 1, e.eps,
-                              e.f32, st);
+        if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
+        BW_TRY(lm::conv_silu(c, r, e.f32, st));
+        BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
+        a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + bc);
+        a.ldq = a.ldk = a.ldv = c.ldo;
+        a.log_decay = w.log_decay; a.weight = w.weight;
+        return recur(e, a, r, st);
     }
-
-private:
     int split_ = 0;
     float *conv_w_ = nullptr, *conv_b_ = nullptr, *dt_bias_ = nullptr, *A_log_ = nullptr, *D_ = nullptr, *norm_ = nullptr, *ring_ = nullptr;
 };
@@ -265,17 +285,20 @@ public:
         w->proj = std::max(w->proj, (long)in_.N);
         return alloc_recurrent(ctx, e, w);
     }
-    int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) override {
+    int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         const int qk8 = s_.heads * pad8(s_.dim), v8 = mixed_ld();
-        BW_TRY(project(e, w, in_, w.xb, w.ldx, r.T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
-        lm::RecurrenceArgs a = recurrence(w);
-        a.groups = s_.heads;
-        a.q = w.proj_b; a.k = e.at(w.proj_b, qk8); a.v = e.at(w.proj_b, 2L * qk8);
-        a.ldq = a.ldk = a.ldv = in_.N;
-        a.head_log_decay = log_decay_;
-        a.const_weight = (float)(1.0 / sqrt((double)s_.dim));
-        BW_TRY(recur(e, a, r, st));
-        return lm::gated_norm(w.mixed_b, v8, w.o32_b, v8, e.at(w.proj_b, 2L * qk8 + v8), in_.N, nullptr, r.T, s_.heads, s_.vdim, s_.heads, 0,
+        BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
+        for (const Span& s : spans) {
+            const Work v = from(e, w, s.row0, in_.N, 0, 0);
+            lm::RecurrenceArgs a = recurrence(v);
+            a.groups = s_.heads;
+            a.q = v.proj_b; a.k = e.at(v.proj_b, qk8); a.v = e.at(v.proj_b, 2L * qk8);
+            a.ldq = a.ldk = a.ldv = in_.N;
+            a.head_log_decay = log_decay_;
+            a.const_weight = (float)(1.0 / sqrt((double)s_.dim));
+            BW_TRY(recur(e, a, s.r, st));
+        }
+        return lm::gated_norm(w.mixed_b, v8, w.o32_b, v8, e.at(w.proj_b, 2L * qk8 + v8), in_.N, nullptr, T, s_.heads, s_.vdim, s_.heads, 0,
                               e.eps, e.f32, st);
     }
 
@@ -322,29 +345,30 @@ public:
         BW_TRY(ctx.alloc(&ring_, (size_t)e.slots * s_.conv * (s_.heads * s_.vdim + 2 * s_.kv_heads * s_.dim)));
         return alloc_recurrent(ctx, e, w);
     }
-    int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) override {
+    int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
+        const int H = s_.heads, inner8 = mixed_ld();
+        BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, split_, w.proj32_b, 2 * H, split_, st));
+        for (const Span& s : spans) BW_TRY(mix(e, from(e, w, s.row0, split_, 2 * H, split_ - inner8), s.r, st));
+        return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, T, H, s_.vdim, H, 0, e.eps, e.f32, st);
+    }
+
+private:
+    int mix(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) const {
         const int H = s_.heads, inner8 = mixed_ld(), qk8 = s_.kv_heads * pad8(s_.dim);
-        BW_TRY(project(e, w, in_, w.xb, w.ldx, r.T, w.proj_b, split_, w.proj32_b, 2 * H, split_, st));
         lm::ConvArgs c{};
         c.u = w.proj_b; c.ldu = split_; c.w = conv_w_; c.ring = ring_; c.taps = s_.conv; c.heads = H; c.V = s_.vdim; c.N = s_.dim;
         c.groups = s_.kv_heads; c.off = inner8; c.out = w.conv_b; c.ldo = split_ - inner8; c.dt_raw = w.proj32_b; c.ld_dt = 2 * H;
         c.beta_raw = w.proj32_b + H; c.dt_bias = dt_bias_; c.A_log = A_log_; c.log_decay = w.log_decay; c.weight = w.weight;
         lm::RecurrenceArgs a = recurrence(w);
         a.groups = s_.kv_heads; a.delta = 1; a.unit_eps = 1e-6f; a.q_scale = (float)(1.0 / sqrt((double)s_.dim)); a.chunk_scratch = w.chunk_b;
-        if (r.row_slot) {
-            BW_TRY(lm::recurrence_step(a, &c, r, e.f32, st));
-        } else {
-            BW_TRY(lm::conv_silu(c, r, e.f32, st));
-            BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
-            a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + qk8);
-            a.ldq = a.ldk = a.ldv = c.ldo;
-            a.log_decay = w.log_decay; a.weight = w.weight;
-            BW_TRY(recur(e, a, r, st));
-        }
-        return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, r.T, H, s_.vdim, H, 0, e.eps, e.f32, st);
+        if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
+        BW_TRY(lm::conv_silu(c, r, e.f32, st));
+        BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
+        a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + qk8);
+        a.ldq = a.ldk = a.ldv = c.ldo;
+        a.log_decay = w.log_decay; a.weight = w.weight;
+        return recur(e, a, r, st);
     }
-
-private:
     int split_ = 0;
     float *conv_w_ = nullptr, *dt_bias_ = nullptr, *A_log_ = nullptr, *norm_ = nullptr, *ring_ = nullptr;
 };
@@ -391,19 +415,23 @@ public:
         cache_ = c;
         return 0;
     }
-    int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) override {
-        BW_TRY(project(e, w, in_, w.xb, w.ldx, r.T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
-        lm::DiffAttnArgs a = base(e);
-        const DiffAttention* own = owner_ ? owner_ : this;
-        a.cache = own->cache_; a.cap = own->cap_; a.slots = e.slots;
-        a.q = w.proj_b; a.ld = in_.N;
-        if (!owner_) {
-            a.k = e.at(w.proj_b, k_);
-            a.v = e.at(w.proj_b, v_);
+    int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
+        BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
+        for (const Span& s : spans) {
+            const Work v = from(e, w, s.row0, in_.N, 0, 0);
+            lm::DiffAttnArgs a = base(e);
+            const DiffAttention* own = owner_ ? owner_ : this;
+            a.cache = own->cache_; a.cap = own->cap_; a.slots = e.slots;
+            a.q = v.proj_b; a.ld = in_.N;
+            if (!owner_) {
+                a.k = e.at(v.proj_b, k_);
+                a.v = e.at(v.proj_b, v_);
+            }
+            a.out = v.mixed_b; a.ldout = mixed_ld();
+            a.splits = lm::diff_attention_splits(a, s.r.T, e.f32);
+            BW_TRY(lm::diff_attention(a, s.r, e.f32, st));
         }
-        a.out = w.mixed_b; a.ldout = mixed_ld();
-        a.splits = lm::diff_attention_splits(a, r.T, e.f32);
-        return lm::diff_attention(a, r, e.f32, st);
+        return 0;
     }
     bool rotates() const override { return true; }
 
@@ -469,18 +497,22 @@ public:
         cache_ = c;
         return 0;
     }
-    int run(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) override {
+    int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         const int ld32 = in_.N - split_;
-        BW_TRY(project(e, w, in_, w.xb, w.ldx, r.T, w.proj_b, split_, w.proj32_b, ld32, split_, st));
-        lm::LatentArgs a = base(e);
-        a.q = w.proj_b; a.ldq = split_; a.ld32 = ld32;
-        a.dkv = owner_ ? nullptr : w.proj32_b;
-        a.gate = w.proj32_b + (owner_ ? 0 : s_.kv_rank + s_.rot_dim);
-        a.dkv_norm = dkv_norm_; a.Wkv = kv_.p; a.ldw = kv_.ld; a.sink = sink_; a.out = w.mixed_b; a.ldout = mixed_ld();
-        a.cache = owner_ ? owner_->cache_ : cache_;
-        a.qabs = w.qabs_b; a.part = w.part_b; a.kv = w.kv_b; a.splits = splits(e, r.T);
-        if (expanded_ && !r.row_slot && r.T > kAbsorbedRows) return lm::latent_expanded(a, r, st);
-        return lm::latent_absorbed(a, r, e.f32, st);
+        BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, split_, w.proj32_b, ld32, split_, st));
+        for (const Span& s : spans) {
+            const Work v = from(e, w, s.row0, split_, ld32, 0);
+            lm::LatentArgs a = base(e);
+            a.q = v.proj_b; a.ldq = split_; a.ld32 = ld32;
+            a.dkv = owner_ ? nullptr : v.proj32_b;
+            a.gate = v.proj32_b + (owner_ ? 0 : s_.kv_rank + s_.rot_dim);
+            a.dkv_norm = dkv_norm_; a.Wkv = kv_.p; a.ldw = kv_.ld; a.sink = sink_; a.out = v.mixed_b; a.ldout = mixed_ld();
+            a.cache = owner_ ? owner_->cache_ : cache_;
+            a.qabs = w.qabs_b; a.part = w.part_b; a.kv = w.kv_b; a.splits = splits(e, s.r.T);
+            if (expanded_ && !s.r.row_slot && s.r.T > kAbsorbedRows) BW_TRY(lm::latent_expanded(a, s.r, st));
+            else BW_TRY(lm::latent_absorbed(a, s.r, e.f32, st));
+        }
+        return 0;
     }
     bool rotates() const override { return true; }
 
@@ -521,16 +553,28 @@ public:
                        cudaStream_t st) override {
         lm::Rows r{};
         r.T = rows; r.row_slot = slots; r.row_pos = pos;
-        BW_TRY(enqueue_layers(ctx, r, tokens, st));
+        BW_TRY(enqueue_layers(ctx, rows, {{0, r}}, tokens, st));
         return head(rows, nullptr, logits, st);
     }
     int max_portion() const override { return env_.max_rows; }
+    int max_group_rows() const override { return env_.pass_rows; }
+    int enqueue_group(DecodeContext& ctx, const std::vector<Portion>& portions, const int* tokens, cudaStream_t st) override {
+        std::vector<Span> spans;
+        int rows = 0;
+        for (const Portion& p : portions) {
+            lm::Rows r{};
+            r.T = p.n; r.slot = p.slot; r.pos0 = p.pos0;
+            spans.push_back({rows, r});
+            rows += p.n;
+        }
+        return enqueue_layers(ctx, rows, spans, tokens, st);
+    }
     int enqueue_portion(DecodeContext& ctx, int slot, int pos0, int n, const int* tokens, int n_want, const int* want, float* logits,
                         cudaStream_t st) override {
         if (n > 0) {
             lm::Rows r{};
             r.T = n; r.slot = slot; r.pos0 = pos0;
-            BW_TRY(enqueue_layers(ctx, r, tokens, st));
+            BW_TRY(enqueue_layers(ctx, n, {{0, r}}, tokens, st));
         }
         for (int i = 0; i < n_want; i += kLogitRows)
             BW_TRY(head(std::min(kLogitRows, n_want - i), want + i, logits + (size_t)i * spec_.vocab, st));
@@ -538,7 +582,7 @@ public:
     }
 
 private:
-    int enqueue_layers(DecodeContext& ctx, const lm::Rows& r, const int* tokens, cudaStream_t st);
+    int enqueue_layers(DecodeContext& ctx, int T, const std::vector<Span>& spans, const int* tokens, cudaStream_t st);
     int head(int rows, const int* want, float* logits, cudaStream_t st) {
         BW_TRY(lm::norm_rows(w_.fin_b, w_.ldx, x_, final_norm_, want, rows, env_.width, env_.eps, env_.f32, st));
         lm::LinearArgs a{};
@@ -569,7 +613,11 @@ int LayeredModel::load(DecodeContext& ctx, const std::string& dir) {
     env_.width = spec_.width;
     env_.eps = (float)spec_.eps;
     env_.sms = sm_count(current_device());
-    env_.max_rows = std::min(c.max_seq, c.max_portion > 0 ? c.max_portion : env_.f32 ? 512 : 4096);
+    const int most = env_.f32 ? 512 : 4096;
+    env_.max_rows = std::min(c.max_seq, c.max_portion > 0 ? c.max_portion : most);
+    // Prompts that begin together share a pass: its products have the rows of all of them (a caller that bounds the portions bounds
+    // the work buffers).
+    env_.pass_rows = c.max_portion > 0 ? env_.max_rows : (int)std::max<long>(env_.max_rows, std::min<long>((long)c.batch * env_.max_rows, most));
     Loader l(ctx);
     if (!l.st.open(dir + "/model.safetensors", &ctx.error)) return -1;
     BW_TRY(l.matrix("embed", spec_.vocab, spec_.width, &embed_));
@@ -640,7 +688,7 @@ int LayeredModel::alloc_state(DecodeContext& ctx) {
         BW_TRY(L.mixer->alloc(ctx, env_, &w_));
         w_.ff = std::max(w_.ff, (long)pad8(L.ff));
     }
-    const size_t rows = std::max(env_.max_rows, env_.slots), el = env_.elem();
+    const size_t rows = std::max(env_.pass_rows, env_.slots), el = env_.elem();
     w_.ldx = pad8(env_.width);
     auto act = [&](void** p, size_t elems) {
         char* c = nullptr;
@@ -671,31 +719,31 @@ int LayeredModel::alloc_state(DecodeContext& ctx) {
     return ctx.alloc(&ctx.logits, (size_t)env_.slots * spec_.vocab);
 }
 
-int LayeredModel::enqueue_layers(DecodeContext& ctx, const lm::Rows& r, const int* tokens, cudaStream_t st) {
+int LayeredModel::enqueue_layers(DecodeContext& ctx, int T, const std::vector<Span>& spans, const int* tokens, cudaStream_t st) {
     const Env& e = env_;
-    BW_TRY(lm::embed(x_, w_.xb, w_.ldx, embed_.p, embed_.ld, tokens, r.T, e.width, spec_.vocab, (float)spec_.embed_scale, layers_[0].in1,
+    BW_TRY(lm::embed(x_, w_.xb, w_.ldx, embed_.p, embed_.ld, tokens, T, e.width, spec_.vocab, (float)spec_.embed_scale, layers_[0].in1,
                      e.eps, e.f32, st));
     for (size_t i = 0; i < layers_.size(); ++i) {
         Layer& L = layers_[i];
         const float* next = i + 1 < layers_.size() ? layers_[i + 1].in1 : nullptr;   // the next layer's input norm
         lm::LinearArgs a{};
-        a.T = r.T; a.f32 = e.f32; a.y = w_.sub; a.ldy = e.width; a.y_f32 = 1; a.N = a.split = e.width;
-        BW_TRY(L.mixer->run(e, w_, r, st));
+        a.T = T; a.f32 = e.f32; a.y = w_.sub; a.ldy = e.width; a.y_f32 = 1; a.N = a.split = e.width;
+        BW_TRY(L.mixer->run(e, w_, T, spans, st));
         const Mat& o = L.mixer->out();
         a.x = w_.mixed_b; a.ldx = L.mixer->mixed_ld(); a.W = o.p; a.ldw = o.ld; a.K = o.K;
         BW_TRY(lm::linear(a, st));
-        BW_TRY(lm::norm_add(x_, w_.xb, w_.ldx, w_.sub, L.out1, L.ff > 0 ? L.in2 : next, r.T, e.width, e.eps, e.f32, st));
+        BW_TRY(lm::norm_add(x_, w_.xb, w_.ldx, w_.sub, L.out1, L.ff > 0 ? L.in2 : next, T, e.width, e.eps, e.f32, st));
         if (L.ff > 0) {
             lm::LinearArgs g{};
-            g.x = w_.xb; g.ldx = w_.ldx; g.W = L.gu.p; g.ldw = L.gu.ld; g.T = r.T; g.N = g.split = L.gu.N; g.K = L.gu.K;
+            g.x = w_.xb; g.ldx = w_.ldx; g.W = L.gu.p; g.ldw = L.gu.ld; g.T = T; g.N = g.split = L.gu.N; g.K = L.gu.K;
             g.y = w_.ff_b; g.ldy = pad8(L.ff); g.epi = lm::kEpiSwiglu; g.f32 = e.f32;
             BW_TRY(lm::linear(g, st));
             a.x = w_.ff_b; a.ldx = pad8(L.ff); a.W = L.down.p; a.ldw = L.down.ld; a.K = L.down.K;
             BW_TRY(lm::linear(a, st));
-            BW_TRY(lm::norm_add(x_, w_.xb, w_.ldx, w_.sub, L.out2, next, r.T, e.width, e.eps, e.f32, st));
+            BW_TRY(lm::norm_add(x_, w_.xb, w_.ldx, w_.sub, L.out2, next, T, e.width, e.eps, e.f32, st));
         }
         if (ctx.watch)
-            BW_TRY(cudaMemcpyAsync(ctx.watch + ((size_t)i * ctx.watch_rows + ctx.watch_row0) * e.width, x_, (size_t)r.T * e.width * 4,
+            BW_TRY(cudaMemcpyAsync(ctx.watch + ((size_t)i * ctx.watch_rows + ctx.watch_row0) * e.width, x_, (size_t)T * e.width * 4,
                                    cudaMemcpyDeviceToDevice, st));
     }
     return 0;
