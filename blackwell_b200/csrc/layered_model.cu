@@ -250,7 +250,6 @@ private:
         a.groups = s_.groups; a.D = D_;
         if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
         BW_TRY(lm::conv_silu(c, r, e.f32, st));
-        BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
         a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + bc);
         a.ldq = a.ldk = a.ldv = c.ldo;
         a.log_decay = w.log_decay; a.weight = w.weight;
@@ -363,7 +362,6 @@ private:
         a.groups = s_.kv_heads; a.delta = 1; a.unit_eps = 1e-6f; a.q_scale = (float)(1.0 / sqrt((double)s_.dim)); a.chunk_scratch = w.chunk_b;
         if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
         BW_TRY(lm::conv_silu(c, r, e.f32, st));
-        BW_TRY(lm::conv_ring_store(c, r, e.f32, st));
         a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + qk8);
         a.ldq = a.ldk = a.ldv = c.ldo;
         a.log_decay = w.log_decay; a.weight = w.weight;

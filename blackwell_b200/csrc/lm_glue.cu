@@ -338,64 +338,113 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(const ConvArgs c, const 
     }
 }
 
-// bf16 prompts and few taps: a thread walks down 16 rows of eight columns (always of one head block) with the last inputs in
-// registers.
-constexpr int kConvWalk = 16;
+// bf16 prompts and few taps: a thread takes eight rows of eight columns (always of one head block) and requests all it reads before
+// it computes; taps and bias come before the dependency wait.  The last columns of blocks take the step sizes, a thread per row and
+// head; the threads of the first rows, which alone read the ring, also store the last inputs there.  Serial chains bounded this: a
+// thread that walked down 16 rows, its loads held back by its stores, and one that went through 16 step sizes took 22 us at 249 rows
+// and 27 at 1,002 (4,352 / 8,192 columns), 67 at 4,096, the ring another 4; now 15 at 249, 18 at
+// 1,002, 41 at 4,096, ring included (four rows a thread: the same).  Four prompts that begin together 2449 -> 2338 us.
+constexpr int kConvRun = 8;
 template <int TAPS>
-__global__ void __launch_bounds__(128) conv_walk_kernel(const ConvArgs c, const Rows r) {
-    pdl_wait();
-    const int channels = c.heads * c.V + 2 * c.groups * c.N, vecs = conv_cols(c) / 8;
-    const int vec = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * kConvWalk, t1 = min(r.T, t0 + kConvWalk);
-    if (vec >= vecs) {
-        if (vec < vecs + c.heads) step_sizes(c, vec - vecs, t0, t1);
+__global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const Rows r) {
+    const int channels = c.heads * c.V + 2 * c.groups * c.N, vec = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * kConvRun;
+    const int steps = (conv_cols(c) / 8 + 127) / 128;
+    if (blockIdx.x >= steps) {
+        const int i = (blockIdx.x - steps) * 128 + threadIdx.x, t = t0 + i / c.heads;
+        pdl_wait();
+        if (i < kConvRun * c.heads && t < r.T) step_sizes(c, i % c.heads, t, t + 1);
         return;
     }
-    const bf16* u = static_cast<const bf16*>(c.u) + c.off + vec * 8;
-    bf16* out = static_cast<bf16*>(c.out) + vec * 8;
-    auto unpack = [](const uint4& v, float (&x)[8]) {
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    if (vec >= conv_cols(c) / 8) return;
+    const int first = conv_channel(c, vec * 8);
+    const bool whole = first >= 0 && conv_channel(c, vec * 8 + 7) == first + 7;   // no padding column
+    float w[8 * TAPS], bias[8];   // w[e * TAPS + j]
+    if (whole && ((uintptr_t)(c.w + (long)first * TAPS) & 15) == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            x[2 * i] = __uint_as_float(w[i] << 16);
-            x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-        }
-    };
-    float w[TAPS][8], bias[8], win[TAPS][8];   // win[i]: the input TAPS - 1 - i rows back
+        for (int i = 0; i < 2 * TAPS; ++i)
+            *reinterpret_cast<float4*>(w + 4 * i) = __ldg(reinterpret_cast<const float4*>(c.w + (long)first * TAPS) + i);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const int ch = conv_channel(c, vec * 8 + e);   // padding columns: zero weights, zero output
-        bias[e] = ch >= 0 && c.bias ? c.bias[ch] : 0.f;
+        for (int e = 0; e < 8; ++e) bias[e] = c.bias ? __ldg(c.bias + first + e) : 0.f;
+    } else {   // padding columns: zero weights, zero output
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) w[j][e] = ch >= 0 ? c.w[ch * TAPS + j] : 0.f;
+        for (int e = 0; e < 8; ++e) {
+            const int ch = conv_channel(c, vec * 8 + e);
+            bias[e] = ch >= 0 && c.bias ? c.bias[ch] : 0.f;
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j) {
-            const int s = t0 - (TAPS - 1) + j, p = r.pos0 + s;
-            float v = 0.f;
-            if (s >= 0) v = to_f(u[(long)s * c.ldu + e]);
-            else if (p >= 0 && ch >= 0) v = c.ring[((long)r.slot * TAPS + p % TAPS) * channels + ch];
-            win[j][e] = v;
+            for (int j = 0; j < TAPS; ++j) w[e * TAPS + j] = ch >= 0 ? c.w[ch * TAPS + j] : 0.f;
         }
     }
-#pragma unroll 4
-    for (int t = t0; t < t1; ++t) {
-        unpack(*reinterpret_cast<const uint4*>(u + (long)t * c.ldu), win[TAPS - 1]);
+    pdl_wait();
+    const bf16* u = static_cast<const bf16*>(c.u) + c.off + vec * 8;
+    bf16* out = static_cast<bf16*>(c.out) + vec * 8;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 x[TAPS - 1 + kConvRun], last[TAPS - 1];   // rows t0 - (TAPS - 1) ..; what the ring gets
+#pragma unroll
+    for (int i = 0; i < TAPS - 1 + kConvRun; ++i) {
+        const int t = t0 - (TAPS - 1) + i;
+        x[i] = t >= 0 && t < r.T ? __ldg(reinterpret_cast<const uint4*>(u + (long)t * c.ldu)) : zero;
+    }
+    auto unpack = [](const uint4& v, float (&f)[8]) {
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[2 * i] = __uint_as_float(q[i] << 16);
+            f[2 * i + 1] = __uint_as_float(q[i] & 0xFFFF0000u);
+        }
+    };
+    if (t0 == 0) {
+        float* ring = c.ring + (long)r.slot * TAPS * channels;
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i)   // (there are more rows than taps)
+            last[i] = __ldg(reinterpret_cast<const uint4*>(u + (long)(r.T - (TAPS - 1) + i) * c.ldu));
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i) {
+            const int p = r.pos0 - (TAPS - 1) + i;
+            if (p < 0) continue;
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int ch = whole ? first + e : conv_channel(c, vec * 8 + e);
+                f[e] = ch >= 0 ? ring[(long)(p % TAPS) * channels + ch] : 0.f;   // a bf16 number
+            }
+            x[i] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        }
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i) {
+            float f[8];
+            unpack(last[i], f);
+            const int at = (r.pos0 + r.T - (TAPS - 1) + i) % TAPS;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int ch = whole ? first + e : conv_channel(c, vec * 8 + e);
+                if (ch >= 0) ring[(long)at * channels + ch] = f[e];
+            }
+        }
+    }
+    float win[TAPS][8];   // win[i]: the input TAPS - 1 - i rows back
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j) unpack(x[j], win[j]);
+#pragma unroll
+    for (int i = 0; i < kConvRun; ++i) {
+        if (t0 + i >= r.T) break;
+        unpack(x[TAPS - 1 + i], win[TAPS - 1]);
         float y[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             y[e] = bias[e];
 #pragma unroll
-            for (int j = 0; j < TAPS; ++j) y[e] = fmaf(w[j][e], win[j][e], y[e]);
+            for (int j = 0; j < TAPS; ++j) y[e] = fmaf(w[e * TAPS + j], win[j][e], y[e]);
             y[e] = __fdividef(y[e], 1.0f + __expf(-y[e]));
 #pragma unroll
             for (int j = 0; j < TAPS - 1; ++j) win[j][e] = win[j + 1][e];
         }
-        *reinterpret_cast<uint4*>(out + (long)t * c.ldo) =
+        *reinterpret_cast<uint4*>(out + (long)(t0 + i) * c.ldo) =
             make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
     }
 }
 template <int TAPS>
-cudaError_t conv_walk(const ConvArgs& c, const Rows& r, cudaStream_t st) {
-    return launch_pdl(conv_walk_kernel<TAPS>, dim3((conv_cols(c) / 8 + c.heads + 127) / 128, (r.T + kConvWalk - 1) / kConvWalk), dim3(128), 0, st, c, r);
+cudaError_t conv_run(const ConvArgs& c, const Rows& r, cudaStream_t st) {
+    return launch_pdl(conv_run_kernel<TAPS>, dim3((conv_cols(c) / 8 + 127) / 128 + (kConvRun * c.heads + 127) / 128, (r.T + kConvRun - 1) / kConvRun), dim3(128), 0, st, c, r);
 }
 
 template <typename A>
@@ -512,20 +561,17 @@ cudaError_t gated_norm(void* out, long ldout, const float* o, long ldo, const vo
 
 cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st) {
     const int n = conv_cols(c) + c.heads;
-    const dim3 grid((n + 127) / 128, (r.T + kConvRows - 1) / kConvRows), block(128);
+    const dim3 grid((n + 127) / 128, (r.T + kConvRows - 1) / kConvRows), ring((conv_cols(c) + 127) / 128), block(128);
     count_launch(1);
-    if (!f32 && r.T >= kConvWalk) {
-        if (c.taps == 2) return conv_walk<2>(c, r, st);
-        if (c.taps == 3) return conv_walk<3>(c, r, st);
-        if (c.taps == 4) return conv_walk<4>(c, r, st);
+    if (!f32 && r.T >= 16) {
+        if (c.taps == 2) return conv_run<2>(c, r, st);
+        if (c.taps == 3) return conv_run<3>(c, r, st);
+        if (c.taps == 4) return conv_run<4>(c, r, st);
     }
-    return f32 ? launch_pdl(conv_silu_kernel<float>, grid, block, 0, st, c, r) : launch_pdl(conv_silu_kernel<bf16>, grid, block, 0, st, c, r);
-}
-
-cudaError_t conv_ring_store(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st) {
-    const dim3 grid((conv_cols(c) + 127) / 128), block(128);
+    const cudaError_t e = f32 ? launch_pdl(conv_silu_kernel<float>, grid, block, 0, st, c, r) : launch_pdl(conv_silu_kernel<bf16>, grid, block, 0, st, c, r);
+    if (e != cudaSuccess) return e;
     count_launch(1);
-    return f32 ? launch_pdl(conv_ring_kernel<float>, grid, block, 0, st, c, r) : launch_pdl(conv_ring_kernel<bf16>, grid, block, 0, st, c, r);
+    return f32 ? launch_pdl(conv_ring_kernel<float>, ring, block, 0, st, c, r) : launch_pdl(conv_ring_kernel<bf16>, ring, block, 0, st, c, r);
 }
 
 }  // namespace lm

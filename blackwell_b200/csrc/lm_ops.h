@@ -79,8 +79,7 @@ struct ConvArgs {
     const float* beta_raw;           // [T][ld_dt] or NULL: the weight is sigmoid(beta_raw) instead of the step size
     float *log_decay, *weight;       // [T][heads]
 };
-cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st);     // several rows of one sequence
-cudaError_t conv_ring_store(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st);  // after conv_silu
+cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st);     // several rows of one sequence, then the ring
 
 // ---------------------------------------------------------------- gated linear recurrence
 //   S_t = exp(log_decay_t) S_(t-1) + weight_t k_t v_t^T,   o_t = S_t^T q_t + D v_t        (per head; S is N x V, fp32)
