@@ -15,6 +15,7 @@
 #include <float.h>
 #include <stdio.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "../../include/blackwell_b200.h"
@@ -29,6 +30,9 @@ namespace bw {
 constexpr int kHd = 128;
 constexpr int kAttnWarps = 4;
 constexpr int kPosPerStep = 4;  // positions handled together by one warp
+constexpr int kClusterSplits = 8;   // splits that merge as a cluster, at most
+__host__ __device__ constexpr int attn_bufs(int warps) { return warps == 4 ? 2 : 3; }   // tiles of a warp in shared memory
+constexpr int kManyWarps = 8;   // warps of its CTA where there is no more than one per SM
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 load4(const __half* p) {
@@ -275,13 +279,50 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_split_kernel(cons
     if (a.nsplit > 1 && a.tickets) last_arriver_merge<GQ>(a, m, kvh, h0, &s_last);
 }
 
-// Tensor-core variant for the binary16 cache (see attention_mma.cuh): same grid, same splits, same partial records
-// and arrival counters as the scalar kernel above.
+// The splits of a (sequence, kv head) as the CTAs of a cluster: rank r merges heads r, r + nsplit, ... from the shared memory of all, the
+// first 128 threads a dimension each.  `o` [GQ][128], `ms` [GQ] (max, sum): this CTA's record.  Called by all threads after a block barrier.
 template <int GQ>
-__global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_mma_kernel(const AttnArgs a) {
+__device__ __forceinline__ void cluster_merge(const AttnArgs& a, int m, int h0, int rank, const float* o, const float2* ms) {
+    cluster_sync_all();   // every CTA's record is in its shared memory
+    const int d = threadIdx.x, nsplit = a.nsplit;
+    for (int h = rank; h < GQ && d < kHd; h += nsplit) {   // (whole warps)
+        float mx[kClusterSplits], ls[kClusterSplits], v[kClusterSplits];
+        const uint32_t at = smem_u32(ms + h), ov = smem_u32(o + h * kHd + d);
+#pragma unroll
+        for (int c = 0; c < kClusterSplits; ++c) {
+            mx[c] = c < nsplit ? ld_dsmem(at, c) : -FLT_MAX;
+            ls[c] = c < nsplit ? ld_dsmem(at + 4, c) : 0.f;
+            v[c] = c < nsplit ? ld_dsmem(ov, c) : 0.f;
+        }
+        float mall = -FLT_MAX, lsum = 0.f, acc = 0.f;   // an empty split has sum 0 and weight 0
+#pragma unroll
+        for (int c = 0; c < kClusterSplits; ++c)
+            if (ls[c] > 0.f) mall = fmaxf(mall, mx[c]);
+#pragma unroll
+        for (int c = 0; c < kClusterSplits; ++c) {
+            const float w = ls[c] > 0.f ? __expf(mx[c] - mall) : 0.f;
+            lsum = fmaf(ls[c], w, lsum);
+            acc = fmaf(w, v[c], acc);
+        }
+        emit_head1(a, (size_t)m * a.nqh + h0 + h, d, acc * (1.0f / (lsum + 1e-9f)));
+    }
+    cluster_sync_all();   // nobody leaves while its record may still be read
+}
+
+// Tensor-core variant for the binary16 cache (see attention_mma.cuh): same grid and splits as the scalar kernel above; up to eight
+// splits are a cluster (a.tickets == NULL) that merges through its shared memory, more leave partial records and an arrival counter.
+// NW warps of attn_bufs(NW) tiles each in shared memory: with four warps two CTAs (and one of the kernel behind) share an SM; with
+// eight, where there is no more than one CTA per SM, most of a split's tiles are requested up front.  What bounds it: at one sequence
+// and 2,048 positions the chain wait - position and query - tiles - merge, where the tiles took 10,800 cycles with four warps of one
+// tile ahead, the merge through records and counters another 3 us.  Measured (us, 32 / 8 heads, before / now; fused form in a chain
+// of its own kind): 1 x 2,048 positions 10.8 / 8.2, 1 x 512 11.3 / 7.9, 3 x 101 7.2 / 4.5, 2 x 1,024 12.0 / 7.7, 8 x 300 11.0 / 6.5,
+// 8 x 2,048 18.7 / 17.0 (67 MB), 32 x 512 16.5 / 13.8, 4 x 16,384 47.1 / 46.7 (268 MB, 5.7 TB/s).
+template <int GQ, int NW>
+__global__ void __launch_bounds__(NW * 32) attn_decode_mma_kernel(const AttnArgs a) {
     const int split = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    extern __shared__ __align__(128) unsigned char attn_dsm[];   // 4 warps x (K, V) x 2 buffers x 4 KB
+    extern __shared__ __align__(128) unsigned char attn_dsm[];   // NW warps x (K, V) x kBufs buffers x 4 KB
+    constexpr int kBufs = attn_bufs(NW), kWarpSmem = amma::warp_smem(kBufs);
     const int p0 = split * a.split_len;
     const __half* Kb = static_cast<const __half*>(a.K) + (size_t)m * a.kv_batch_elems + a.kv_layer_elems +
                        (size_t)kvh * a.max_seq * kHd;
@@ -289,55 +330,69 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_mma_kernel(const 
                        (size_t)kvh * a.max_seq * kHd;
     pdl_trigger();
     // Fused form: the cache rows below this step's position were written by earlier steps, so every warp requests its
-    // first tile before waiting for the kernel before (whose QKV output and position this kernel needs): the tile's
-    // DRAM latency then overlaps that wait and the query prologue.  Which rows are usable is decided after the wait.
-    const bool early = a.qkv != nullptr && warp * amma::kTile < a.split_len && p0 + warp * amma::kTile < a.max_seq;
-    if (early)
-        amma::issue_tile(Kb, Vb, smem_u32(attn_dsm + warp * amma::kWarpSmem), 0, p0 + warp * amma::kTile, a.max_seq - 1);
+    // first tiles before waiting for the kernel before (whose QKV output and position this kernel needs): their
+    // DRAM latency then overlaps that wait and the query prologue.
+    float2 freq = make_float2(0.f, 0.f);
+    float4 q_norm = make_float4(0.f, 0.f, 0.f, 0.f), k_norm = q_norm;
+    if (a.qkv) {
+#pragma unroll
+        for (int i = 0; i < kBufs - 1; ++i) {
+            const int at = (warp + i * NW) * amma::kTile;
+            if ((at < a.split_len || split == a.nsplit - 1) && p0 + at < a.max_seq)   // (the last split may have grown)
+                amma::issue_tile(Kb, Vb, smem_u32(attn_dsm + warp * kWarpSmem), i, p0 + at, a.max_seq - 1);
+            amma::cp_async_commit();
+        }
+        freq = rope_frequencies(a.rope_base, lane);
+        q_norm = *reinterpret_cast<const float4*>(a.q_norm_w + 4 * lane);
+        k_norm = *reinterpret_cast<const float4*>(a.k_norm_w + 4 * lane);
+    }
     pdl_wait();
+    // this warp's query head and, in the last warps, the new K and V rows: in flight together with the position
+    const int h0 = kvh * GQ, heads = a.nqh + 2 * a.nkv;
+    const float* row = a.qkv + (size_t)m * heads * kHd + 4 * lane;
+    float4 q_in = q_norm, kv_in = q_norm;
+    if (a.qkv) {
+        if (warp < GQ) q_in = *reinterpret_cast<const float4*>(row + (size_t)(h0 + warp) * kHd);
+        if (warp >= NW - 2) kv_in = *reinterpret_cast<const float4*>(row + (size_t)(a.nqh + (warp == NW - 1 ? a.nkv : 0) + kvh) * kHd);
+    }
     const int seq_pos = a.d_seq_pos ? a.d_seq_pos[a.per_seq ? m : 0] : a.seq_pos;
     const int npos = min(seq_pos + 1, a.max_seq);
     // The last split runs to the sequence's own end: the split length is sized from a hint of the context, and a
     // sequence that has grown past the hint must still see all its positions.
     const int p1 = split == a.nsplit - 1 ? npos : min(npos, p0 + a.split_len);
-    const int h0 = kvh * GQ;
-
     __shared__ __align__(16) float s_q[GQ][kHd];
-    __shared__ float s_m[kAttnWarps][GQ], s_l[kAttnWarps][GQ];
+    __shared__ float s_m[NW][GQ], s_l[NW][GQ];
+    __shared__ __align__(16) float s_rec[GQ][kHd];   // this CTA's record of a cluster
+    __shared__ float2 s_ms[GQ];
+    __shared__ uint4 s_new[32];   // the new position's K and V rows, 128 halves each
     __shared__ int s_last;
+    const bool cluster = a.nsplit > 1 && !a.tickets;
     // The per-warp results reuse the warp's own K/V staging area once its stream has drained.
-    auto s_o = [&](int w, int h) { return reinterpret_cast<float*>(attn_dsm + w * amma::kWarpSmem) + h * kHd; };
+    auto s_o = [&](int w, int h) { return reinterpret_cast<float*>(attn_dsm + w * kWarpSmem) + h * kHd; };
     if (a.qkv == nullptr) {
         for (int i = t; i < GQ * kHd; i += blockDim.x) s_q[i / kHd][i % kHd] = a.Q[((size_t)m * a.nqh + h0) * kHd + i];
     } else {
         // Fused head norm + RoPE + cache write (what bw_qk_norm_rope_kv_f16 does in a launch of its own): every CTA
         // norms and rotates its own query heads; the CTA whose split holds the new position also norms and rotates that
-        // position's K row, converts its V row, stores both in the cache and then streams them like any other row.
-        const int heads = a.nqh + 2 * a.nkv;
-        const float* row = a.qkv + (size_t)m * heads * kHd;
-        for (int h = warp; h < GQ; h += kAttnWarps) {
-            float4 v = *reinterpret_cast<const float4*>(row + (size_t)(h0 + h) * kHd + 4 * lane);
-            v = head_norm_rope(v, a.q_norm_w, a.eps, seq_pos, a.rope_base, lane);
-            *reinterpret_cast<float4*>(&s_q[h][4 * lane]) = v;
+        // position's K row, converts its V row, stores both in the cache and takes them from shared memory itself (read back
+        // from the cache behind a fence they cost the last split of every sequence a second round trip).
+        const float4 turn = rope_angles(seq_pos, freq);
+        for (int h = warp; h < GQ; h += NW) {
+            if (h > warp) q_in = *reinterpret_cast<const float4*>(row + (size_t)(h0 + h) * kHd);
+            *reinterpret_cast<float4*>(&s_q[h][4 * lane]) = head_norm_turn(q_in, q_norm, a.eps, turn);
         }
-        if (seq_pos >= p0 && seq_pos < p1 && seq_pos < a.max_seq && warp < 2) {
-            __half* Kw = const_cast<__half*>(Kb) + (size_t)seq_pos * kHd + 4 * lane;
-            __half* Vw = const_cast<__half*>(Vb) + (size_t)seq_pos * kHd + 4 * lane;
-            if (warp == 0) {
-                float4 v = *reinterpret_cast<const float4*>(row + (size_t)(a.nqh + kvh) * kHd + 4 * lane);
-                store_half4(Kw, head_norm_rope(v, a.k_norm_w, a.eps, seq_pos, a.rope_base, lane));
-            } else {
-                store_half4(Vw, *reinterpret_cast<const float4*>(row + (size_t)(a.nqh + a.nkv + kvh) * kHd + 4 * lane));
-            }
-            __threadfence();  // the rows are read back through cp.async (L2) by all four warps
+        if (seq_pos >= p0 && seq_pos < p1 && seq_pos < a.max_seq && warp >= NW - 2) {
+            const int v = warp - (NW - 2);   // 0: K, 1: V
+            if (v == 0) kv_in = head_norm_turn(kv_in, k_norm, a.eps, turn);
+            store_half4(const_cast<__half*>(v == 0 ? Kb : Vb) + (size_t)seq_pos * kHd + 4 * lane, kv_in);
+            store_half4(reinterpret_cast<__half*>(s_new) + v * kHd + 4 * lane, kv_in);
         }
     }
     __syncthreads();
 
     float m_run, l_run, o[32];
-    // rows that were final when the early tile was requested: all below this step's position (and inside the split)
-    amma::warp_stream<GQ>(Kb, Vb, &s_q[0][0], a.scale, p0, p1, warp, kAttnWarps, attn_dsm + warp * amma::kWarpSmem,
-                          m_run, l_run, o, early, min(p1, seq_pos));
+    amma::warp_stream<GQ, kBufs>(Kb, Vb, &s_q[0][0], a.scale, p0, p1, warp, NW, attn_dsm + warp * kWarpSmem, m_run, l_run, o,
+                                     a.qkv != nullptr, a.qkv ? min(p1, seq_pos) : INT_MAX, s_new);
     {
         const int g = lane >> 2, tq = lane & 3;
         if (g < GQ) {
@@ -348,28 +403,36 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_mma_kernel(const 
         }
     }
     __syncthreads();
-    for (int idx = t; idx < GQ * kHd; idx += blockDim.x) {
-        const int h = idx / kHd, d = idx - h * kHd;
+    for (int idx = t; idx < GQ * 32; idx += NW * 32) {   // four dimensions of a head, a warp per head
+        const int h = idx >> 5, d = 4 * lane;
         float mm = -FLT_MAX;
 #pragma unroll
-        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, s_m[w][h]);
-        float ls = 0.f, os = 0.f;
+        for (int w = 0; w < NW; ++w) mm = fmaxf(mm, s_m[w][h]);
+        float ls = 0.f;
+        float4 os = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < kAttnWarps; ++w) {
+        for (int w = 0; w < NW; ++w) {
             const float c = __expf(s_m[w][h] - mm);
+            const float4 v = *reinterpret_cast<const float4*>(s_o(w, h) + d);
             ls = fmaf(s_l[w][h], c, ls);
-            os = fmaf(s_o(w, h)[d], c, os);
+            os.x = fmaf(v.x, c, os.x); os.y = fmaf(v.y, c, os.y); os.z = fmaf(v.z, c, os.z); os.w = fmaf(v.w, c, os.w);
         }
         const size_t head = (size_t)m * a.nqh + h0 + h;
         if (a.nsplit == 1) {
-            emit_head1(a, head, d, os * (1.0f / (ls + 1e-9f)));
+            const float inv = 1.0f / (ls + 1e-9f);
+            emit_head4(a, head, lane, make_float4(os.x * inv, os.y * inv, os.z * inv, os.w * inv));
+        } else if (cluster) {
+            *reinterpret_cast<float4*>(&s_rec[h][d]) = os;
+            if (lane == 0) s_ms[h] = make_float2(mm, ls);
         } else {
-            float* rec = a.part + (head * a.nsplit + split) * kPartStride;
-            rec[d] = os;
-            if (d == 0) { rec[kHd] = mm; rec[kHd + 1] = ls; }
+            float* rec = a.part + (head * a.nsplit + split) * kPartStride;   // 8-byte aligned
+            *reinterpret_cast<float2*>(rec + d) = make_float2(os.x, os.y);
+            *reinterpret_cast<float2*>(rec + d + 2) = make_float2(os.z, os.w);
+            if (lane == 0) *reinterpret_cast<float2*>(rec + kHd) = make_float2(mm, ls);
         }
     }
-    if (a.nsplit > 1 && a.tickets) last_arriver_merge<GQ>(a, m, kvh, h0, &s_last);
+    if (cluster) cluster_merge<GQ>(a, m, h0, split, &s_rec[0][0], s_ms);
+    else if (a.nsplit > 1) last_arriver_merge<GQ>(a, m, kvh, h0, &s_last);
 }
 
 // Merges the per-split partial records of one (sequence, head).
@@ -465,6 +528,33 @@ size_t attn_scratch_bytes(int M, int nqh, int nkv, int ctx) {
     return kTicketBytes + (size_t)M * nqh * 64 * kPartStride * sizeof(float);  // at most 64 splits
 }
 
+// Clusters of `splits` eight-warp CTAs that are resident at once on the current device: one CTA per SM, the SMs of a cluster in one GPC.
+template <int GQ>
+static int resident_clusters(int splits) {
+    static std::atomic<int> cached[kMaxDevices][kClusterSplits + 1];
+    std::atomic<int>& c = cached[current_device()][splits];
+    int n = c.load();
+    if (n > 0) return n;
+    auto kern = attn_decode_mma_kernel<GQ, kManyWarps>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits);
+    cfg.blockDim = dim3(kManyWarps * 32);
+    cfg.dynamicSmemBytes = kManyWarps * amma::warp_smem(attn_bufs(kManyWarps));
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = 1;
+    }
+    c = n;
+    return n;
+}
+
 template <typename KVT>
 static cudaError_t attn_launch(AttnArgs a, int ctx_hint, cudaStream_t st) {
     if ((!a.out && !a.out_q) || (!a.Q && !a.qkv) || !a.K || !a.V || a.nqh < 1 || a.nkv < 1 || a.nqh % a.nkv != 0 || a.M < 1 || a.max_seq < 1)
@@ -477,6 +567,12 @@ static cudaError_t attn_launch(AttnArgs a, int ctx_hint, cudaStream_t st) {
     if ((a.qkv || a.out_q) && !use_mma) return cudaErrorInvalidValue;  // these forms exist in the tensor-core kernel only
     int nsplit = choose_splits(a.M * a.nkv, ctx_hint, sm_count(current_device()));
     if ((size_t)a.M * a.nkv * sizeof(unsigned int) > kTicketBytes) nsplit = 1;  // thousands of pairs fill the GPU unsplit
+    // More than eight short splits: a cluster of eight instead.  Measured (us, 32 / 8 heads, partial records / a cluster): one sequence
+    // 12.5 / 10.8 at 4,096 positions, 13.9 / 12.0 at 6,000, 15.4 / 15.9 at 8,192; where the eight-warp CTAs of all clusters are not
+    // resident at once, 12.6 / 11.8 at 4 x 2,048, but 13.9 / 15.2 at 2 x 4,096.
+    const int pairs = a.M * a.nkv;
+    auto resident = [&](int splits) { return gq == 4 ? resident_clusters<4>(splits) : resident_clusters<8>(splits); };
+    if (use_mma && nsplit > kClusterSplits && ctx_hint <= kClusterSplits * (pairs <= resident(kClusterSplits) ? 768 : 320)) nsplit = kClusterSplits;
     a.split_len = (ctx_hint + nsplit - 1) / nsplit;
     a.split_len = (a.split_len + kPosPerStep - 1) / kPosPerStep * kPosPerStep;
     nsplit = (ctx_hint + a.split_len - 1) / a.split_len;
@@ -484,7 +580,8 @@ static cudaError_t attn_launch(AttnArgs a, int ctx_hint, cudaStream_t st) {
     a.scale = 1.0f / sqrtf((float)kHd);
     a.part = nullptr;
     a.tickets = nullptr;
-    if (nsplit > 1) {
+    const bool cluster = use_mma && nsplit > 1 && nsplit <= kClusterSplits;
+    if (nsplit > 1 && !cluster) {
         // scratch = [arrival counters, one per (sequence, kv head)] [partial records]
         const size_t tick_bytes = kTicketBytes;
         unsigned char* base = nullptr;
@@ -497,14 +594,28 @@ static cudaError_t attn_launch(AttnArgs a, int ctx_hint, cudaStream_t st) {
     const dim3 grid(nsplit, a.nkv, a.M);
     cudaError_t le;
     if (use_mma) {  // the tensor-core kernel
-        const size_t dsm = (size_t)kAttnWarps * amma::kWarpSmem;
-        static std::once_flag once[kMaxDevices];
-        std::call_once(once[current_device()], [&] {
-            cudaFuncSetAttribute(attn_decode_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
-            cudaFuncSetAttribute(attn_decode_mma_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
-        });
-        le = gq == 4 ? launch_pdl(attn_decode_mma_kernel<4>, grid, dim3(kAttnWarps * 32), dsm, st, a)
-                     : launch_pdl(attn_decode_mma_kernel<8>, grid, dim3(kAttnWarps * 32), dsm, st, a);
+        const bool many = nsplit == 1 ? pairs <= sm_count(current_device()) : cluster && pairs <= resident(nsplit);
+        const int nw = many ? kManyWarps : kAttnWarps;
+        const size_t dsm = (size_t)nw * amma::warp_smem(attn_bufs(nw));
+        auto kern = gq == 4 ? (many ? attn_decode_mma_kernel<4, kManyWarps> : attn_decode_mma_kernel<4, kAttnWarps>)
+                            : (many ? attn_decode_mma_kernel<8, kManyWarps> : attn_decode_mma_kernel<8, kAttnWarps>);
+        static std::once_flag once[kMaxDevices][4];
+        std::call_once(once[current_device()][(gq == 8) * 2 + many],
+                       [&] { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm); });
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(nw * 32);
+        cfg.dynamicSmemBytes = dsm;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = nsplit;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cluster ? 2 : 1;
+        le = cudaLaunchKernelEx(&cfg, kern, a);
         count_launch(1);
         return le != cudaSuccess ? le : cudaPeekAtLastError();
     }

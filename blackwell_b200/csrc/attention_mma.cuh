@@ -2,7 +2,7 @@
 //
 // With eight (or four) query heads per KV head the scalar kernel spends more instructions per cache byte than an SM
 // can issue at HBM speed; here the heads of one KV head form the 16 rows of an MMA tile (rows >= the group size are
-// zero), K and V rows stream through shared memory (cp.async, double-buffered per warp, XOR-swizzled 16-byte chunks,
+// zero), K and V rows stream through shared memory (cp.async, three buffers per warp, XOR-swizzled 16-byte chunks,
 // read back with ldmatrix), and a warp handles 16 positions per step:
 //     S = Q K^T   : 8 k-steps x 2 position tiles                 (Q fragments live in registers)
 //     online softmax on the accumulator fragment (row = head: quad shuffles)
@@ -12,6 +12,7 @@
 // Splits, per-warp merge and the last-arriver split merge are those of the scalar kernel.
 #pragma once
 #include <cuda_fp16.h>
+#include <limits.h>
 
 #include "common.cuh"
 
@@ -52,7 +53,8 @@ __device__ __forceinline__ void split_hi_lo(float x, float y, uint32_t& hi, uint
 
 constexpr int kTile = 16;                   // positions per warp step
 constexpr int kTileBytes = kTile * 256;     // one K or V tile: 16 rows x 128 halves
-constexpr int kWarpSmem = 4 * kTileBytes;   // K and V, two buffers each
+// staging area of a warp: K and V, NB buffers each
+__host__ __device__ constexpr int warp_smem(int nb) { return 2 * nb * kTileBytes; }
 // byte offset of 16-byte chunk c of row r inside a tile (chunks XOR-swizzled by the row)
 __device__ __forceinline__ uint32_t tile_off(int r, int c) { return (uint32_t)(r * 256 + ((c ^ (r & 7)) << 4)); }
 
@@ -69,17 +71,16 @@ __device__ __forceinline__ void issue_tile(const __half* Kb, const __half* Vb, u
         cp_async16(sbase + buf * 2 * kTileBytes + tile_off(r, c), Kb + (size_t)pos * 128 + c * 8);
         cp_async16(sbase + buf * 2 * kTileBytes + kTileBytes + tile_off(r, c), Vb + (size_t)pos * 128 + c * 8);
     }
-    cp_async_commit();
 }
 
 // Streams the positions [p0, p1) of one (sequence, kv head) through one warp: returns, for head g = lane / 4, the
 // running maximum, this thread's share of the softmax sum and the un-normalised outputs of dimensions
 // 8 * j + 2 * (lane % 4) + {0, 1}, j = 0..15, in o[2 * j + {0, 1}].
-template <int GQ>
+template <int GQ, int NB>
 __device__ __forceinline__ void warp_stream(const __half* Kb, const __half* Vb, const float* q_heads /* [GQ][128] */,
                                             float scale, int p0, int p1, int warp, int nwarps, unsigned char* wsmem,
-                                            float& m_run, float& l_run, float (&o)[32], bool first_issued = false,
-                                            int fresh_end = 0) {
+                                            float& m_run, float& l_run, float (&o)[32], bool early, int final_end,
+                                            const uint4* new_row) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     // Q fragments for the 8 k-steps: a0 = Q[g][16 ks + 2t, +1], a2 = Q[g][16 ks + 8 + 2t, +1]
     uint32_t qh0[8], qh2[8], ql0[8], ql2[8];
@@ -102,27 +103,33 @@ __device__ __forceinline__ void warp_stream(const __half* Kb, const __half* Vb, 
     const int ntile = (p1 - p0 + kTile - 1) / kTile;
     // tiles of this warp: warp, warp + nwarps, ...
     auto issue = [&](int tile_idx, int buf) { issue_tile(Kb, Vb, sbase, buf, p0 + tile_idx * kTile, p1 - 1); };
-    int it = 0;
-    // `first_issued`: the caller requested this warp's first tile (rows p0 + 16 warp ...) before it knew the sequence's
-    // position.  The copy is good if all its rows lie below `fresh_end` (the end of the rows that were final then);
-    // otherwise it is requested again (after the first has landed: both write the same buffer).
-    if (first_issued && p0 + (warp + 1) * kTile > fresh_end) {
-        cp_async_wait<0>();
-        __syncwarp();
-        first_issued = false;
-    }
-    if (warp < ntile && !first_issued) issue(warp, 0);
-    for (int ti = warp; ti < ntile; ti += nwarps, ++it) {
-        const int buf = it & 1;
-        if (ti + nwarps < ntile) {
-            issue(ti + nwarps, buf ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+    // `early`: the caller requested (and committed one by one) this warp's first NB - 1 tiles (rows p0 + 16 warp ..., p0 + 16 (warp +
+    // nwarps) ..., ...) before it knew the sequence's position.  Rows below `final_end` are in the cache; of those from there on, row
+    // `final_end` itself comes from `new_row` (K and V, 256 bytes each; only where it lies below p1) and the others, which are masked,
+    // become zeros: what the cache holds there may be anything.
+    if (!early) {
+#pragma unroll
+        for (int i = 0; i < NB - 1; ++i) {
+            if (warp + i * nwarps < ntile) issue(warp + i * nwarps, i);
+            cp_async_commit();
         }
+    }
+    int buf = 0;
+    for (int ti = warp; ti < ntile; ti += nwarps) {
+        const int ahead = buf == 0 ? NB - 1 : buf - 1;   // the buffer read last
+        if (ti + (NB - 1) * nwarps < ntile) issue(ti + (NB - 1) * nwarps, ahead);
+        cp_async_commit();
+        cp_async_wait<NB - 1>();
         __syncwarp();
         const uint32_t kt = sbase + buf * 2 * kTileBytes, vt = kt + kTileBytes;
         const int tpos = p0 + ti * kTile;
+        if (tpos + kTile > final_end) {
+            for (int r = max(0, final_end - tpos); r < kTile; ++r) {   // lanes 0-15 the K row, 16-31 the V row
+                const uint4 v = tpos + r == final_end && final_end < p1 ? new_row[lane] : make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(wsmem + buf * 2 * kTileBytes + (lane >> 4) * kTileBytes + tile_off(r, lane & 15)) = v;
+            }
+            __syncwarp();
+        }
 
         // ---- S = Q K^T for 16 positions: s0/s1 = positions 2t, 2t+1 ; s4/s5 = positions 8 + 2t, 8 + 2t + 1
         // four independent accumulator chains (high and low part of Q, two position tiles): a chain of dependent
@@ -174,7 +181,8 @@ __device__ __forceinline__ void warp_stream(const __half* Kb, const __half* Vb, 
             mma_16816(o[2 * jn + 2], o[2 * jn + 3], z0, z1, ph0, ph2, b2, b3);
             mma_16816(o[2 * jn + 2], o[2 * jn + 3], z0, z1, pl0, pl2, b2, b3);
         }
-        __syncwarp();  // the buffer is refilled two iterations later by this same warp
+        __syncwarp();  // the buffer is refilled in the next iteration by this same warp
+        buf = buf == NB - 1 ? 0 : buf + 1;
     }
     cp_async_wait<0>();   // an early first tile this warp turned out not to need
     // the four threads of a head each hold a quarter of the sum

@@ -387,3 +387,32 @@ def test_norm_pending_hand_over_between_two_gemvs(cuda, M, from_swiglu, K1):
     k.gemv_w4a8_decode(out2, 0, None, y, None, 0, to_dev(nw), eps, W2d, s2d, H, N2, M)
     assert max_abs_rel(out.cpu().numpy(), out2.cpu().numpy()) < 1e-3
     assert k.device_status() == 0
+
+
+# eight and four warps, one split, clusters of 2 to 8, partial records; positions at the edges of tiles and splits
+@pytest.mark.parametrize("nq,nkv,hint", [(32, 8, 110), (32, 8, 700), (32, 8, 2064), (64, 8, 2064), (16, 4, 9000)])
+@pytest.mark.parametrize("M", [1, 3, 20])
+def test_fused_attention_reads_no_row_from_its_position_on(cuda, nq, nkv, hint, M):
+    """The cache holds NaN there; the two launches on a clean cache give the same bits."""
+    import torch
+
+    from blackwell_b200 import kernels as k
+
+    max_seq, per = hint + 40, nkv * (hint + 40) * 128
+    g = torch.Generator(device="cuda").manual_seed(hint + M)
+    edges = [0, 1, 15, 16, 17, 63, 64, 100, hint // 8 - 1, hint // 8, hint // 2, hint - 2, hint - 1, hint, hint + 1, max_seq - 1, max_seq]
+    qkv = torch.randn(M, (nq + 2 * nkv) * 128, device="cuda", generator=g)
+    qn, kn = (1 + 0.1 * torch.randn(128, device="cuda", generator=g) for _ in range(2))
+    clean = [torch.randn(M, nkv, max_seq, 128, device="cuda", generator=g).half() for _ in range(2)]
+    for first in range(0, len(edges), M):
+        pos = torch.tensor([edges[(first + m) % len(edges)] for m in range(M)], dtype=torch.int32, device="cuda")
+        later = torch.arange(max_seq, device="cuda")[None, :] >= pos[:, None]
+        dirty = [c.masked_fill(later[:, None, :, None], float("nan")) for c in clean]
+        kc, vc = (c.clone() for c in clean)
+        q, want, got = (torch.empty(M, nq * 128, device="cuda") for _ in range(3))
+        k.qk_norm_rope_kv_f16(q, kc, vc, qkv, qn, kn, pos, nq, nkv, 128, max_seq, M, per, 0, 1e-6, 1e6)
+        k.attention_decode_f16kv(want, q, kc, vc, pos, hint, nq, nkv, 128, max_seq, M, per, 0)
+        k.attention_decode_f16kv_fused(got, qkv, qn, kn, *dirty, pos, hint, nq, nkv, 128, max_seq, M, per, 0, 1e-6, 1e6)
+        assert torch.equal(got, want), pos.tolist()
+        seen = later & (torch.arange(max_seq, device="cuda")[None, :] == pos[:, None])
+        assert all(torch.equal(d.transpose(1, 2)[seen], c.transpose(1, 2)[seen]) for d, c in zip(dirty, (kc, vc)))
