@@ -95,25 +95,6 @@ struct WideArgs {
 __host__ __device__ constexpr int xhalf_bytes(int NP) { return 8 * 2 * 3 * NP * 16; }
 __host__ __device__ constexpr int xchunk_bytes(int NP) { return 2 * xhalf_bytes(NP) + NP * 4; }
 
-// Bounded wait that is a probe and a branch in the common case.  After more than a second, or once another has given up (a non-zero
-// word of shared memory at `flag`), it sets that word and returns; the caller looks at it now and then.  What is computed in between
-// is never stored.
-__device__ __forceinline__ void mbar_wait_or_abort(uint32_t bar, uint32_t parity, uint32_t flag) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b32 f;\n\t.reg .b64 t0, t1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra D%=;\n\t"
-        "mov.u64 t0, %%clock64;\n"
-        "W%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra D%=;\n\t"
-        "ld.volatile.shared.u32 f, [%2];\n\tsetp.ne.u32 p, f, 0;\n\t@p bra D%=;\n\t"
-        "mov.u64 t1, %%clock64;\n\tsub.s64 t1, t1, t0;\n\tsetp.lt.s64 p, t1, 2500000000;\n\t@p bra W%=;\n\t"
-        "st.volatile.shared.u32 [%2], 1;\nD%=:\n\t}"
-        ::"r"(bar), "r"(parity), "r"(flag) : "memory");
-}
-// Arrival of the lanes for which `yes` holds, without a branch around it (94 against 85 us, 65,536 x 4096 at 32 sequences).
-__device__ __forceinline__ void mbar_arrive_by(bool yes, uint32_t bar) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
-                 ::"r"(bar), "r"((uint32_t)yes) : "memory");
-}
 // D = A * B (accumulate == 0) or D += A * B; A (bf16, row = lane, two k per column) in tensor memory, B in shared memory.
 __device__ __forceinline__ void tc_mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

@@ -6,6 +6,8 @@
 #include "../../include/blackwell_b200.h"
 #include "host_util.h"
 #include "latent_attention.cuh"
+#include "latent_flash_tc.cuh"
+#include "tensor_map.h"
 
 namespace bw {
 namespace lm {
@@ -71,6 +73,32 @@ cudaError_t flash(const LatentArgs& a, const Rows& r, cudaStream_t st) {
                       FlashSmem(D, VT, MT).total, st, a, r);
 }
 
+template <int ND, int NV>
+cudaError_t flash_tc(const LatentArgs& a, const Rows& r, cudaStream_t st) {
+    static std::once_flag once[kMaxDevices];
+    auto kern = latent_flash_tc_kernel<ND, NV>;
+    cudaError_t e = allow_smem(kern, once);
+    if (e != cudaSuccess) return e;
+    const int q_head = a.dim + a.rot, nkeys = r.pos0 + r.T, cols = a.heads * (a.dim + a.V);
+    CUtensorMap mq, mkv, mrot;   // rows from `nkeys` on read as zeros
+    if (!make_map(&mq, a.q, a.heads * q_head, r.T, a.ldq, kTcFlashQ) || !make_map(&mkv, a.kv, cols, nkeys, cols, kTcFlashK) ||
+        !make_map(&mrot, static_cast<const bf16*>(a.cache) + (long)r.slot * a.max_seq * a.ldc, (int)a.ldc, nkeys, a.ldc, kTcFlashK))
+        return cudaErrorInvalidValue;
+    TcFlashArgs f{};
+    f.gate = a.gate; f.sink = a.sink; f.out = static_cast<bf16*>(a.out); f.ld32 = a.ld32; f.ldout = a.ldout; f.heads = a.heads;
+    f.T = r.T; f.pos0 = r.pos0; f.q_head = q_head; f.k_head = a.dim; f.v_head = a.V; f.v_first = a.heads * a.dim; f.k_rot = pad8(a.R);
+    f.sl2 = a.scale * 1.4426950408889634f; f.status = status_word_ptr();
+    count_launch(1);
+    return launch_pdl(kern, dim3(a.heads, (r.T + kTcFlashQ - 1) / kTcFlashQ), dim3(kTcFlashThreads), TcFlashShape<ND, NV>::kSmem, st, mq, mkv,
+                      mrot, f);
+}
+
+bool flash_tc_can(const LatentArgs& a, const Rows& r) {
+    auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    return (a.dim == 64 || a.dim == 128) && (a.V == 64 || a.V == 128) && a.rot == 64 && a.scale > 0.f && a.ldq % 8 == 0 && a.ldout % 8 == 0 &&
+           a.ldc % 8 == 0 && aligned(a.q) && aligned(a.kv) && aligned(a.cache) && aligned(a.out) && encode_fn() && status_word_ptr() && r.T > 0;
+}
+
 // value columns / 8 per block, 0 if no form fits shared memory
 int flash_vt(const LatentArgs& a) {
     const int D = pad16(pad8(a.dim) + pad8(a.rot));
@@ -120,6 +148,12 @@ cudaError_t latent_expanded(const LatentArgs& a, const Rows& r, cudaStream_t st)
     x.N = a.heads * (pad8(a.dim) + pad8(a.V)); x.y = a.kv; x.ldy = x.N; x.split = x.N;
     e = linear(x, st);
     if (e != cudaSuccess) return e;
+    // tcgen05 for every number of rows: with the products of keys and values, 16 heads of 128 (64 of them rotated again) and 128 values,
+    // mma.sync / tcgen05: 12.5 / 10.2 us at 17 rows, 14.3 / 11.9 at 64, 28 / 19.4 at 256, 75 / 41 at 1024, 449 / 134 at 4096; 17 rows
+    // after 4000 keys 270 / 101, 300 rows 290 / 116; 64 heads at 300 rows 40 / 25.  Error against 64 bits the same in six digits.
+    if (flash_tc_can(a, r))
+        return a.dim == 64 ? (a.V == 64 ? flash_tc<1, 1>(a, r, st) : flash_tc<1, 2>(a, r, st))
+                           : (a.V == 64 ? flash_tc<2, 1>(a, r, st) : flash_tc<2, 2>(a, r, st));
     const int vt = flash_vt(a);
     // 256 query rows per block where that still gives every SM a block
     const bool tall = vt <= 16 && FlashSmem(pad16(pad8(a.dim) + pad8(a.rot)), vt, 2).total <= kMaxDynSmem &&

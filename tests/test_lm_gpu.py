@@ -131,6 +131,21 @@ def test_long_prompt_many_heads(cuda, tmp_path, vdim):
     d.close()
 
 
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_prompt_attention_of_whole_panels(cuda, tmp_path, dim, vdim):
+    """Heads of 64 and 128 columns, 64 of them rotated: the tcgen05 kernel, in portions that end inside and at its tiles of 64 keys and
+    128 queries.  A scale that makes scores grow along the prompt, so that the running maximum moves."""
+    m = lm.Model(tmp_path, lm.config(64, 50, [lm.latent(3, dim, 64, 72, vdim, 1.0)], [None]), 8)
+    tok = tokens_for(m, 521)
+    want, bar = m.plain(tok)[0], m.bar(tok, False)
+    d = driver(m, False, max_seq=521)
+    for cuts in ([521], [128, 129, 127, 64, 65, 8], [17, 63, 191, 250]):
+        d.release(0)
+        err = lm.rel_error(run(d, 0, tok, cuts), want)
+        assert err.max() < bar, (cuts, int(err.argmax()), err.max(), bar)
+    d.close()
+
+
 @both
 def test_layers_one_by_one(cuda, tmp_path, f32):
     m = lm.Model(tmp_path, lm.mixed(), 6)
