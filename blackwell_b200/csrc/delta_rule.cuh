@@ -26,18 +26,20 @@ inline __host__ __device__ int delta_prepare_front(int N) {
 }
 inline __host__ __device__ int delta_prepare_smem(int N) { return delta_prepare_front(N) + kChunk * kInvRow * 4 + 4 * kChunk * 4; }
 
-// Block (head, chunk).
-__global__ void __launch_bounds__(256) delta_prepare_kernel(const RecurrenceArgs a, const Rows r) {
+// Block (head, chunk, run).
+__global__ void __launch_bounds__(256) delta_prepare_kernel(const RecurrenceArgs a, const __grid_constant__ Runs rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int NP = pad16(a.N), N8 = pad8(a.N), qrow = NP * 2 + 16;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q4 = lane & 3;
+    const Run r = rs.run[blockIdx.z];
     const int h = blockIdx.x, ch = blockIdx.y, grp = h / (a.heads / a.groups);
+    if (ch * kChunk >= r.T) return;
     float* At = reinterpret_cast<float*>(smem + delta_prepare_front(a.N));   // [column of A][row of A]
     float *cum = At + kChunk * kInvRow, *beta = cum + kChunk, *rk = beta + kChunk, *rq = rk + kChunk;
-    unsigned char* unit = static_cast<unsigned char*>(a.chunk_scratch) + ((long)ch * a.heads + h) * kDeltaUnit;
+    unsigned char* unit = static_cast<unsigned char*>(a.chunk_scratch) + ((long)(r.chunk0 + ch) * a.heads + h) * kDeltaUnit;
     const uint32_t qb = smem_u32(smem), kb = qb + kChunk * qrow;
-    const bf16* qg = static_cast<const bf16*>(a.q) + grp * N8;
-    const bf16* kg = static_cast<const bf16*>(a.k) + grp * N8;
+    const bf16* qg = static_cast<const bf16*>(a.q) + r.row0 * a.ldq + grp * N8;
+    const bf16* kg = static_cast<const bf16*>(a.k) + r.row0 * a.ldk + grp * N8;
     pdl_wait();
     for (RowWalk w(t, 256, NP / 8); w.row < kChunk; w.next()) {
         const int col = w.col * 8, tok = ch * kChunk + w.row;
@@ -52,8 +54,8 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(const RecurrenceArgs
         for (int i = 0; i < 2; ++i) {
             const int tok = ch * kChunk + 2 * lane + i;
             const bool ok = tok < r.T;   // rows past the end: no decay, nothing written
-            l[i] = ok ? a.log_decay[(long)tok * a.heads + h] * kLog2e : 0.f;
-            b[i] = ok ? a.weight[(long)tok * a.heads + h] : 0.f;
+            l[i] = ok ? a.log_decay[(long)(r.row0 + tok) * a.heads + h] * kLog2e : 0.f;
+            b[i] = ok ? a.weight[(long)(r.row0 + tok) * a.heads + h] : 0.f;
         }
         float s = l[0] + l[1];
 #pragma unroll
@@ -226,7 +228,7 @@ struct DeltaSmem {
 
 // NTW: 16-row state tiles per warp; VT: state columns per CTA (64 or 32).
 template <int NTW, int VT>
-__global__ void __launch_bounds__(256) delta_chunk_kernel(const RecurrenceArgs a, const Rows r, int nbuf) {
+__global__ void __launch_bounds__(256) delta_chunk_kernel(const RecurrenceArgs a, const __grid_constant__ Runs rs, int nbuf) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NT = VT / 8;
     const DeltaSmem L(a.N, VT, nbuf);
@@ -234,11 +236,12 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(const RecurrenceArgs a
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q4 = lane & 3;
     const int h = blockIdx.y, v0 = blockIdx.x * VT, grp = h / (a.heads / a.groups);
     const uint32_t sb = smem_u32(smem);
+    const Run r = rs.run[blockIdx.z];
     const int nchunks = (r.T + kChunk - 1) / kChunk;
-    const bf16* qg = static_cast<const bf16*>(a.q) + grp * N8;
-    const bf16* kg = static_cast<const bf16*>(a.k) + grp * N8;
-    const bf16* vg = static_cast<const bf16*>(a.v) + h * V8 + v0;
-    const unsigned char* units = static_cast<const unsigned char*>(a.chunk_scratch) + (long)h * kDeltaUnit;
+    const bf16* qg = static_cast<const bf16*>(a.q) + r.row0 * a.ldq + grp * N8;
+    const bf16* kg = static_cast<const bf16*>(a.k) + r.row0 * a.ldk + grp * N8;
+    const bf16* vg = static_cast<const bf16*>(a.v) + r.row0 * a.ldv + h * V8 + v0;
+    const unsigned char* units = static_cast<const unsigned char*>(a.chunk_scratch) + ((long)r.chunk0 * a.heads + h) * kDeltaUnit;
     pdl_wait();
 
     const RowWalk walk(t, 256, NP / 8);
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(256) delta_chunk_kernel(const RecurrenceArgs a
                 for (int p = 0; p < 2; ++p) {
                     const int col = 8 * j + 2 * q4, tok = ch * kChunk + r0 + g + 8 * p;
                     if (tok < r.T && v0 + col < V8)
-                        *reinterpret_cast<float2*>(a.o + (long)tok * a.ldo + h * V8 + v0 + col) = make_float2(acc[j][2 * p], acc[j][2 * p + 1]);
+                        *reinterpret_cast<float2*>(a.o + (long)(r.row0 + tok) * a.ldo + h * V8 + v0 + col) = make_float2(acc[j][2 * p], acc[j][2 * p + 1]);
                 }
         }
         // state: S = exp(total) S + k^T (weighted U)

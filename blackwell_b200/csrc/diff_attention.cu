@@ -23,13 +23,13 @@ cudaError_t allow_smem(F kern, std::once_flag (&once)[kMaxDevices]) {
 int decode_blocks(const DiffAttnArgs& a, int rows) { return a.kv_heads * ((a.heads / a.kv_heads + 7) / 8) * rows; }
 
 template <typename A, int VW>
-cudaError_t prep(const DiffAttnArgs& a, const Rows& r, cudaStream_t st) {
+cudaError_t prep(const DiffAttnArgs& a, const Rows& r, const Runs& rs, cudaStream_t st) {
     const int half = a.rot_dims / 2;
     int items = a.heads * 2 * (half / VW);
     if (a.k) items += a.kv_heads * (2 * (half / VW) + 2 * ((pad8(a.dim) - a.rot_dims) / VW) + pad8(a.V) / VW);
     if (items == 0) return cudaSuccess;
     count_launch(1);
-    return launch_pdl(diff_prep_kernel<A, VW>, dim3((items + 255) / 256, r.T), dim3(256), 0, st, a, r);
+    return launch_pdl(diff_prep_kernel<A, VW>, dim3((items + 255) / 256, rs.n ? rs.longest() : r.T, rs.n ? rs.n : 1), dim3(256), 0, st, a, r, rs);
 }
 
 template <typename A>
@@ -76,13 +76,14 @@ cudaError_t decode(const DiffAttnArgs& a, const Rows& r, cudaStream_t st) {
 }
 
 template <int VT, int MT, int KK>
-cudaError_t flash(const DiffAttnArgs& a, const Rows& r, cudaStream_t st) {
+cudaError_t flash(const DiffAttnArgs& a, const Runs& rs, cudaStream_t st) {
     static std::once_flag once[kMaxDevices];
     auto kern = diff_flash_kernel<VT, MT, KK>;
     cudaError_t e = allow_smem(kern, once);
     if (e != cudaSuccess) return e;
     count_launch(1);
-    return launch_pdl(kern, dim3(a.heads, (r.T + 64 * MT - 1) / (64 * MT)), dim3(256), DiffFlashSmem(a.dim, VT, MT, KK).total, st, a, r);
+    return launch_pdl(kern, dim3(a.heads, rs.n, (rs.longest() + 64 * MT - 1) / (64 * MT)), dim3(256), DiffFlashSmem(a.dim, VT, MT, KK).total, st, a,
+                      rs);
 }
 
 // Sizes of the tensor-core kernels: the smallest instance that holds them, 0 if none does.
@@ -114,7 +115,7 @@ int diff_attention_splits(const DiffAttnArgs& a, int rows, int f32) {
 cudaError_t diff_attention(const DiffAttnArgs& a, const Rows& r, int f32, cudaStream_t st) {
     if (r.T < 1 || !diff_attention_supported(a)) return cudaErrorInvalidValue;
     if (f32) {
-        const cudaError_t e = prep<float, 1>(a, r, st);
+        const cudaError_t e = prep<float, 1>(a, r, Runs{}, st);
         return e != cudaSuccess ? e : scalar<float>(a, r, st);
     }
     if (r.row_slot && (a.splits == 1 || a.splits == 2 || a.splits == 4 || a.splits == 8)) {
@@ -123,16 +124,27 @@ cudaError_t diff_attention(const DiffAttnArgs& a, const Rows& r, int f32, cudaSt
         if (size == 128) return decode<8, 16>(a, r, st);
         if (size == 256) return decode<16, 32>(a, r, st);
     }
-    const cudaError_t e = a.rot_dims % 16 == 0 ? prep<bf16, 8>(a, r, st) : prep<bf16, 1>(a, r, st);
-    if (e != cudaSuccess || r.row_slot) return e != cudaSuccess ? e : scalar<bf16>(a, r, st);
+    if (!r.row_slot && diff_runs_supported(a)) return diff_runs(a, one_run(r), st);
+    const cudaError_t e = a.rot_dims % 16 == 0 ? prep<bf16, 8>(a, r, Runs{}, st) : prep<bf16, 1>(a, r, Runs{}, st);
+    return e != cudaSuccess ? e : scalar<bf16>(a, r, st);
+}
+
+bool diff_runs_supported(const DiffAttnArgs& a) { return flash_fits<8, 1, 64>(a) || flash_fits<16, 1, 64>(a) || flash_fits<32, 1, 32>(a); }
+
+cudaError_t diff_runs(const DiffAttnArgs& a, const Runs& rs, cudaStream_t st) {
+    if (rs.n < 1 || !diff_attention_supported(a)) return cudaErrorInvalidValue;
+    const cudaError_t e = a.rot_dims % 16 == 0 ? prep<bf16, 8>(a, Rows{}, rs, st) : prep<bf16, 1>(a, Rows{}, rs, st);
+    if (e != cudaSuccess) return e;
     // 128 query rows per block where that still gives every SM a block
-    const bool tall = (r.T + 127) / 128 * a.heads >= sm_count(current_device());
-    if (flash_fits<8, 2, 64>(a) && tall) return flash<8, 2, 64>(a, r, st);
-    if (flash_fits<8, 1, 64>(a)) return flash<8, 1, 64>(a, r, st);
-    if (flash_fits<16, 2, 64>(a) && tall) return flash<16, 2, 64>(a, r, st);
-    if (flash_fits<16, 1, 64>(a)) return flash<16, 1, 64>(a, r, st);
-    if (flash_fits<32, 1, 32>(a)) return flash<32, 1, 32>(a, r, st);
-    return scalar<bf16>(a, r, st);
+    int blocks = 0;
+    for (int i = 0; i < rs.n; ++i) blocks += (rs.run[i].T + 127) / 128 * a.heads;
+    const bool tall = blocks >= sm_count(current_device());
+    if (flash_fits<8, 2, 64>(a) && tall) return flash<8, 2, 64>(a, rs, st);
+    if (flash_fits<8, 1, 64>(a)) return flash<8, 1, 64>(a, rs, st);
+    if (flash_fits<16, 2, 64>(a) && tall) return flash<16, 2, 64>(a, rs, st);
+    if (flash_fits<16, 1, 64>(a)) return flash<16, 1, 64>(a, rs, st);
+    if (flash_fits<32, 1, 32>(a)) return flash<32, 1, 32>(a, rs, st);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace lm

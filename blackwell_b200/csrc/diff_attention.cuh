@@ -57,12 +57,22 @@ __device__ __forceinline__ void store_vec(A* p, const float (&v)[VW]) {
     }
 }
 
-// VW elements per thread: query pairs, key pairs, unrotated key elements, values.
+// VW elements per thread: query pairs, key pairs, unrotated key elements, values.  Rows `r`, or (n > 0) the runs `rs`.
 template <typename A, int VW>
-__global__ void __launch_bounds__(256) diff_prep_kernel(const DiffAttnArgs a, const Rows r) {
+__global__ void __launch_bounds__(256) diff_prep_kernel(const DiffAttnArgs a, const Rows r, const __grid_constant__ Runs rs) {
     pdl_trigger();
     pdl_wait();
-    const int row = blockIdx.y, slot = r.slot_of(row), pos = r.pos_of(row);
+    int row = blockIdx.y, slot, pos;
+    if (rs.n > 0) {
+        const Run run = rs.run[blockIdx.z];
+        if (row >= run.T) return;
+        slot = run.slot;
+        pos = run.pos0 + row;
+        row += run.row0;
+    } else {
+        slot = r.slot_of(row);
+        pos = r.pos_of(row);
+    }
     if (slot < 0 || pos >= a.max_seq) return;
     const int D8 = pad8(a.dim), V8 = pad8(a.V), half = a.rot_dims / 2, per = half / VW, rest = (D8 - a.rot_dims) / VW;
     const int nq = a.heads * 2 * per, nk = a.k ? a.kv_heads * 2 * per : 0, nr = a.k ? a.kv_heads * 2 * rest : 0;
@@ -457,16 +467,18 @@ struct DiffFlashSmem {
     }
 };
 
-// Block (head, 64 * MT query rows); a warp has MT tiles of 16 rows of one map (warps 0-3 map 1, warps 4-7 map 2), so that every
+// Block (head, run, 64 * MT query rows); a warp has MT tiles of 16 rows of one map (warps 0-3 map 1, warps 4-7 map 2), so that every
 // key and value fragment it reads from shared memory serves MT products.  KK: keys per shared-memory tile.
 template <int VT, int MT, int KK>
-__global__ void __launch_bounds__(256, 1) diff_flash_kernel(const DiffAttnArgs a, const Rows r) {
+__global__ void __launch_bounds__(256, 1) diff_flash_kernel(const DiffAttnArgs a, const __grid_constant__ Runs rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int kQ = 64 * MT, KT = 4;   // KT: 8-key tiles per softmax step
     const int D8 = pad8(a.dim), D16 = pad16(a.dim), V8 = pad8(a.V), seg = diff_row(a.dim, a.V);
     const DiffFlashSmem L(a.dim, VT, MT, KK);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q4 = lane & 3, map = warp >> 2;
-    const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kQ, h = blockIdx.x;   // longest rows first
+    const Run r = rs.run[blockIdx.y];
+    const int q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * kQ, h = blockIdx.x;   // longest rows first
+    if (q0 >= r.T) return;
     const uint32_t sb = smem_u32(smem);
     const long ldc = (long)a.kv_heads * seg;
     const bf16* cache = static_cast<const bf16*>(a.cache) + (long)r.slot * a.cap * ldc + h / (a.heads / a.kv_heads) * seg;
@@ -499,7 +511,7 @@ __global__ void __launch_bounds__(256, 1) diff_flash_kernel(const DiffAttnArgs a
         const int c = w.col * 8, cm = c < D16 ? c : c - D16;
         const bool ok = q0 + w.row < r.T && cm < D8;
         const bf16* src = static_cast<const bf16*>(a.q);
-        cp_async16z(sb + w.row * L.row + c * 2, ok ? src + (long)(q0 + w.row) * a.ld + (2 * h + (c < D16 ? 0 : 1)) * D8 + cm : src, ok);
+        cp_async16z(sb + w.row * L.row + c * 2, ok ? src + (long)(r.row0 + q0 + w.row) * a.ld + (2 * h + (c < D16 ? 0 : 1)) * D8 + cm : src, ok);
     }
     issue(0, 0);
     float O[MT][VT][4] = {};
@@ -636,7 +648,7 @@ __global__ void __launch_bounds__(256, 1) diff_flash_kernel(const DiffAttnArgs a
             ss += __shfl_xor_sync(0xffffffffu, ss, 2);
             if (q >= r.T) continue;
             const float f = a.out_scale / sqrtf(ss / (float)a.V + a.eps);
-            bf16* out = static_cast<bf16*>(a.out) + (long)q * a.ldout + h * V8;
+            bf16* out = static_cast<bf16*>(a.out) + (long)(r.row0 + q) * a.ldout + h * V8;
 #pragma unroll
             for (int j = 0; j < VT; ++j) {
                 const int col = 8 * j + 2 * q4;

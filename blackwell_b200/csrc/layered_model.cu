@@ -166,6 +166,27 @@ protected:
         v.weight = w.weight + (long)row * s_.heads;
         return v;
     }
+    // Where `can`, the spans of at least `rows` rows share launches (several sequences' chains at once, and tiles for all their rows);
+    // the others, and decode steps, come alone.
+    template <typename Group, typename Single>
+    static int by_runs(const std::vector<Span>& spans, bool can, int rows, Group group, Single single) {
+        std::vector<lm::Run> runs;
+        for (const Span& s : spans) {
+            if (can && !s.r.row_slot && s.r.T >= rows) runs.push_back({s.row0, s.r.T, s.r.slot, s.r.pos0, 0});
+            else BW_TRY(single(s));
+        }
+        std::stable_sort(runs.begin(), runs.end(), [](const lm::Run& a, const lm::Run& b) { return a.T > b.T; });
+        for (size_t i = 0; i < runs.size();) {
+            lm::Runs rs{};
+            for (int chunk = 0; i < runs.size() && rs.n < lm::kMaxRuns; ++i) {
+                runs[i].chunk0 = chunk;
+                chunk += (runs[i].T + lm::kDeltaRows - 1) / lm::kDeltaRows;
+                rs.run[rs.n++] = runs[i];
+            }
+            BW_TRY(group(rs));
+        }
+        return 0;
+    }
     MixerSpec s_;
     Mat in_, o_;
     const float2* cs_ = nullptr;
@@ -191,12 +212,24 @@ protected:
         return a;
     }
     // chunks on the tensor cores from 16 rows on (bf16); token by token with fp32 FMAs otherwise
+    static constexpr int kChunkRows = 16;
+    static bool chunks(const lm::RecurrenceArgs& a) { return a.delta ? lm::delta_chunk_supported(a) : lm::recurrence_chunk_supported(a); }
+    static int recur_runs(const lm::RecurrenceArgs& a, const lm::Runs& rs, cudaStream_t st) {
+        return a.delta ? lm::delta_chunk(a, rs, st) : lm::recurrence_chunk(a, rs, st);
+    }
     int recur(const Env& e, const lm::RecurrenceArgs& a, const lm::Rows& r, cudaStream_t st) const {
-        if (!e.f32 && !r.row_slot && r.T >= 16) {
-            if (a.delta && lm::delta_chunk_supported(a)) return lm::delta_chunk(a, r, st);
-            if (!a.delta && lm::recurrence_chunk_supported(a)) return lm::recurrence_chunk(a, r, st);
-        }
+        if (!e.f32 && !r.row_slot && r.T >= kChunkRows && chunks(a)) return recur_runs(a, lm::one_run(r), st);
         return lm::recurrence_step(a, nullptr, r, e.f32, st);
+    }
+    // convolution (args c, a) and recurrence of one span, or of several
+    int mix(const Env& e, const lm::ConvArgs& c, const lm::RecurrenceArgs& a, const lm::Rows& r, cudaStream_t st) const {
+        if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
+        BW_TRY(lm::conv_silu(c, r, e.f32, st));
+        return recur(e, a, r, st);
+    }
+    static int mix_runs(const lm::ConvArgs& c, const lm::RecurrenceArgs& a, const lm::Runs& rs, cudaStream_t st) {
+        BW_TRY(lm::conv_runs(c, rs, st));
+        return recur_runs(a, rs, st);
     }
 };
 
@@ -234,13 +267,23 @@ public:
     int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         const int inner8 = mixed_ld();
         BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, split_, w.proj32_b, s_.heads, split_, st));
-        for (const Span& s : spans) BW_TRY(mix(e, from(e, w, s.row0, split_, s_.heads, split_ - inner8), s.r, st));
+        lm::ConvArgs c;
+        lm::RecurrenceArgs a;
+        args(e, w, &c, &a);
+        BW_TRY(by_runs(spans, !e.f32 && lm::conv_runs_supported(c) && chunks(a), kChunkRows,
+                       [&](const lm::Runs& rs) { return mix_runs(c, a, rs, st); },
+                       [&](const Span& s) {
+                           lm::ConvArgs c1;
+                           lm::RecurrenceArgs a1;
+                           args(e, from(e, w, s.row0, split_, s_.heads, split_ - inner8), &c1, &a1);
+                           return mix(e, c1, a1, s.r, st);
+                       }));
         return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, T, s_.heads, s_.vdim, s_.norm_groups, 1, e.eps,
                               e.f32, st);
     }
 
 private:
-    int mix(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) const {
+    void args(const Env& e, const Work& w, lm::ConvArgs* conv, lm::RecurrenceArgs* rec) const {
         const int inner8 = mixed_ld(), bc = s_.groups * pad8(s_.state);
         lm::ConvArgs c{};
         c.u = w.proj_b; c.ldu = split_; c.w = conv_w_; c.bias = conv_b_; c.ring = ring_; c.taps = s_.conv; c.heads = s_.heads;
@@ -248,12 +291,11 @@ private:
         c.dt_raw = w.proj32_b; c.ld_dt = s_.heads; c.dt_bias = dt_bias_; c.A_log = A_log_; c.log_decay = w.log_decay; c.weight = w.weight;
         lm::RecurrenceArgs a = recurrence(w);
         a.groups = s_.groups; a.D = D_;
-        if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
-        BW_TRY(lm::conv_silu(c, r, e.f32, st));
         a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + bc);
         a.ldq = a.ldk = a.ldv = c.ldo;
         a.log_decay = w.log_decay; a.weight = w.weight;
-        return recur(e, a, r, st);
+        *conv = c;
+        *rec = a;
     }
     int split_ = 0;
     float *conv_w_ = nullptr, *conv_b_ = nullptr, *dt_bias_ = nullptr, *A_log_ = nullptr, *D_ = nullptr, *norm_ = nullptr, *ring_ = nullptr;
@@ -287,16 +329,18 @@ public:
     int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         const int qk8 = s_.heads * pad8(s_.dim), v8 = mixed_ld();
         BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
-        for (const Span& s : spans) {
-            const Work v = from(e, w, s.row0, in_.N, 0, 0);
+        auto args = [&](const Work& v) {
             lm::RecurrenceArgs a = recurrence(v);
             a.groups = s_.heads;
             a.q = v.proj_b; a.k = e.at(v.proj_b, qk8); a.v = e.at(v.proj_b, 2L * qk8);
             a.ldq = a.ldk = a.ldv = in_.N;
             a.head_log_decay = log_decay_;
             a.const_weight = (float)(1.0 / sqrt((double)s_.dim));
-            BW_TRY(recur(e, a, s.r, st));
-        }
+            return a;
+        };
+        const lm::RecurrenceArgs all = args(w);
+        BW_TRY(by_runs(spans, !e.f32 && chunks(all), kChunkRows, [&](const lm::Runs& rs) { return recur_runs(all, rs, st); },
+                       [&](const Span& s) { return recur(e, args(from(e, w, s.row0, in_.N, 0, 0)), s.r, st); }));
         return lm::gated_norm(w.mixed_b, v8, w.o32_b, v8, e.at(w.proj_b, 2L * qk8 + v8), in_.N, nullptr, T, s_.heads, s_.vdim, s_.heads, 0,
                               e.eps, e.f32, st);
     }
@@ -340,19 +384,29 @@ public:
         w->proj32 = std::max(w->proj32, 2L * s_.heads);
         w->conv = std::max(w->conv, (long)split_ - mixed_ld());
         w->heads = std::max(w->heads, (long)s_.heads);
-        if (!e.f32) w->chunk_bytes = std::max(w->chunk_bytes, (long)lm::delta_chunk_bytes(e.max_rows, s_.heads));
+        if (!e.f32) w->chunk_bytes = std::max(w->chunk_bytes, (long)lm::delta_chunk_bytes(e.pass_rows + lm::kDeltaRows * std::min(e.slots, lm::kMaxRuns), s_.heads));
         BW_TRY(ctx.alloc(&ring_, (size_t)e.slots * s_.conv * (s_.heads * s_.vdim + 2 * s_.kv_heads * s_.dim)));
         return alloc_recurrent(ctx, e, w);
     }
     int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         const int H = s_.heads, inner8 = mixed_ld();
         BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, split_, w.proj32_b, 2 * H, split_, st));
-        for (const Span& s : spans) BW_TRY(mix(e, from(e, w, s.row0, split_, 2 * H, split_ - inner8), s.r, st));
+        lm::ConvArgs c;
+        lm::RecurrenceArgs a;
+        args(e, w, &c, &a);
+        BW_TRY(by_runs(spans, !e.f32 && lm::conv_runs_supported(c) && chunks(a), kChunkRows,
+                       [&](const lm::Runs& rs) { return mix_runs(c, a, rs, st); },
+                       [&](const Span& s) {
+                           lm::ConvArgs c1;
+                           lm::RecurrenceArgs a1;
+                           args(e, from(e, w, s.row0, split_, 2 * H, split_ - inner8), &c1, &a1);
+                           return mix(e, c1, a1, s.r, st);
+                       }));
         return lm::gated_norm(w.mixed_b, inner8, w.o32_b, inner8, w.proj_b, split_, norm_, T, H, s_.vdim, H, 0, e.eps, e.f32, st);
     }
 
 private:
-    int mix(const Env& e, const Work& w, const lm::Rows& r, cudaStream_t st) const {
+    void args(const Env& e, const Work& w, lm::ConvArgs* conv, lm::RecurrenceArgs* rec) const {
         const int H = s_.heads, inner8 = mixed_ld(), qk8 = s_.kv_heads * pad8(s_.dim);
         lm::ConvArgs c{};
         c.u = w.proj_b; c.ldu = split_; c.w = conv_w_; c.ring = ring_; c.taps = s_.conv; c.heads = H; c.V = s_.vdim; c.N = s_.dim;
@@ -360,12 +414,11 @@ private:
         c.beta_raw = w.proj32_b + H; c.dt_bias = dt_bias_; c.A_log = A_log_; c.log_decay = w.log_decay; c.weight = w.weight;
         lm::RecurrenceArgs a = recurrence(w);
         a.groups = s_.kv_heads; a.delta = 1; a.unit_eps = 1e-6f; a.q_scale = (float)(1.0 / sqrt((double)s_.dim)); a.chunk_scratch = w.chunk_b;
-        if (r.row_slot) return lm::recurrence_step(a, &c, r, e.f32, st);
-        BW_TRY(lm::conv_silu(c, r, e.f32, st));
         a.v = w.conv_b; a.k = e.at(w.conv_b, inner8); a.q = e.at(w.conv_b, inner8 + qk8);
         a.ldq = a.ldk = a.ldv = c.ldo;
         a.log_decay = w.log_decay; a.weight = w.weight;
-        return recur(e, a, r, st);
+        *conv = c;
+        *rec = a;
     }
     int split_ = 0;
     float *conv_w_ = nullptr, *dt_bias_ = nullptr, *A_log_ = nullptr, *norm_ = nullptr, *ring_ = nullptr;
@@ -415,8 +468,7 @@ public:
     }
     int run(const Env& e, const Work& w, int T, const std::vector<Span>& spans, cudaStream_t st) override {
         BW_TRY(project(e, w, in_, w.xb, w.ldx, T, w.proj_b, in_.N, nullptr, 0, in_.N, st));
-        for (const Span& s : spans) {
-            const Work v = from(e, w, s.row0, in_.N, 0, 0);
+        auto args = [&](const Work& v) {
             lm::DiffAttnArgs a = base(e);
             const DiffAttention* own = owner_ ? owner_ : this;
             a.cache = own->cache_; a.cap = own->cap_; a.slots = e.slots;
@@ -426,10 +478,15 @@ public:
                 a.v = e.at(v.proj_b, v_);
             }
             a.out = v.mixed_b; a.ldout = mixed_ld();
-            a.splits = lm::diff_attention_splits(a, s.r.T, e.f32);
-            BW_TRY(lm::diff_attention(a, s.r, e.f32, st));
-        }
-        return 0;
+            return a;
+        };
+        const lm::DiffAttnArgs all = args(w);
+        return by_runs(spans, !e.f32 && lm::diff_runs_supported(all), 1, [&](const lm::Runs& rs) { return (int)lm::diff_runs(all, rs, st); },
+                       [&](const Span& s) {
+                           lm::DiffAttnArgs a = args(from(e, w, s.row0, in_.N, 0, 0));
+                           a.splits = lm::diff_attention_splits(a, s.r.T, e.f32);
+                           return (int)lm::diff_attention(a, s.r, e.f32, st);
+                       });
     }
     bool rotates() const override { return true; }
 

@@ -346,13 +346,15 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(const ConvArgs c, const 
 // 1,002, 41 at 4,096, ring included (four rows a thread: the same).  Four prompts that begin together 2449 -> 2338 us.
 constexpr int kConvRun = 8;
 template <int TAPS>
-__global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const Rows r) {
+__global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const __grid_constant__ Runs rs) {
+    const Run r = rs.run[blockIdx.z];
     const int channels = c.heads * c.V + 2 * c.groups * c.N, vec = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * kConvRun;
+    if (t0 >= r.T) return;
     const int steps = (conv_cols(c) / 8 + 127) / 128;
     if (blockIdx.x >= steps) {
         const int i = (blockIdx.x - steps) * 128 + threadIdx.x, t = t0 + i / c.heads;
         pdl_wait();
-        if (i < kConvRun * c.heads && t < r.T) step_sizes(c, i % c.heads, t, t + 1);
+        if (i < kConvRun * c.heads && t < r.T) step_sizes(c, i % c.heads, r.row0 + t, r.row0 + t + 1);
         return;
     }
     if (vec >= conv_cols(c) / 8) return;
@@ -375,8 +377,8 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const R
         }
     }
     pdl_wait();
-    const bf16* u = static_cast<const bf16*>(c.u) + c.off + vec * 8;
-    bf16* out = static_cast<bf16*>(c.out) + vec * 8;
+    const bf16* u = static_cast<const bf16*>(c.u) + r.row0 * c.ldu + c.off + vec * 8;
+    bf16* out = static_cast<bf16*>(c.out) + r.row0 * c.ldo + vec * 8;
     const uint4 zero = make_uint4(0, 0, 0, 0);
     uint4 x[TAPS - 1 + kConvRun], last[TAPS - 1];   // rows t0 - (TAPS - 1) ..; what the ring gets
 #pragma unroll
@@ -443,8 +445,10 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const R
     }
 }
 template <int TAPS>
-cudaError_t conv_run(const ConvArgs& c, const Rows& r, cudaStream_t st) {
-    return launch_pdl(conv_run_kernel<TAPS>, dim3((conv_cols(c) / 8 + 127) / 128 + (kConvRun * c.heads + 127) / 128, (r.T + kConvRun - 1) / kConvRun), dim3(128), 0, st, c, r);
+cudaError_t conv_run(const ConvArgs& c, const Runs& rs, cudaStream_t st) {
+    const dim3 grid((conv_cols(c) / 8 + 127) / 128 + (kConvRun * c.heads + 127) / 128, (rs.longest() + kConvRun - 1) / kConvRun, rs.n);
+    count_launch(1);
+    return launch_pdl(conv_run_kernel<TAPS>, grid, dim3(128), 0, st, c, rs);
 }
 
 template <typename A>
@@ -559,15 +563,17 @@ cudaError_t gated_norm(void* out, long ldout, const float* o, long ldo, const vo
                                gate_first, eps, st);
 }
 
+bool conv_runs_supported(const ConvArgs& c) { return c.taps >= 2 && c.taps <= 4; }
+
+cudaError_t conv_runs(const ConvArgs& c, const Runs& rs, cudaStream_t st) {
+    return c.taps == 2 ? conv_run<2>(c, rs, st) : c.taps == 3 ? conv_run<3>(c, rs, st) : c.taps == 4 ? conv_run<4>(c, rs, st) : cudaErrorInvalidValue;
+}
+
 cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st) {
     const int n = conv_cols(c) + c.heads;
     const dim3 grid((n + 127) / 128, (r.T + kConvRows - 1) / kConvRows), ring((conv_cols(c) + 127) / 128), block(128);
+    if (!f32 && r.T >= 16 && conv_runs_supported(c)) return conv_runs(c, one_run(r), st);
     count_launch(1);
-    if (!f32 && r.T >= 16) {
-        if (c.taps == 2) return conv_run<2>(c, r, st);
-        if (c.taps == 3) return conv_run<3>(c, r, st);
-        if (c.taps == 4) return conv_run<4>(c, r, st);
-    }
     const cudaError_t e = f32 ? launch_pdl(conv_silu_kernel<float>, grid, block, 0, st, c, r) : launch_pdl(conv_silu_kernel<bf16>, grid, block, 0, st, c, r);
     if (e != cudaSuccess) return e;
     count_launch(1);

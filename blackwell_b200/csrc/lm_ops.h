@@ -46,6 +46,23 @@ struct Rows {
     __device__ __forceinline__ int pos_of(int r) const { return row_pos ? row_pos[r] : pos0 + r; }
 };
 
+// Rows of several sequences in one launch of a prompt kernel: runs of consecutive rows (block index z), longest first.
+constexpr int kMaxRuns = 8;
+struct Run {
+    int row0, T, slot, pos0;   // row0: first row in the buffers
+    int chunk0;                // first chunk in the delta rule's scratch
+};
+struct Runs {
+    int n;
+    Run run[kMaxRuns];
+    int longest() const {
+        int t = 0;
+        for (int i = 0; i < n; ++i) t = run[i].T > t ? run[i].T : t;
+        return t;
+    }
+};
+inline Runs one_run(const Rows& r) { return Runs{1, {{0, r.T, r.slot, r.pos0, 0}}}; }
+
 // ---------------------------------------------------------------- embedding, norms
 // xb = norm(x) * next in the activation type, or x itself where next is NULL: the next sublayer's input.
 // x <- table[token] * scale
@@ -80,6 +97,8 @@ struct ConvArgs {
     float *log_decay, *weight;       // [T][heads]
 };
 cudaError_t conv_silu(const ConvArgs& c, const Rows& r, int f32, cudaStream_t st);     // several rows of one sequence, then the ring
+bool conv_runs_supported(const ConvArgs& c);
+cudaError_t conv_runs(const ConvArgs& c, const Runs& rs, cudaStream_t st);              // bf16, 16 rows of each sequence at least
 
 // ---------------------------------------------------------------- gated linear recurrence
 //   S_t = exp(log_decay_t) S_(t-1) + weight_t k_t v_t^T,   o_t = S_t^T q_t + D v_t        (per head; S is N x V, fp32)
@@ -104,10 +123,11 @@ struct RecurrenceArgs {
 // `conv` != NULL (one row per sequence): q, k, v and the decays come from the projection through the convolution.
 cudaError_t recurrence_step(const RecurrenceArgs& a, const ConvArgs* conv, const Rows& r, int f32, cudaStream_t st);
 bool recurrence_chunk_supported(const RecurrenceArgs& a);
-cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Rows& r, cudaStream_t st);   // bf16, rows of one sequence
-size_t delta_chunk_bytes(int rows, int heads);
+cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st);   // bf16
+size_t delta_chunk_bytes(int rows, int heads);   // of one run; several take kDeltaRows rows more each
+constexpr int kDeltaRows = 64;
 bool delta_chunk_supported(const RecurrenceArgs& a);
-cudaError_t delta_chunk(const RecurrenceArgs& a, const Rows& r, cudaStream_t st);        // bf16, rows of one sequence
+cudaError_t delta_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st);        // bf16
 
 // ---------------------------------------------------------------- latent attention
 constexpr int kPartStats = 4;   // floats after a split's outputs: running maximum, sum, padding
@@ -169,6 +189,8 @@ inline __host__ __device__ int diff_row(int dim, int V) { return 2 * pad8(dim) +
 bool diff_attention_supported(const DiffAttnArgs& a);
 int diff_attention_splits(const DiffAttnArgs& a, int rows, int f32);
 cudaError_t diff_attention(const DiffAttnArgs& a, const Rows& r, int f32, cudaStream_t st);
+bool diff_runs_supported(const DiffAttnArgs& a);
+cudaError_t diff_runs(const DiffAttnArgs& a, const Runs& rs, cudaStream_t st);   // bf16, rows of prompts
 
 }  // namespace lm
 }  // namespace bw

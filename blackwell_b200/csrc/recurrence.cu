@@ -29,7 +29,7 @@ cudaError_t step_nr(const RecurrenceArgs& a, const ConvArgs& c, const Rows& r, c
 }
 
 template <int NTW, int VT>
-cudaError_t chunk_inst(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) {
+cudaError_t chunk_inst(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
     static std::once_flag once[kMaxDevices];
     auto kern = recurrence_chunk_kernel<NTW, VT>;
     cudaError_t e = cudaSuccess;
@@ -39,11 +39,11 @@ cudaError_t chunk_inst(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     const int nbuf = ChunkSmem(a.N, VT, 2).total <= kMaxDynSmem ? 2 : 1;
     count_launch(1);
-    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads), dim3(256), ChunkSmem(a.N, VT, nbuf).total, st, a, r, nbuf);
+    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads, rs.n), dim3(256), ChunkSmem(a.N, VT, nbuf).total, st, a, rs, nbuf);
 }
 
 template <int NTW, int VT>
-cudaError_t delta_inst(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) {
+cudaError_t delta_inst(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
     static std::once_flag once[kMaxDevices];
     auto kern = delta_chunk_kernel<NTW, VT>;
     cudaError_t e = cudaSuccess;
@@ -53,10 +53,10 @@ cudaError_t delta_inst(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) 
     });
     if (e != cudaSuccess) return e;
     count_launch(2);
-    e = launch_pdl(delta_prepare_kernel, dim3(a.heads, (r.T + kChunk - 1) / kChunk), dim3(256), delta_prepare_smem(a.N), st, a, r);
+    e = launch_pdl(delta_prepare_kernel, dim3(a.heads, (rs.longest() + kChunk - 1) / kChunk, rs.n), dim3(256), delta_prepare_smem(a.N), st, a, rs);
     if (e != cudaSuccess) return e;
     const int nbuf = DeltaSmem(a.N, VT, 2).total <= kMaxDynSmem ? 2 : 1;
-    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads), dim3(256), DeltaSmem(a.N, VT, nbuf).total, st, a, r, nbuf);
+    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads, rs.n), dim3(256), DeltaSmem(a.N, VT, nbuf).total, st, a, rs, nbuf);
 }
 
 }  // namespace
@@ -70,29 +70,29 @@ cudaError_t recurrence_step(const RecurrenceArgs& a, const ConvArgs* conv, const
 
 bool recurrence_chunk_supported(const RecurrenceArgs& a) { return a.N <= 256 && ChunkSmem(a.N, 32, 1).total <= kMaxDynSmem; }
 
-cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) {
-    if (a.groups < 1 || a.heads % a.groups != 0 || r.row_slot || a.delta || !recurrence_chunk_supported(a)) return cudaErrorInvalidValue;
+cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
+    if (a.groups < 1 || a.heads % a.groups != 0 || a.delta || !recurrence_chunk_supported(a)) return cudaErrorInvalidValue;
     // narrow state tiles while the wide ones leave SMs idle or two narrow CTAs share an SM
     const int wide = (pad8(a.V) + 63) / 64 * a.heads, sms = sm_count(current_device());
     const bool pairs = ChunkSmem(a.N, 32, 2).total <= 112 * 1024;
     const bool narrow = a.V <= 32 || wide <= (pairs ? sms : sms / 2) || ChunkSmem(a.N, 64, 1).total > kMaxDynSmem;
-    if (pad16(a.N) <= 128) return narrow ? chunk_inst<1, 32>(a, r, st) : chunk_inst<1, 64>(a, r, st);
-    return narrow ? chunk_inst<2, 32>(a, r, st) : chunk_inst<2, 64>(a, r, st);
+    if (pad16(a.N) <= 128) return narrow ? chunk_inst<1, 32>(a, rs, st) : chunk_inst<1, 64>(a, rs, st);
+    return narrow ? chunk_inst<2, 32>(a, rs, st) : chunk_inst<2, 64>(a, rs, st);
 }
 
 size_t delta_chunk_bytes(int rows, int heads) { return (size_t)((rows + kChunk - 1) / kChunk) * heads * kDeltaUnit; }
 
 bool delta_chunk_supported(const RecurrenceArgs& a) { return a.N <= 256 && DeltaSmem(a.N, 32, 1).total <= kMaxDynSmem; }
 
-cudaError_t delta_chunk(const RecurrenceArgs& a, const Rows& r, cudaStream_t st) {
-    if (a.groups < 1 || a.heads % a.groups != 0 || r.row_slot || !a.delta || !a.chunk_scratch || !a.log_decay || !a.weight ||
+cudaError_t delta_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
+    if (a.groups < 1 || a.heads % a.groups != 0 || !a.delta || !a.chunk_scratch || !a.log_decay || !a.weight ||
         !delta_chunk_supported(a))
         return cudaErrorInvalidValue;
     // wide state tiles only where the narrow ones need more than one round of CTAs
     const int sms = sm_count(current_device()), narrow = (pad8(a.V) + 31) / 32 * a.heads;
     const bool wide = a.V > 32 && narrow > sms && DeltaSmem(a.N, 64, 1).total <= kMaxDynSmem;
-    if (pad16(a.N) <= 128) return wide ? delta_inst<1, 64>(a, r, st) : delta_inst<1, 32>(a, r, st);
-    return wide ? delta_inst<2, 64>(a, r, st) : delta_inst<2, 32>(a, r, st);
+    if (pad16(a.N) <= 128) return wide ? delta_inst<1, 64>(a, rs, st) : delta_inst<1, 32>(a, rs, st);
+    return wide ? delta_inst<2, 64>(a, rs, st) : delta_inst<2, 32>(a, rs, st);
 }
 
 }  // namespace lm
@@ -119,7 +119,7 @@ extern "C" int bw_linear_recurrence(const bw_recurrence_args* a, const bw_rows* 
     bw::lm::Rows w{};
     if (!recurrence_args(a, rows, &r, &w)) return cudaErrorInvalidValue;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (chunked) return f32 ? cudaErrorInvalidValue : bw::lm::recurrence_chunk(r, w, st);
+    if (chunked) return f32 || w.row_slot ? cudaErrorInvalidValue : bw::lm::recurrence_chunk(r, bw::lm::one_run(w), st);
     return bw::lm::recurrence_step(r, nullptr, w, f32, st);
 }
 
@@ -132,6 +132,6 @@ extern "C" int bw_delta_rule(const bw_recurrence_args* a, float unit_eps, float 
     if (!recurrence_args(a, rows, &r, &w) || !r.log_decay || r.D) return cudaErrorInvalidValue;
     r.delta = 1; r.unit_eps = unit_eps; r.q_scale = q_scale; r.chunk_scratch = scratch;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (chunked) return f32 ? cudaErrorInvalidValue : bw::lm::delta_chunk(r, w, st);
+    if (chunked) return f32 || w.row_slot ? cudaErrorInvalidValue : bw::lm::delta_chunk(r, bw::lm::one_run(w), st);
     return bw::lm::recurrence_step(r, nullptr, w, f32, st);
 }

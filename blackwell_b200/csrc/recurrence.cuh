@@ -241,7 +241,7 @@ struct ChunkSmem {
 
 // NTW: 16-row state tiles per warp; VT: state columns per CTA (64 or 32).
 template <int NTW, int VT>
-__global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceArgs a, const Rows r, int nbuf) {
+__global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceArgs a, const __grid_constant__ Runs rs, int nbuf) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int kVRow = VT * 2 + 16, NJ = VT / 16;   // NJ: 8-column output tiles per warp
     const ChunkSmem L(a.N, VT, nbuf);
@@ -250,10 +250,11 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
     const int h = blockIdx.y, v0 = blockIdx.x * VT, grp = h / (a.heads / a.groups);
     const uint32_t sb = smem_u32(smem);
     float* dec = reinterpret_cast<float*>(smem + L.f_off);   // [2][cumulative log2 decay, weight, weight left at the end][chunk]
+    const Run r = rs.run[blockIdx.z];
     const int nchunks = (r.T + kChunk - 1) / kChunk;
-    const bf16* qg = static_cast<const bf16*>(a.q) + grp * N8;
-    const bf16* kg = static_cast<const bf16*>(a.k) + grp * N8;
-    const bf16* vg = static_cast<const bf16*>(a.v) + h * V8 + v0;
+    const bf16* qg = static_cast<const bf16*>(a.q) + r.row0 * a.ldq + grp * N8;
+    const bf16* kg = static_cast<const bf16*>(a.k) + r.row0 * a.ldk + grp * N8;
+    const bf16* vg = static_cast<const bf16*>(a.v) + r.row0 * a.ldv + h * V8 + v0;
     pdl_wait();
 
     const RowWalk walk(t, 256, NP / 8);
@@ -300,8 +301,8 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
         for (int i = 0; i < 2; ++i) {
             const int tok = ch * kChunk + 2 * lane + i;
             const bool ok = tok < r.T;   // rows past the end: no decay, no weight
-            l[i] = !ok ? 0.f : a.log_decay ? a.log_decay[(long)tok * a.heads + h] : a.head_log_decay[h];
-            w[i] = !ok ? 0.f : a.log_decay ? a.weight[(long)tok * a.heads + h] : a.const_weight;
+            l[i] = !ok ? 0.f : a.log_decay ? a.log_decay[(long)(r.row0 + tok) * a.heads + h] : a.head_log_decay[h];
+            w[i] = !ok ? 0.f : a.log_decay ? a.weight[(long)(r.row0 + tok) * a.heads + h] : a.const_weight;
         }
     };
     auto store_decay = [&](int buf) {
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
                         o2.x = fmaf(Dh, __uint_as_float(vv << 16), o2.x);
                         o2.y = fmaf(Dh, __uint_as_float(vv & 0xFFFF0000u), o2.y);
                     }
-                    *reinterpret_cast<float2*>(a.o + (long)tok * a.ldo + h * V8 + v0 + col) = o2;
+                    *reinterpret_cast<float2*>(a.o + (long)(r.row0 + tok) * a.ldo + h * V8 + v0 + col) = o2;
                 }
             }
         // state: S = exp(total) S + k^T (weighted v)
