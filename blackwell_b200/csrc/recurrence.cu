@@ -28,10 +28,10 @@ cudaError_t step_nr(const RecurrenceArgs& a, const ConvArgs& c, const Rows& r, c
          : nr <= 16 ? step_inst<A, 16, CONV>(a, c, r, st) : cudaErrorInvalidValue;
 }
 
-template <int NTW, int VT>
+template <int NW, int WR, int NTW, int VT>
 cudaError_t chunk_inst(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
     static std::once_flag once[kMaxDevices];
-    auto kern = recurrence_chunk_kernel<NTW, VT>;
+    auto kern = recurrence_chunk_kernel<NW, WR, NTW, VT>;
     cudaError_t e = cudaSuccess;
     std::call_once(once[current_device()], [&] {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
@@ -39,7 +39,7 @@ cudaError_t chunk_inst(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st)
     if (e != cudaSuccess) return e;
     const int nbuf = ChunkSmem(a.N, VT, 2).total <= kMaxDynSmem ? 2 : 1;
     count_launch(1);
-    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads, rs.n), dim3(256), ChunkSmem(a.N, VT, nbuf).total, st, a, rs, nbuf);
+    return launch_pdl(kern, dim3((pad8(a.V) + VT - 1) / VT, a.heads, rs.n), dim3(NW * 32), ChunkSmem(a.N, VT, nbuf).total, st, a, rs, nbuf);
 }
 
 template <int NTW, int VT>
@@ -76,8 +76,8 @@ cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream
     const int wide = (pad8(a.V) + 63) / 64 * a.heads, sms = sm_count(current_device());
     const bool pairs = ChunkSmem(a.N, 32, 2).total <= 112 * 1024;
     const bool narrow = a.V <= 32 || wide <= (pairs ? sms : sms / 2) || ChunkSmem(a.N, 64, 1).total > kMaxDynSmem;
-    if (pad16(a.N) <= 128) return narrow ? chunk_inst<1, 32>(a, rs, st) : chunk_inst<1, 64>(a, rs, st);
-    return narrow ? chunk_inst<2, 32>(a, rs, st) : chunk_inst<2, 64>(a, rs, st);
+    if (pad16(a.N) <= 128) return narrow ? chunk_inst<16, 8, 1, 32>(a, rs, st) : chunk_inst<16, 8, 1, 64>(a, rs, st);
+    return narrow ? chunk_inst<16, 16, 1, 32>(a, rs, st) : chunk_inst<16, 16, 1, 64>(a, rs, st);
 }
 
 size_t delta_chunk_bytes(int rows, int heads) { return (size_t)((rows + kChunk - 1) / kChunk) * heads * kDeltaUnit; }

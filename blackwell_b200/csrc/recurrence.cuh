@@ -239,11 +239,12 @@ struct ChunkSmem {
     }
 };
 
-// NTW: 16-row state tiles per warp; VT: state columns per CTA (64 or 32).
-template <int NTW, int VT>
-__global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceArgs a, const __grid_constant__ Runs rs, int nbuf) {
+// NW warps; state: WR warps along its rows, NTW tiles of 16 rows each, the others along its columns; VT: state columns per CTA.
+template <int NW, int WR, int NTW, int VT>
+__global__ void __launch_bounds__(NW * 32) recurrence_chunk_kernel(const RecurrenceArgs a, const __grid_constant__ Runs rs, int nbuf) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int kVRow = VT * 2 + 16, NJ = VT / 16;   // NJ: 8-column output tiles per warp
+    constexpr int kThreads = NW * 32, kVRow = VT * 2 + 16, CG = NW / 4, SJ = kChunk / 8 / CG, NJ = VT / 8 / CG;   // 8-column tiles per warp: scores, output
+    constexpr int SV = VT * WR / NW, VJ = SV / 8;   // state columns of a warp
     const ChunkSmem L(a.N, VT, nbuf);
     const int NP = pad16(a.N), N8 = pad8(a.N), V8 = pad8(a.V);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, q4 = lane & 3;
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
     const bf16* vg = static_cast<const bf16*>(a.v) + r.row0 * a.ldv + h * V8 + v0;
     pdl_wait();
 
-    const RowWalk walk(t, 256, NP / 8);
+    const RowWalk walk(t, kThreads, NP / 8);
     auto issue = [&](int ch, int buf) {
         const uint32_t base = sb + buf * L.buf;
         for (RowWalk w = walk; w.row < kChunk; w.next()) {
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
             cp_async16z(base + w.row * L.qrow + col * 2, ok ? qg + (long)tok * a.ldq + col : qg, ok);
             cp_async16z(base + L.k_off + w.row * L.qrow + col * 2, ok ? kg + (long)tok * a.ldk + col : kg, ok);
         }
-        for (int i = t; i < kChunk * (VT / 8); i += 256) {
+        for (int i = t; i < kChunk * (VT / 8); i += kThreads) {
             const int row = i / (VT / 8), col = (i % (VT / 8)) * 8, tok = ch * kChunk + row;
             const bool ok = tok < r.T && v0 + col < V8;
             cp_async16z(base + L.v_off + row * kVRow + col * 2, ok ? vg + (long)tok * a.ldv + col : vg, ok);
@@ -274,21 +275,22 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
         cp_async_commit();
     };
 
-    // state fragments: rows 16 * (i * 8 + warp) .., columns 8 * j ..
-    float S[NTW][VT / 8][4];
+    // state fragments: rows 16 * (i * WR + wr) .., columns sv0 + 8 * j ..
+    const int wr = warp % WR, sv0 = warp / WR * SV;
+    float S[NTW][VJ][4];
     float* Sg = a.S + (((long)r.slot * a.heads + h) * a.N) * V8 + v0;
     auto state_to_smem = [&] {
 #pragma unroll
         for (int i = 0; i < NTW; ++i) {
-            const int n0 = 16 * (i * 8 + warp);
+            const int n0 = 16 * (i * WR + wr);
             if (n0 >= NP) continue;
 #pragma unroll
-            for (int j = 0; j < VT / 8; ++j)
+            for (int j = 0; j < VJ; ++j)
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
                     uint32_t hi, lo;
                     split_bf16(S[i][j][2 * p], S[i][j][2 * p + 1], hi, lo);
-                    const int off = L.s_off + (n0 + g + 8 * p) * kVRow + (8 * j + 2 * q4) * 2;
+                    const int off = L.s_off + (n0 + g + 8 * p) * kVRow + (sv0 + 8 * j + 2 * q4) * 2;
                     *reinterpret_cast<uint32_t*>(smem + off) = hi;
                     *reinterpret_cast<uint32_t*>(smem + off + NP * kVRow) = lo;
                 }
@@ -327,10 +329,10 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
 #pragma unroll
     for (int i = 0; i < NTW; ++i)
 #pragma unroll
-        for (int j = 0; j < VT / 8; ++j)
+        for (int j = 0; j < VJ; ++j)
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-                const int n = 16 * (i * 8 + warp) + g + 8 * p, v = 8 * j + 2 * q4;
+                const int n = 16 * (i * WR + wr) + g + 8 * p, v = sv0 + 8 * j + 2 * q4;
                 float2 s = make_float2(0.f, 0.f);
                 if (r.pos0 > 0 && n < a.N && v0 + v < V8) s = *reinterpret_cast<const float2*>(Sg + (long)n * V8 + v);
                 S[i][j][2 * p] = s.x;
@@ -347,24 +349,29 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
         if (warp == 0) load_decay(ch + 1);
         const float *cum = dec + (ch & 1) * 3 * kChunk, *wt = cum + kChunk, *left = wt + kChunk;
         const float total = cum[kChunk - 1];
-        const int r0 = 16 * (warp & 3), c0 = 32 * (warp >> 2);   // score columns; output columns start at
-        const int o0 = (VT / 2) * (warp >> 2);
+        const int r0 = 16 * (warp & 3), c0 = 8 * SJ * (warp >> 2), o0 = 8 * NJ * (warp >> 2);   // rows; first score and output columns
         const float cg0 = cum[r0 + g], cg1 = cum[r0 + g + 8];
 
         // scores q k^T and inter-chunk part q S, both over the N dimension
-        float sc[4][4] = {}, out[NJ][4] = {};
+        float sc[SJ][4] = {}, out[NJ][4] = {};
 #pragma unroll 2
         for (int k0 = 0; k0 < NP; k0 += 16) {
             uint32_t fa[4];
             ldsm4(qb + (r0 + (lane & 15)) * L.qrow + (k0 + (lane >> 4) * 8) * 2, fa);
 #pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
+            for (int jj = 0; jj < SJ / 2; ++jj) {
                 if (c0 + 16 * jj <= r0 + 15) {
                     uint32_t fb[4];   // two 8-token tiles of k rows: (k low, k high) each
                     ldsm4(kb + (c0 + 16 * jj + (lane & 7) + (lane >> 4) * 8) * L.qrow + (k0 + ((lane >> 3) & 1) * 8) * 2, fb);
                     mma_bf16(sc[2 * jj], fa[0], fa[1], fa[2], fa[3], fb[0], fb[1]);
                     mma_bf16(sc[2 * jj + 1], fa[0], fa[1], fa[2], fa[3], fb[2], fb[3]);
                 }
+            }
+            if constexpr (NJ == 1) {   // high parts and remainders in one load
+                uint32_t fs[4];
+                ldsm4t(sb + L.s_off + ((lane >> 4) * NP + k0 + (lane & 15)) * kVRow + o0 * 2, fs);
+                mma_bf16(out[0], fa[0], fa[1], fa[2], fa[3], fs[0], fs[1]);
+                mma_bf16(out[0], fa[0], fa[1], fa[2], fa[3], fs[2], fs[3]);
             }
 #pragma unroll
             for (int jj = 0; jj < NJ / 2; ++jj)
@@ -380,7 +387,7 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
 #pragma unroll
         for (int j = 0; j < NJ; ++j) { out[j][0] *= e0; out[j][1] *= e0; out[j][2] *= e1; out[j][3] *= e1; }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < SJ; ++j) {
             const int col = c0 + 8 * j + 2 * q4, ra = r0 + g, rb = ra + 8;
             const float cc0 = cum[col], cc1 = cum[col + 1], w0 = wt[col], w1 = wt[col + 1];
             const float p0 = col <= ra ? sc[j][0] * exp2_fast(cg0 - cc0) * w0 : 0.f, p1 = col + 1 <= ra ? sc[j][1] * exp2_fast(cg0 - cc1) * w1 : 0.f;
@@ -395,7 +402,7 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
             *reinterpret_cast<uint32_t*>(pd + 8 * kPRow + kChunk * kPRow) = lo;
         }
         // values weighted by what is left of them at the end of the chunk
-        for (int i = t; i < kChunk * VT / 2; i += 256) {
+        for (int i = t; i < kChunk * VT / 2; i += kThreads) {
             const int row = i / (VT / 2), col = (i % (VT / 2)) * 2;
             const uint32_t vv = *reinterpret_cast<const uint32_t*>(smem + buf * L.buf + L.v_off + row * kVRow + col * 2);
             const float f = left[row];
@@ -413,6 +420,12 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
             const uint32_t pa = sb + L.p_off + (r0 + (lane & 15)) * kPRow + (k0 + (lane >> 4) * 8) * 2;
             ldsm4(pa, ph);
             ldsm4(pa + kChunk * kPRow, pl);
+            if constexpr (NJ == 1) {
+                uint32_t fv[2];
+                ldsm2t(vb + (k0 + (lane & 15)) * kVRow + o0 * 2, fv);
+                mma_bf16(out[0], ph[0], ph[1], ph[2], ph[3], fv[0], fv[1]);
+                mma_bf16(out[0], pl[0], pl[1], pl[2], pl[3], fv[0], fv[1]);
+            }
 #pragma unroll
             for (int jj = 0; jj < NJ / 2; ++jj) {
                 uint32_t fv[4];
@@ -443,10 +456,10 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
         const float et = exp2_fast(total);
 #pragma unroll
         for (int i = 0; i < NTW; ++i) {
-            const int n0 = 16 * (i * 8 + warp);
+            const int n0 = 16 * (i * WR + wr);
             if (n0 >= NP) continue;
 #pragma unroll
-            for (int j = 0; j < VT / 8; ++j)
+            for (int j = 0; j < VJ; ++j)
 #pragma unroll
                 for (int p = 0; p < 4; ++p) S[i][j][p] *= et;
 #pragma unroll
@@ -454,11 +467,11 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
                 uint32_t fk[4];   // k^T: row n, column token
                 ldsm4t(kb + (k0 + (lane & 7) + (lane >> 4) * 8) * L.qrow + (n0 + ((lane >> 3) & 1) * 8) * 2, fk);
 #pragma unroll
-                for (int jj = 0; jj < VT / 16; ++jj)
+                for (int jj = 0; jj < VJ / 2; ++jj)
 #pragma unroll
                     for (int part = 0; part < 2; ++part) {
                         uint32_t fv[4];
-                        ldsm4t(sb + L.vw_off + (part * kChunk + k0 + (lane & 15)) * kVRow + (16 * jj + (lane >> 4) * 8) * 2, fv);
+                        ldsm4t(sb + L.vw_off + (part * kChunk + k0 + (lane & 15)) * kVRow + (sv0 + 16 * jj + (lane >> 4) * 8) * 2, fv);
                         mma_bf16(S[i][2 * jj], fk[0], fk[1], fk[2], fk[3], fv[0], fv[1]);
                         mma_bf16(S[i][2 * jj + 1], fk[0], fk[1], fk[2], fk[3], fv[2], fv[3]);
                     }
@@ -473,10 +486,10 @@ __global__ void __launch_bounds__(256) recurrence_chunk_kernel(const RecurrenceA
 #pragma unroll
     for (int i = 0; i < NTW; ++i)
 #pragma unroll
-        for (int j = 0; j < VT / 8; ++j)
+        for (int j = 0; j < VJ; ++j)
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-                const int n = 16 * (i * 8 + warp) + g + 8 * p, v = 8 * j + 2 * q4;
+                const int n = 16 * (i * WR + wr) + g + 8 * p, v = sv0 + 8 * j + 2 * q4;
                 if (n < a.N && v0 + v < V8)
                     *reinterpret_cast<float2*>(Sg + (long)n * V8 + v) = make_float2(S[i][j][2 * p], S[i][j][2 * p + 1]);
             }
