@@ -156,9 +156,9 @@ struct StreamPlan {
     size_t smem = 0;
 };
 
-template <int M, typename WS, bool kMulti, bool kPending = false>
+template <int M, typename WS, bool kMulti, bool kPending = false, int RG = RowsPerGroup<M>::value>
 static cudaError_t launch_stream_inst(const GemvArgs& a, const StreamPlan& p, cudaStream_t st) {
-    auto kern = gemv_w4_stream_kernel<M, WS, kMulti, kPending>;
+    auto kern = gemv_w4_stream_kernel<M, WS, kMulti, kPending, RG>;
     static std::once_flag once[kMaxDevices];
     const int dev = current_device();
     cudaError_t attr_err = cudaSuccess;
@@ -198,6 +198,9 @@ static cudaError_t launch_stream_inst(const GemvArgs& a, const StreamPlan& p, cu
 
 template <int M, typename WS>
 static cudaError_t launch_stream_m(const GemvArgs& a, const StreamPlan& p, cudaStream_t st) {
+    if constexpr (M == 3 || M == 4) {
+        if (p.J == 1 && p.rg == 8) return launch_stream_inst<M, WS, false, false, 8>(a, p, st);
+    }
     return p.J > 1 ? launch_stream_inst<M, WS, true>(a, p, st) : launch_stream_inst<M, WS, false>(a, p, st);
 }
 
@@ -248,7 +251,10 @@ static StreamPlan plan_stream(const GemvArgs& a, int M, int ws_bytes, int min_ro
     if (a.x2 && !aligned(a.x2, 16)) return p;
     if (a.norm_w && !aligned(a.norm_w, 16)) return p;
     const int nch = K / 32;
-    const int tmax = M <= 2 ? 512 : 256;
+    // 3 and 4 sequences: up to 384 threads where one pass over K is then enough (two passes of 192 threads read the activations from
+    // shared memory again for every tile, six warps on an SM; 4 sequences of 4,096 x 10,944: 18.4 us, now 15.2 with binary16 scales,
+    // 19.9 / 14.0 with fp32 scales; 4,096 x 12,288 22.7 / 15.5 and 20.7 / 14.2).
+    const int tmax = M <= 2 ? 512 : M <= 4 && nch <= 384 ? 384 : 256;
     p.J = (nch + tmax - 1) / tmax;
     p.Tg = (((nch + p.J - 1) / p.J) + 31) / 32 * 32;
     const int tt = g_tune_threads.load() > 0 ? g_tune_threads.load() : 256;
@@ -264,8 +270,19 @@ static StreamPlan plan_stream(const GemvArgs& a, int M, int ws_bytes, int min_ro
         const size_t R = (size_t)rows_per_group * p.G;
         return align128(R * row_nib) + align128(R * row_sc);
     };
-    // fewer rows per tile when three stages of the full tile do not fit
-    while (rg > 1 && fixed + 3 * stage_of(rg) > (size_t)kMaxDynSmem) rg /= 2;
+    const size_t half_sm = (size_t)(228 * 1024 / 2 - 1024 - 512);
+    // 3 and 4 sequences: eight rows per group where two such stages fit, twice to an SM (or once, for CTAs of more than 256 threads),
+    // and every SM gets a tile.  The reduction and the two barriers of a tile cost as much as four rows of products.  3 / 4 sequences,
+    // K = 4096, us, four rows and eight: 65,536 rows 46.7 / 50.5 and 38.1 / 43.4, 21,888 rows 19.4 / 21.0 and 16.7 / 18.8, 10,944 rows
+    // 13.0 / 14.0 and 12.1 / 13.3.  With one CTA of 256 threads to an SM (fp32 scales) eight rows lose (21,888 rows 18.0 / 19.7 and
+    // 19.3 / 21.0), as they do where SMs stay without a tile (1,024 rows 5.1 / 5.9 and 5.9 / 6.5).
+    if ((M == 3 || M == 4) && p.J == 1 && g_tune_rg.load() == 0) {
+        const size_t stage = stage_of(8);
+        const bool pairs = fixed + 2 * stage <= half_sm, one = p.Tg > 256 && fixed + 2 * stage <= (size_t)kMaxDynSmem;
+        if ((pairs || one) && N >= 8 * p.G * sm_count(current_device())) rg = 8;
+    }
+    // fewer rows per tile when three stages of the full tile (two of eight rows for 3 and 4 sequences) do not fit
+    while (rg > 1 && fixed + (rg == 8 && M > 2 ? 2 : 3) * stage_of(rg) > (size_t)kMaxDynSmem) rg /= 2;
     const size_t stage = stage_of(rg);
     p.rg = rg;
     if (fixed + 2 * stage > (size_t)kMaxDynSmem) return p;
@@ -274,7 +291,6 @@ static StreamPlan plan_stream(const GemvArgs& a, int M, int ws_bytes, int min_ro
     if (want <= 0) {
         // Two resident CTAs per SM hide each other's barrier and reduction phases, which measured faster
         // than one CTA with a deeper ring: take as many stages (up to 4) as half an SM's shared memory holds.
-        const size_t half_sm = (size_t)(228 * 1024 / 2 - 1024 - 512);
         want = fixed + 2 * stage <= half_sm ? (int)((half_sm - fixed) / stage) : 4;
         if (want > 4) want = 4;
     }

@@ -265,7 +265,12 @@ __device__ __forceinline__ void tile_column(const unsigned char* st, size_t stag
                                             const XChunk (&xr)[M], float* acc) {
     const bool full = g + G * (rg - 1) < rows;
     if (full && rg == RG) {
-        rows_full<M, WS, RG>(st, stage_nib, row_nib, row_sc, g, G, c, xr, acc);
+        if constexpr (RG * M > 16) {   // the weights of half of the rows at a time in registers
+            rows_full<M, WS, RG / 2>(st, stage_nib, row_nib, row_sc, g, G, c, xr, acc);
+            rows_full<M, WS, RG / 2>(st, stage_nib, row_nib, row_sc, g + G * (RG / 2), G, c, xr, acc + RG / 2 * M);
+        } else {
+            rows_full<M, WS, RG>(st, stage_nib, row_nib, row_sc, g, G, c, xr, acc);
+        }
     } else if (full && RG >= 4 && rg == RG / 2) {
         rows_full<M, WS, (RG >= 2 ? RG / 2 : 1)>(st, stage_nib, row_nib, row_sc, g, G, c, xr, acc);
     } else {
@@ -302,10 +307,9 @@ __host__ __device__ inline size_t align128(size_t v) { return (v + 127) & ~(size
 
 // kPending: the instantiation that serves the norm-pending hand-over (one sequence); the ordinary one carries none of
 // its code (the hand-over's extra registers cost the M = 1 kernel 3 % on the small matrices).
-template <int M, typename WS, bool kMultiPass, bool kPending = false>
-__global__ void __launch_bounds__(M <= 2 ? 512 : 256, 1)
+template <int M, typename WS, bool kMultiPass, bool kPending = false, int RG = RowsPerGroup<M>::value>
+__global__ void __launch_bounds__(M <= 2 ? 512 : M <= 4 ? 384 : 256, 1)
 gemv_w4_stream_kernel(const GemvArgs a) {
-    constexpr int RG = RowsPerGroup<M>::value;
     constexpr int V = RG * M;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = smem_raw;

@@ -141,6 +141,15 @@ def test_w4a8_matches_oracle(k, M, K, N):
     assert k.device_status() == 0
 
 
+# Eight rows per group and CTAs of up to 384 threads (3 and 4 sequences): around the number of rows that gives every SM a tile of
+# 8 * G rows (G = 2 for K = 4096, 8 for 1024, 1 above), ragged last tiles, K at the edges of one pass (8192, 12288) and beyond.
+@pytest.mark.parametrize("M,K,N", [(3, 4096, 2367), (4, 4096, 2368), (4, 4096, 2371), (3, 1024, 9473), (4, 1024, 9500), (3, 8192, 1184),
+                                   (4, 8224, 1183), (3, 8224, 1185), (4, 10944, 1184), (3, 12288, 1190), (4, 12288, 1187), (4, 12320, 1200)])
+def test_three_and_four_sequences(k, M, K, N):
+    test_w4a8_matches_oracle(k, M, K, N)
+    test_w4a4_matches_oracle(k, M, K, N)
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 4096, 4096), (2, 10944, 512), (8, 4096, 300), (1, 5120, 1280)])
 def test_w4a8_fused_f16_quantize_is_bit_identical_to_unfused(k, M, K, N):
     """The fused prologue quantizes with the same code as the stand-alone quantizer, so the two paths agree
