@@ -76,25 +76,32 @@ int alloc_driver(bw_decode* d) {
 
 // The first prompt_len[m] - 1 tokens of every slot, in passes of portions of different slots: as many rows as a pass holds, so that
 // its products fill the SMs and read the weights once.  (Two portions of one slot in a pass would not do: a layer that reads an
-// earlier layer's ring comes after that one has written both.)  `ids` holds the tokens of all passes and must outlive the copies.
+// earlier layer's ring comes after that one has written both.)  While the layers are watched a pass is one portion, slot after slot: the
+// caller's buffer has the rows of one.  `ids` holds the tokens of all passes and must outlive the copies.
 int feed_prompts(bw_decode* d, const int* prompt_ids, const int* prompt_len, int max_prompt, std::vector<int>* ids, cudaStream_t st) {
     const int M = d->ctx.cfg.batch, cap = d->model->max_group_rows();
     size_t total = 0;
     for (int m = 0; m < M; ++m) total += prompt_len[m] - 1;
     ids->reserve(total);   // the copies below read it in place
+    const bool alone = d->ctx.watch != nullptr;
+    d->ctx.watch_row0 = 0;
     for (bool more = true; more;) {
         more = false;
         for (int m = 0; m < M;) {
             std::vector<bw::Portion> pass;
             const size_t first = ids->size();
-            for (; m < M; ++m) {
+            while (m < M) {
                 const int at = d->at[m], n = std::min(prompt_len[m] - 1 - at, d->model->max_portion());
-                if (n < 1) continue;
-                if ((int)(ids->size() - first) + n > cap) break;
+                if (n < 1) {
+                    ++m;
+                    continue;
+                }
+                if (!pass.empty() && (alone || (int)(ids->size() - first) + n > cap)) break;
                 pass.push_back({m, at, n});
                 ids->insert(ids->end(), prompt_ids + (size_t)m * max_prompt + at, prompt_ids + (size_t)m * max_prompt + at + n);
                 d->at[m] += n;
                 more |= d->at[m] < prompt_len[m] - 1;
+                if (!alone) ++m;
             }
             if (pass.empty()) continue;
             BW_TRY(cudaMemcpyAsync(d->p_tokens, ids->data() + first, (ids->size() - first) * 4, cudaMemcpyHostToDevice, st));

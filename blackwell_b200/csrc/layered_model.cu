@@ -797,8 +797,9 @@ int LayeredModel::enqueue_layers(DecodeContext& ctx, int T, const std::vector<Sp
             BW_TRY(lm::linear(a, st));
             BW_TRY(lm::norm_add(x_, w_.xb, w_.ldx, w_.sub, L.out2, next, T, e.width, e.eps, e.f32, st));
         }
-        if (ctx.watch)
-            BW_TRY(cudaMemcpyAsync(ctx.watch + ((size_t)i * ctx.watch_rows + ctx.watch_row0) * e.width, x_, (size_t)T * e.width * 4,
+        const long watched = ctx.watch ? std::min<long>(T, ctx.watch_rows - ctx.watch_row0) : 0;   // rows past the caller's buffer are not stored
+        if (watched > 0)
+            BW_TRY(cudaMemcpyAsync(ctx.watch + ((size_t)i * ctx.watch_rows + ctx.watch_row0) * e.width, x_, (size_t)watched * e.width * 4,
                                    cudaMemcpyDeviceToDevice, st));
     }
     return 0;

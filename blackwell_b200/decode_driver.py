@@ -158,7 +158,8 @@ class ModelDriver(_Driver):
 
     def watch(self, rows: int):
         """From now on portions also leave the residual stream after every layer in the returned device tensor
-        [layers][rows][width]; rows = 0 switches it off."""
+        [layers][rows][width] (``begin``: each portion of each prompt from row 0 on, over the one before); rows that the tensor
+        does not have are left out; rows = 0 switches it off."""
         import torch
 
         buf = torch.zeros((self.layers, rows, self.width), dtype=torch.float32, device="cuda") if rows else None

@@ -381,7 +381,9 @@ int bw_decode_destroy(bw_decode* d);
  * returns to host memory the logits [n_want][vocab] at the places want[] (ascending, within the portion); it
  * synchronises.  bw_decode_release gives a slot back: the next portion starts a new sequence.  bw_decode_held is the number
  * of tokens a slot holds.  bw_decode_watch_layers: while buffer (device, [layers][rows][hidden] fp32) is not NULL,
- * portions also store the residual stream after every layer there. */
+ * portions also store the residual stream after every layer there: rows that the buffer does not have are left out.
+ * bw_decode_portion stores token i of the call in row i.  bw_decode_begin takes the portions of all prompts one by one
+ * then, slot after slot, and stores each from row 0 on, over what the one before it left there. */
 typedef struct bw_model_info {
     char architecture[64];
     int layers, width, vocab;

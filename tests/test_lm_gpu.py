@@ -382,6 +382,41 @@ def test_daemon_generates_from_ids(cuda, tmp_path):
 
 
 @both
+@pytest.mark.parametrize("portion", [0, 16])
+def test_watching_prompts_that_begin_together(cuda, tmp_path, f32, portion):
+    """A buffer with the rows of the longest portion, or fewer: nothing outside of it is written, and each layer's rows are those of
+    the portions alone, the later ones on top."""
+    import torch
+
+    from blackwell_b200.decode_driver import _L
+
+    m = lm.Model(tmp_path, lm.mixed(), 19)
+    prompts = [tokens_for(m, n, 400 + n).tolist() for n in (41, 40, 30, 19)]   # (one token alone would take the step's kernels)
+    d = driver(m, f32, batch=4, max_portion=portion, max_prompt=64)
+    for rows in (40, 12):
+        want = torch.full((d.layers, rows, d.width), -7.0, device="cuda")
+        buf = d.watch(64)
+        for p in prompts:
+            for at in range(0, len(p) - 1, portion or 400):
+                n = min(portion or 400, len(p) - 1 - at)
+                if at == 0:
+                    d.release(0)
+                d.portion(0, p[at:at + n], want=[])
+                want[:, :min(n, rows)] = buf[:, :min(n, rows)]
+        d.release(0)
+        held = torch.full((d.layers * rows + 200, d.width), -7.0, device="cuda")
+        assert _L.bw_decode_watch_layers(d._h, held[100:].data_ptr(), rows) == 0
+        d.begin(prompts)
+        torch.cuda.synchronize()
+        assert bool((held[:100] == -7).all()) and bool((held[100 + d.layers * rows:] == -7).all())
+        assert torch.equal(held[100:100 + d.layers * rows].view_as(want), want)
+        for i in range(4):
+            d.release(i)
+    d.watch(0)
+    d.close()
+
+
+@both
 def test_trace_runner(cuda, tmp_path, f32):
     m = lm.Model(tmp_path / "m", lm.mixed(), 18)
     out = tmp_path / "out"
