@@ -16,7 +16,7 @@ __device__ __forceinline__ float row_rstd(const GemvArgs& a, int m, int t, float
     float ss = 0.f;
     const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride);
     for (int i = t; i < a.K / 4; i += 256) {
-        const float4 f = __ldg(p + i);
+        const float4 f = p[i];
         ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); ss = fmaf(f.z, f.z, ss); ss = fmaf(f.w, f.w, ss);
     }
     ss = warp_sum(ss);
@@ -34,19 +34,19 @@ __device__ __forceinline__ void load_elements(const GemvArgs& a, int m, int e0, 
     for (int i = 0; i < E / 4; ++i) {
         float* o = v + 4 * i;
         if (a.xkind == kXHalf) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const __half*>(a.x) + at) + i);
+            const uint2 u = reinterpret_cast<const uint2*>(static_cast<const __half*>(a.x) + at)[i];
             const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
             const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
             o[0] = f0.x; o[1] = f0.y; o[2] = f1.x; o[3] = f1.y;
             continue;
         }
-        const float4 f = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + at) + i);
+        const float4 f = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + at)[i];
         o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
         if (a.xkind == kXFloatNorm) {
-            const float4 gw = __ldg(reinterpret_cast<const float4*>(a.norm_w + e0) + i);
+            const float4 gw = reinterpret_cast<const float4*>(a.norm_w + e0)[i];
             o[0] = o[0] * gw.x * rstd; o[1] = o[1] * gw.y * rstd; o[2] = o[2] * gw.z * rstd; o[3] = o[3] * gw.w * rstd;
         } else if (a.xkind == kXSwiglu) {
-            const float4 u = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(a.x2) + at) + i);
+            const float4 u = reinterpret_cast<const float4*>(static_cast<const float*>(a.x2) + at)[i];
             o[0] = silu_mul(o[0], u.x); o[1] = silu_mul(o[1], u.y); o[2] = silu_mul(o[2], u.z); o[3] = silu_mul(o[3], u.w);
         }
     }

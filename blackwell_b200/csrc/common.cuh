@@ -113,6 +113,8 @@ __device__ __forceinline__ void mbar_arrive_by(bool yes, uint32_t bar) {
 // is still running.  pdl_wait() blocks until the predecessor has completed and its writes are visible: everything
 // that reads the predecessor's output, or writes what it may still read, comes after it.  pdl_trigger() lets the
 // successor begin its own preamble.  Both are no-ops for a kernel launched the ordinary way.
+// What the predecessor may write is read by ordinary loads, never by __ldg: a non-coherent load is defined only for memory that nothing
+// writes as long as the kernel runs, and neither a fence nor the wait orders it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

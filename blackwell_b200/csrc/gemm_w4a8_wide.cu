@@ -41,10 +41,10 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
     float sc = 0.f;
     if (a.xkind == kXInt8) {
         if (valid) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2*>(static_cast<const int8_t*>(a.x) + (size_t)m * a.K + e0));
+            const uint2 u = *reinterpret_cast<const uint2*>(static_cast<const int8_t*>(a.x) + (size_t)m * a.K + e0);
 #pragma unroll
             for (int i = 0; i < 8; ++i) q[i] = (i < 4 ? u.x : u.y) >> (8 * (i & 3));
-            sc = __ldg(a.xsc + (size_t)m * (a.K / 16) + (e0 >> 4));
+            sc = a.xsc[(size_t)m * (a.K / 16) + (e0 >> 4)];
         }
     } else {
         float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};

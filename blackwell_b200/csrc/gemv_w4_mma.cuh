@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_w4_mma_kernel(const GemvArgs
                 float ss = 0.f;
                 const float4* px = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride);
                 for (int i = ct; i < K / 4; i += kConsumerWarps * 32) {
-                    const float4 f = __ldg(px + i);
+                    const float4 f = px[i];
                     ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); ss = fmaf(f.z, f.z, ss); ss = fmaf(f.w, f.w, ss);
                 }
                 ss = warp_sum(ss);
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_w4_mma_kernel(const GemvArgs
                     }
                     if (kPending && a.next_q && m < M) {   // one window of K (the host's rule): val is final
                         const int col = r0 + row;
-                        const float v = valid ? val * __ldg(a.next_norm_w + col) : 0.f;
+                        const float v = valid ? val * a.next_norm_w[col] : 0.f;
                         float am = fabsf(v), ss = val * val;
 #pragma unroll
                         for (int sh = 1; sh < 16; sh <<= 1) {

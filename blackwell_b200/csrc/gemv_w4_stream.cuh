@@ -129,22 +129,22 @@ __device__ __forceinline__ void make_xblock(const GemvArgs& a, int m, int kb, fl
     const size_t nkb = (size_t)(K / 16);
     if (a.xkind == kXInt8) {
         const uint2* p = reinterpret_cast<const uint2*>(static_cast<const int8_t*>(a.x) + (size_t)m * K + 16 * (size_t)kb);
-        const uint2 q0 = __ldg(p), q1 = __ldg(p + 1);
+        const uint2 q0 = p[0], q1 = p[1];
         e[0] = prmt(q0.x, q0.y, 0x6420); o[0] = prmt(q0.x, q0.y, 0x7531);
         e[1] = prmt(q1.x, q1.y, 0x6420); o[1] = prmt(q1.x, q1.y, 0x7531);
-        s = __ldg(a.xsc + (size_t)m * nkb + kb) * 0.0625f * rstd;   // rstd is 1 unless the norm is pending
+        s = a.xsc[(size_t)m * nkb + kb] * 0.0625f * rstd;   // rstd is 1 unless the norm is pending
     } else if (a.xkind == kXInt4) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(a.x) + (size_t)m * (K / 2) + 8 * (size_t)kb));
+        const uint2 q = *reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(a.x) + (size_t)m * (K / 2) + 8 * (size_t)kb);
         e[0] = bytes_minus8(q.x & 0x0F0F0F0Fu); o[0] = bytes_minus8((q.x >> 4) & 0x0F0F0F0Fu);
         e[1] = bytes_minus8(q.y & 0x0F0F0F0Fu); o[1] = bytes_minus8((q.y >> 4) & 0x0F0F0F0Fu);
-        s = __ldg(a.xsc + (size_t)m * nkb + kb) * 0.0625f;
+        s = a.xsc[(size_t)m * nkb + kb] * 0.0625f;
     } else {
         float v[16];
         if (a.xkind == kXHalf) {
             const uint4* p = reinterpret_cast<const uint4*>(static_cast<const __half*>(a.x) + (size_t)m * a.x_stride + 16 * (size_t)kb);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const uint4 q = __ldg(p + i);
+                const uint4 q = p[i];
                 const __half2* h = reinterpret_cast<const __half2*>(&q);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -157,14 +157,14 @@ __device__ __forceinline__ void make_xblock(const GemvArgs& a, int m, int kb, fl
             const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride + 16 * (size_t)kb);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 f = __ldg(p + i);
+                const float4 f = p[i];
                 v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
             }
             if (a.xkind == kXFloatNorm || a.xkind == kXFloatNormI4) {
                 const float4* wp = reinterpret_cast<const float4*>(a.norm_w + 16 * (size_t)kb);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float4 gw = __ldg(wp + i);
+                    const float4 gw = wp[i];
                     v[4 * i] = v[4 * i] * gw.x * rstd;
                     v[4 * i + 1] = v[4 * i + 1] * gw.y * rstd;
                     v[4 * i + 2] = v[4 * i + 2] * gw.z * rstd;
@@ -174,7 +174,7 @@ __device__ __forceinline__ void make_xblock(const GemvArgs& a, int m, int kb, fl
                 const float4* up = reinterpret_cast<const float4*>(static_cast<const float*>(a.x2) + (size_t)m * a.x_stride + 16 * (size_t)kb);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float4 u = __ldg(up + i);
+                    const float4 u = up[i];
                     v[4 * i] = silu_mul(v[4 * i], u.x);
                     v[4 * i + 1] = silu_mul(v[4 * i + 1], u.y);
                     v[4 * i + 2] = silu_mul(v[4 * i + 2], u.z);
@@ -397,7 +397,7 @@ gemv_w4_stream_kernel(const GemvArgs a) {
             } else {
                 const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.x) + (size_t)m * a.x_stride);
                 for (int i = t; i < K / 4; i += T) {
-                    const float4 f = __ldg(p + i);
+                    const float4 f = p[i];
                     ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss); ss = fmaf(f.z, f.z, ss); ss = fmaf(f.w, f.w, ss);
                 }
             }
@@ -450,7 +450,7 @@ gemv_w4_stream_kernel(const GemvArgs a) {
 
     // ------------------------------------------------------------- main loop
     bool aborted = false;
-    float held = 0.f;   // norm-pending hand-over with tiles of 8 rows: the even tile's value of this lane
+    float held = 0.f, held_w = 0.f;   // norm-pending hand-over with tiles of 8 rows: the even tile's value and weight of this lane
     for (int tile = 0; tile < ntiles; ++tile) {
         const int s = tile % S;
         const uint32_t parity = (uint32_t)(tile / S) & 1u;
@@ -493,7 +493,8 @@ gemv_w4_stream_kernel(const GemvArgs a) {
 
         if (t < R * M) {
             const int r = t / M, m = t - r * M;
-            float val = 0.f;
+            float val = 0.f, next_w = 0.f;
+            if (kPending && M == 1 && a.next_q && r < rows) next_w = a.next_norm_w[r0 + r];   // in flight with the sums (after y's store: 1 % of a step)
             if (r < rows) {
                 const int gg = r % G, rr = r / G;
                 float sum = 0.f;
@@ -510,9 +511,10 @@ gemv_w4_stream_kernel(const GemvArgs a) {
                 if (R == 8) {
                     if ((tile & 1) == 0) {
                         held = val;
+                        held_w = next_w;
                     } else {
                         const int col = r0 - 8 + r;          // the first half's row; the second is col + 8
-                        const float v0 = held * __ldg(a.next_norm_w + col), v1 = val * __ldg(a.next_norm_w + col + 8);
+                        const float v0 = held * held_w, v1 = val * next_w;
                         float am = fmaxf(fabsf(v0), fabsf(v1)), ss = fmaf(held, held, val * val);
 #pragma unroll
                         for (int o = 1; o < 8; o <<= 1) {
@@ -527,7 +529,7 @@ gemv_w4_stream_kernel(const GemvArgs a) {
                 } else {
                     const unsigned mask = R == 16 ? 0xFFFFu : 0xFFFFFFFFu;
                     const int col = r0 + r;
-                    const float v = r < rows ? val * __ldg(a.next_norm_w + col) : 0.f;
+                    const float v = r < rows ? val * next_w : 0.f;
                     float am = fabsf(v), ss = val * val;
 #pragma unroll
                     for (int o = 1; o < 16; o <<= 1) {

@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const _
 #pragma unroll
     for (int i = 0; i < TAPS - 1 + kConvRun; ++i) {
         const int t = t0 - (TAPS - 1) + i;
-        x[i] = t >= 0 && t < r.T ? __ldg(reinterpret_cast<const uint4*>(u + (long)t * c.ldu)) : zero;
+        x[i] = t >= 0 && t < r.T ? *reinterpret_cast<const uint4*>(u + (long)t * c.ldu) : zero;
     }
     auto unpack = [](const uint4& v, float (&f)[8]) {
         const uint32_t q[4] = {v.x, v.y, v.z, v.w};
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(128) conv_run_kernel(const ConvArgs c, const _
         float* ring = c.ring + (long)r.slot * TAPS * channels;
 #pragma unroll
         for (int i = 0; i < TAPS - 1; ++i)   // (there are more rows than taps)
-            last[i] = __ldg(reinterpret_cast<const uint4*>(u + (long)(r.T - (TAPS - 1) + i) * c.ldu));
+            last[i] = *reinterpret_cast<const uint4*>(u + (long)(r.T - (TAPS - 1) + i) * c.ldu);
 #pragma unroll
         for (int i = 0; i < TAPS - 1; ++i) {
             const int p = r.pos0 - (TAPS - 1) + i;
