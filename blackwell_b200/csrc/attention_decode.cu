@@ -333,7 +333,6 @@ __global__ void __launch_bounds__(NW * 32) attn_decode_mma_kernel(const AttnArgs
     // first tiles before waiting for the kernel before (whose QKV output and position this kernel needs): their
     // DRAM latency then overlaps that wait and the query prologue.
     float2 freq = make_float2(0.f, 0.f);
-    float4 q_norm = make_float4(0.f, 0.f, 0.f, 0.f), k_norm = q_norm;
     if (a.qkv) {
 #pragma unroll
         for (int i = 0; i < kBufs - 1; ++i) {
@@ -343,15 +342,15 @@ __global__ void __launch_bounds__(NW * 32) attn_decode_mma_kernel(const AttnArgs
             amma::cp_async_commit();
         }
         freq = rope_frequencies(a.rope_base, lane);
-        q_norm = *reinterpret_cast<const float4*>(a.q_norm_w + 4 * lane);
-        k_norm = *reinterpret_cast<const float4*>(a.k_norm_w + 4 * lane);
     }
     pdl_wait();
-    // this warp's query head and, in the last warps, the new K and V rows: in flight together with the position
+    // the norm weights, this warp's query head and, in the last warps, the new K and V rows: in flight together with the position
     const int h0 = kvh * GQ, heads = a.nqh + 2 * a.nkv;
     const float* row = a.qkv + (size_t)m * heads * kHd + 4 * lane;
-    float4 q_in = q_norm, kv_in = q_norm;
+    float4 q_norm = make_float4(0.f, 0.f, 0.f, 0.f), k_norm = q_norm, q_in = q_norm, kv_in = q_norm;
     if (a.qkv) {
+        q_norm = *reinterpret_cast<const float4*>(a.q_norm_w + 4 * lane);
+        k_norm = *reinterpret_cast<const float4*>(a.k_norm_w + 4 * lane);
         if (warp < GQ) q_in = *reinterpret_cast<const float4*>(row + (size_t)(h0 + warp) * kHd);
         if (warp >= NW - 2) kv_in = *reinterpret_cast<const float4*>(row + (size_t)(a.nqh + (warp == NW - 1 ? a.nkv : 0) + kvh) * kHd);
     }

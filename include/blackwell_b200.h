@@ -250,7 +250,8 @@ int bw_sample_argmax_merge(const int* cand_all_pairs, int world, int M, int* out
 /* bw_qk_norm_rope_kv_f16 + bw_attention_decode_f16kv in ONE launch: qkv f32 [M][(nqh + 2 nkv) * 128] is the output
  * of the fused QKV projection; every CTA norms and rotates its own query heads, and the CTA whose context split
  * holds the sequence's position norms, rotates and stores that position's K row and stores its V row before
- * streaming the cache (a position outside the cache is not written).  Only for the shapes the tensor-core kernel
+ * streaming the cache (a position outside the cache is not written).  Cache rows below a sequence's position may be read before the
+ * kernel in front of this call has completed; everything else is read after it.  Only for the shapes the tensor-core kernel
  * takes -- binary16 cache, 4 or 8 query heads per kv head -- otherwise cudaErrorInvalidValue.  Replaces, with the
  * attention call, head_norm_kernel / apply_rope_kernel / update_kv_cache of
  * server/inference_server_int4_batched.cu:49-70,262-266. */

@@ -416,3 +416,30 @@ def test_fused_attention_reads_no_row_from_its_position_on(cuda, nq, nkv, hint, 
         assert torch.equal(got, want), pos.tolist()
         seen = later & (torch.arange(max_seq, device="cuda")[None, :] == pos[:, None])
         assert all(torch.equal(d.transpose(1, 2)[seen], c.transpose(1, 2)[seen]) for d, c in zip(dirty, (kc, vc)))
+
+
+def test_fused_attention_takes_norm_weights_of_the_kernel_before(cuda):
+    """The kernel in front writes the norm weights and lets this one start early: they are read after it has completed."""
+    import torch
+
+    from blackwell_b200 import kernels as k
+
+    nq, nkv, hint, M, K, eps = 32, 8, 2048, 2, 16384, 1e-6
+    g = torch.Generator(device="cuda").manual_seed(11)
+    qkv = torch.randn(M, (nq + 2 * nkv) * 128, device="cuda", generator=g)
+    kc, vc = (torch.randn(M, nkv, hint, 128, device="cuda", generator=g).half() for _ in range(2))
+    pos = torch.tensor([hint - 1, 700], dtype=torch.int32, device="cuda")
+    W, sc = synth.int4_weights_device(256, K, 12)
+    x = synth.activations_f16_device(1, K, 13)
+    norms, got = torch.full((256,), float("nan"), device="cuda"), []
+    for wait in (True, False):
+        norms.fill_(float("nan"))
+        out = torch.empty(M, nq * 128, device="cuda")
+        torch.cuda.synchronize()
+        k.gemv_w4a8_f16in(norms, x, W, sc, K, 256, 1)
+        if wait:
+            torch.cuda.synchronize()
+        k.attention_decode_f16kv_fused(out, qkv, norms[:128], norms[128:], kc, vc, pos, hint, nq, nkv, 128, hint, M, nkv * hint * 128, 0, eps, 1e6)
+        torch.cuda.synchronize()
+        got.append(out)
+    assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], got[1])
