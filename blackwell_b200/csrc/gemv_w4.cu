@@ -462,8 +462,10 @@ static cudaError_t gemv_dispatch(GemvArgs a, int M, cudaStream_t st) {
         use_mma = forced || !(windows && tc_can);
     }
     // 9 to 16 sequences of a matrix that is not small: the bf16 tcgen05 kernel (wide::preferred).  Pre-quantized input that the mma.sync
-    // kernel takes stays there, which needs no scratch memory, and so does a call that would have to grow the scratch under capture.
-    if (sizeof(WS) == 2 && M > 8 && M <= 16 && g_tune_mma_min.load() <= 0 && !a.next_q && !a.x_sumsq && (a.xkind != kXInt8 || !use_mma) &&
+    // kernel takes stays there, which needs no scratch memory, and so does a call that would have to grow the scratch under capture, or
+    // one that a range or border set by the caller keeps there.
+    const bool ours = g_tune_mma_min.load() <= 0 && (g_tune_mma_max.load() <= 0 || !use_mma) && M >= tc_min;
+    if (sizeof(WS) == 2 && M > 8 && M <= 16 && ours && !a.next_q && !a.x_sumsq && (a.xkind != kXInt8 || !use_mma) &&
         tc::eligible(a, M) && wide::preferred(M, a.N, a.K) && wide::scratch_at_hand(M, a.N, a.K, st))
         return wide::launch(a, M, st);
     const bool use_tc = !use_mma && sizeof(WS) == 2 && M >= tc_min && tc::eligible(a, M < 64 ? M : 64);

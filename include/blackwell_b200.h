@@ -516,7 +516,9 @@ int bw_peer_comm_destroy(void* comm);
  * streams of the device -- two calls of the same family must not overlap on one GPU -- and grows (cudaMalloc +
  * cudaMemset, synchronising) when a larger problem arrives; an outgrown block stays allocated until the library is
  * unloaded, because launches already enqueued or captured in a CUDA graph still point at it.  A call that would
- * have to grow while its stream is being captured fails with cudaErrorStreamCaptureUnsupported.  To keep the
+ * have to grow while its stream is being captured fails with cudaErrorStreamCaptureUnsupported; a W4A8 product from 9 sequences on
+ * first looks for a kernel that needs less, so that a captured call may add in another order (other last bits) than the same call
+ * outside of a capture, unless its scratch has been reserved or used before.  To keep the
  * serving path free of allocations, reserve the largest sizes once at start-up: bw_gemv_scratch_bytes /
  * bw_attention_scratch_bytes give upper bounds for a shape (take the maximum over the shapes in use).  No
  * counterpart in the reference, whose kernels need no scratch. */
@@ -527,13 +529,15 @@ int bw_reserve_scratch(size_t gemv_bytes, size_t attention_bytes);
 /* Tuning knobs for experiments: key 0 = ring stages (0 = automatic),
  * key 1 = CTAs per SM cap (0 = automatic), key 2 = force the plain-load kernel,
  * key 3 = rows per thread group and tile cap, key 4 = threads per CTA target,
- * key 5 = smallest batch sent to the tensor-core kernel (0 = default 8), key 6 = its K-split (0 = automatic),
+ * key 5 = smallest batch sent to the tcgen05 kernels (0 = default 8; which calls of up to 16 sequences go there stands at
+ * bw_gemv_w4a8), key 6 = their K-split (0 = automatic),
  * key 8 = programmatic dependent launch on (1, default) / off (0), key 9 = tensor-core attention kernel
  * for the binary16 cache on (1, default) / off (0: scalar kernel, for comparison runs), key 10 = smallest vector in
  * KiB that the peer all-reduce sums in two steps on four or more ranks (0 = default 4096), key 11 = longest wait of
  * the peer all-reduce for another rank in milliseconds (0 = default, about 2000), key 12 = 32-k columns per slab of
- * the mma.sync streaming kernel (0 = default 64), keys 13 / 14 = smallest / largest batch it takes (0 = defaults 3 and
- * 16; a smallest batch above 16 switches it off), key 15 = its ring stages (0 = automatic), key 16 = shrink the
+ * the mma.sync streaming kernel (0 = default 64), keys 13 / 14 = smallest / largest batch it takes (0 = defaults 5 and
+ * 16; a smallest batch above 16 switches it off; a smallest batch that is set keeps every matrix of the range there, a largest
+ * one those whose activations fit in one window of K), key 15 = its ring stages (0 = automatic), key 16 = shrink the
  * small-batch kernel's ring to the tiles a CTA has (1, default) or not (0), key 17 = timing experiments on the
  * mma.sync kernel (0 = off; 1 = skip its arithmetic, 2 = skip its copies: results are then meaningless), key 18 =
  * its packed form for up to 4 sequences on (1, default) / off (0), key 19 = timing experiments on the tcgen05
@@ -543,7 +547,7 @@ int bw_reserve_scratch(size_t gemv_bytes, size_t attention_bytes);
  * same for the SwiGLU prologue (0 = default 1), key 22 = decode attention: the earlier split rule with pct % of the SMs
  * as CTA slots (0 = default rule: one wave of two CTAs per SM, at least 224 positions per split),
  * key 23 = bfloat16 linear: up to value - 1 rows (8 at most) take the weight-streaming kernel, more the tcgen05 kernel (0 =
- * automatic), key 24 = products of more than 16 sequences on the tcgen05 kernel's bf16 form (positive: always, negative:
+ * automatic), key 24 = products of more than 8 sequences on the tcgen05 kernel's bf16 form (positive: always, negative:
  * never, 0 = by its estimate of both forms; key 6 there: 1 = whole tiles, 2 to 8 = CTAs of a cluster that share a tile,
  * more = equal shares of all chunks). */
 int bw_set_tuning(int key, int value);

@@ -302,3 +302,27 @@ def test_huge_k_scale_rows_not_16_byte_multiples(k):
     torch.cuda.synchronize()
     assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(x8, x8s, W, sc16)) < 2e-5
     assert k.device_status() == 0
+
+
+@pytest.mark.parametrize("key, value", [(5, 17), (14, 16)])
+@pytest.mark.parametrize("M", [9, 16])
+def test_borders_that_are_set_keep_float_input_on_the_mma_sync_kernel(cuda, M, key, value):
+    """The bits are those of the pre-quantized call, which has no other route; by default the tcgen05 kernel adds in another order."""
+    import torch
+
+    from blackwell_b200 import kernels
+
+    K, N = 2048, 4096
+    W, sc = synth.int4_weights_device(N, K, 31)
+    x = synth.activations_f16_device(M, K, 32)
+    xq, xs = torch.empty((M, K), dtype=torch.int8, device="cuda"), torch.empty((M, K // 16), device="cuda")
+    kernels.quantize_int8_f16(xq, xs, x, M * K)
+    want, by_default, got = (torch.empty((M, N), device="cuda") for _ in range(3))
+    kernels.gemv_w4a8(want, xq, xs, W, sc, K, N, M)
+    kernels.gemv_w4a8_f16in(by_default, x, W, sc, K, N, M)
+    kernels.set_tuning(key, value)
+    try:
+        kernels.gemv_w4a8_f16in(got, x, W, sc, K, N, M)
+    finally:
+        kernels.set_tuning(key, 0)
+    assert torch.equal(got, want) and not torch.equal(by_default, want)
