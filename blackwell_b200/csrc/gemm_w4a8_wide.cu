@@ -602,7 +602,7 @@ void set_force(int v) { g_force = v; }
 // 13 / 33; 633 x 64 7.4 / 8.9, 7.4 / 8.8, 8.7 / 11, 10 / 12: this one is faster at every one of 24 shapes, by 0.16 to 0.9.
 // It does not come here where its chains of chunks would be longer than that form's, unless neither splits K: a narrow matrix of very
 // long rows (300 x 32768), which that form splits finer.
-// Error against 64 bits (2-norm, three seeds; five products / six / the forms that these calls took before): 633 x 64
+// Error against 64 bits (2-norm, three seeds, normal activations and scales; others in the .cuh file; five products / six / the forms that these calls took before): 633 x 64
 // 8.9e-8 / 2.8e-8 / 4.0e-8, 2481 x 1024 1.0e-7 / 4.9e-8 / 8.3e-8, 3072 x 2048 1.04e-7 / 5.6e-8 / 8.8e-8, 2048 x 5632 1.09e-7 / 6.6e-8 /
 // 1.30e-7, 4096 x 4096 1.08e-7 / 6.4e-8 / 1.28e-7, 21888 x 4096 1.12e-7 / 7.1e-8 / 2.0e-7, 4096 x 12288 1.17e-7 / 7.8e-8 / 2.1e-7 to
 // 2.5e-7.  Hence six products up to kSixK, where five would lose more than those did; above, the sixth costs 5 to 10 % of the time.

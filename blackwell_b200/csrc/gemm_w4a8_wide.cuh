@@ -9,9 +9,16 @@
 //   five bits, |s - sh| <= 32 units of s's last place); a nibble q in [-8, 7] has three, so q sh and q sl are bf16 numbers: exact.
 //   Activations: x = xq x_sc is cut into x1 + x2 + x3 in units of a power of two u per (sequence, chunk), u the place of the eighth
 //   bit of the chunk's largest |x|: x1 = x rounded to whole units (|x1| <= 256), x2 the rest as a bf16 number, x3 what is still
-//   left as another: 2^-27 of the chunk's largest |x| or less is lost (an fp32 number loses 2^-25 of itself).
+//   left as another.  Of an element 2^-19 u is lost at most, 2^-26 of the chunk's largest |x|, and never more than 2^-18 of itself.
 // Products: q sh x1 | q sh x2, q sh x3, q sl x1, q sl x2, and q sl x3 where the chains of sums are short (WideArgs::six): without
-// it 8e-8 of a result is lost, whatever its length.
+// it up to 2^-15 u |w| more is lost, never more than 2^-14 of the element's own product.
+// So this is fixed point over 256 k of a sequence, not 24 bits of every block.  Where activations of about one size meet weights of about
+// one size that is 8e-8 of a result with five products and 3e-8 with six, less than the sums of the other forms lose.  Where one block of a
+// chunk is f times the others and its weights are zero, the others' bits are what counts: 4,096 x 4096, 2-norm against 64 bits, five
+// products / six (12 sequences) / every block scaled by itself: f = 4 2.9e-7 / 0.7e-7 / 1.5e-7, f = 64 4.5e-6 / 5.5e-7 / 1.5e-7, f = 1,024
+// 2.2e-5 / 2.6e-6 / 1.5e-7 (quantizing to int8 loses 5e-3).  Finer places of x1 for such blocks do not help: the first sum is then
+// no longer exact (below) and blocks of very different sizes lose 2.8e-7 where they now lose 1.1e-7.  bw_set_tuning key 24 < 0 chooses
+// the forms that scale every block by itself.
 // The first product has an accumulator of its own: x1 and, where the scales of a row's chunk share an exponent, q sh are whole
 // numbers of one unit below 2^8 in magnitude, so its sum over 256 k stays below 2^24 units and is exact -- the tensor core cuts off
 // what an addition shifts out, which in one accumulator would cost up to a unit of the last place at every step, always towards

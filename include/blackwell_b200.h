@@ -50,7 +50,10 @@ int bw_gemv_int4_warp(float* y_out, const void* x_packed, const float* x_scale, 
  * the borders): up to 4 sequences run in the streaming dp4a kernel, 5 to 8 in the streaming mma.sync kernel, 9 to 16 there
  * too where the matrix is small (K < 2048 and K * N < 8,000,000) or the input pre-quantized, everything else from 9 sequences on
  * (K % 32 == 0, 16-byte aligned W and x) in one of the tcgen05 kernels, 64 sequences per launch; operands the
- * tensor-core kernel cannot take fall back to passes of 16 through the mma.sync kernel (or 8 through dp4a). */
+ * tensor-core kernel cannot take fall back to passes of 16 through the mma.sync kernel (or 8 through dp4a).
+ *   The tcgen05 kernel's usual form takes activations in fixed point over 256 k of a sequence: of x = x_q * x_scale at most 2^-26 of the
+ * largest |x| there is lost (2^-22 above 16 sequences with K > 3072), and never more than 2^-18 (2^-14) of x itself.  Key 24 < 0
+ * chooses the forms that scale every block of 16 by itself. */
 int bw_gemv_w4a8(float* y_out, const int8_t* x_q, const float* x_scale, const uint8_t* W_packed,
                  const uint16_t* W_scale_f16, int K, int N, int M, void* stream);
 

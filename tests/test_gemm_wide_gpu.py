@@ -259,3 +259,33 @@ def test_a_call_that_may_not_grow_the_scratch_is_still_taken(k, M, K):
     torch.cuda.synchronize()
     xq, xs = oracle.quantize_int8(x16.astype(np.float32))
     assert max_abs_rel(y.cpu().numpy(), oracle.gemv_w4a8_f64(xq, xs, W, sc16)) < 2e-5
+
+
+@pytest.mark.parametrize("M,K,N,factor", [(17, 1024, 300, 64), (12, 2048, 300, 1024), (20, 3104, 300, 4), (32, 4096, 300, 64), (64, 4096, 300, 1024)])
+def test_blocks_far_below_the_largest_of_their_chunk(k, M, K, N, factor):
+    """One block in 16 carries larger activations on weights that are zero.  Of an element min(2^-19 u, 2^-18 |x|) is lost, u = 2^-7 of
+    the power of two below the chunk's largest |x|, and min(2^-15 u, 2^-14 |x|) more with five products.  These roundings are independent and
+    of both signs: their 2-norm bounds that of the error, beside the fp32 sums.  Without x3 at all 2^-9 |x| would be lost."""
+    import torch
+
+    W, sc16, _ = synth.int4_weights(N, K, seed=K, full_range=True)
+    large = np.arange(K // 16) % 16 == 5
+    W.reshape(N, K // 16, 8)[:, large] = 0x88
+    x16 = synth.activations_f16(M, K, 99).astype(np.float32)
+    x16.reshape(M, K // 16, 16)[:, large] *= factor
+    x16 = x16.astype(np.float16)
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    k.gemv_w4a8_f16in(y, to_dev(x16.view(np.uint16)), to_dev(W), to_dev(sc16.view(np.uint16)), K, N, M)
+    xq, xs = oracle.quantize_int8(x16.astype(np.float32))
+    ref = oracle.gemv_w4a8_f64(xq, xs, W, sc16)
+    x = np.abs(xq.astype(np.float64) * np.repeat(xs, 16, 1))
+    q = np.stack([W & 15, W >> 4], 2).reshape(N, K).astype(np.float64) - 8
+    w = q * np.repeat(sc16.astype(np.float64), 16, 1)
+    top = np.maximum.reduceat(x, np.arange(0, K, 256), axis=1)
+    u = np.repeat(2.0 ** (np.floor(np.log2(top)) - 7), 256, 1)[:, :K]
+    lost = np.minimum(2.0 ** -19 * u, 2.0 ** -18 * x)
+    if M > 16 and K > 3072:
+        lost += np.minimum(2.0 ** -15 * u, 2.0 ** -14 * x)
+    bound = np.sqrt((lost ** 2 @ (w ** 2).T).sum()) + (K // 256 + 2) ** 0.5 * 2.0 ** -24 * np.linalg.norm(ref)
+    assert np.linalg.norm(y.cpu().numpy() - ref) < bound
+    assert bound < 2.0 ** -12 * np.linalg.norm(ref)
