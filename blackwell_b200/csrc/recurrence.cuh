@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kRecThreads) recurrence_step_kernel(const Recu
 
 // ---------------------------------------------------------------------------------------------- chunks of 64 tokens
 constexpr int kChunk = 64;
+static_assert(kChunk == kDeltaRows, "the delta rule's scratch of several runs is laid out by kDeltaRows");
 constexpr int kPRow = kChunk * 2 + 16;   // bytes of a row of scores in shared memory (odd multiple of 16)
 constexpr float kLog2e = 1.4426950408889634f;
 

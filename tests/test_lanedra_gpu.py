@@ -12,7 +12,7 @@ import pytest
 
 from oracle import lm_layers as plain
 from tests import lm_models as lm
-from tests.test_lm_gpu import ROOT, both, driver, run, tokens_for
+from tests.test_lm_gpu import GROUPS, ROOT, both, check_group, driver, run, tokens_for
 
 pytestmark = pytest.mark.gpu
 
@@ -357,3 +357,17 @@ def test_trace_runner(cuda, tmp_path, f32):
     for i, want in rows.items():
         got = np.fromfile(out / f"{i}.f32", "<f4").reshape(want.shape)
         assert lm.rel_error(got, want).max() < m.bar(a, f32)
+
+
+@pytest.mark.parametrize("lens, portion", GROUPS, ids=["twelve", "full pass", "twelve continue"])
+def test_prompts_that_share_passes(cuda, tmp_path, lens, portion):
+    """With portions of 64 the rests continue at 192 in rings of 121 rows and less."""
+    check_group(lm.Model(tmp_path, lm.lanedra_mixed(), 20), lens, portion)
+
+
+@pytest.mark.parametrize("vdim", [136, 264, 512])
+def test_wide_delta_heads(cuda, tmp_path, vdim):
+    m = lm.Model(tmp_path, lm.lanedra(60, 83, [lm.delta(2, 1, 20, vdim, 4)], [None]), 21)
+    d = driver(m, False)
+    check(m, d, tokens_for(m, 90), ([90], [50, 1]), False)
+    d.close()

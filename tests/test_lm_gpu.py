@@ -440,3 +440,43 @@ def test_trace_runner(cuda, tmp_path, f32):
     for i, want in rows.items():
         got = np.fromfile(out / f"{i}.f32", "<f4").reshape(want.shape)
         assert lm.rel_error(got, want).max() < m.bar(a, f32)
+
+
+# ----------------------------------------------------------------------------------------------- shared passes
+def check_group(m, lens, portion):
+    """Prompts that begin together, the slots used twice: the first step's logits of each against the plain ones."""
+    import torch
+
+    prompts = [tokens_for(m, n, 500 + i).tolist() for i, n in enumerate(lens)]
+    d = driver(m, False, batch=len(lens), max_prompt=max(lens), max_new=4, max_portion=portion)
+    for _ in range(2):
+        d.begin(prompts)
+        d.step()
+        torch.cuda.synchronize()
+        got = d.logits().cpu().numpy()
+        for i, p in enumerate(prompts):
+            assert lm.rel_error(got[i:i + 1], m.plain(p)[0][-1:]).max() < m.bar(p, False), (i, len(p))
+    d.close()
+
+
+# One pass of twelve sequences: kernels along sequences take eight at most.  Portions of 64: passes of one, then the three rests, which fill
+# a pass to its last row and continue at 192.  Portions of 256: twelve rests continue at 256 in one pass.
+GROUPS = [([18 + 3 * i for i in range(12)], 0), ([210, 213, 220, 10, 1], 64), ([274 + i % 6 for i in range(12)], 256)]
+
+
+@pytest.mark.parametrize("lens, portion", GROUPS, ids=["twelve", "full pass", "twelve continue"])
+def test_prompts_that_share_passes(cuda, tmp_path, lens, portion):
+    check_group(lm.Model(tmp_path, lm.mixed(), 20), lens, portion)
+
+
+@pytest.mark.parametrize("vdim", [136, 256, 264, 512])
+def test_wide_heads_with_the_gate_last(cuda, tmp_path, vdim):
+    """The gated norm of a head by a warp with two and four vectors a lane: prompts and steps."""
+    m = lm.Model(tmp_path, lm.config(60, 83, [lm.retention(2, 28, vdim, [0.9, 0.99])], [None]), 21)
+    tok = tokens_for(m, 90)
+    want, bar = m.plain(tok)[0], m.bar(tok, False)
+    d = driver(m, False)
+    for cuts in ([90], [50, 1]):
+        d.release(0)
+        assert lm.rel_error(run(d, 0, tok, cuts), want).max() < bar
+    d.close()
