@@ -10,6 +10,7 @@
 #include "act_prep.cuh"
 #include "gemm_w4a8_tc.cuh"
 #include "host_util.h"
+#include "tensor_map.h"
 
 namespace bw {
 #ifdef BW_GEMV_TIMELINE
@@ -503,25 +504,6 @@ gemm_w4a8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const TcArgs a) {
 // ----------------------------------------------------------------------------------------------------------
 // Host side
 // ----------------------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver's tensor-map encoder, looked up through the runtime so that the library carries no link-time
-// dependency on libcuda (it must load on machines without a driver).
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    });
-    return fn;
-}
-
 // Per-device scratch: activation chunks, K-split partials, tickets (zeroed by the prep kernel of a call that splits K).
 static GrowScratch g_tc_scratch;
 cudaError_t scratch(size_t bytes, cudaStream_t st, unsigned char** p) { return g_tc_scratch.get(bytes, (size_t)16 << 20, st, p); }
@@ -562,7 +544,7 @@ bool eligible(const GemvArgs& a, int M) {
     if (reinterpret_cast<uintptr_t>(a.x) & 15) return false;
     if (a.xkind != kXInt8 && a.xkind != kXHalf && a.xkind != kXFloat && a.xkind != kXFloatNorm && a.xkind != kXSwiglu)
         return false;
-    return encode_fn() != nullptr;
+    return lm::encode_fn() != nullptr;
 }
 
 template <int NMMA>
@@ -629,7 +611,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     const cuuint64_t strides[1] = {(cuuint64_t)(a.K / 2)};
     const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 4), (cuuint32_t)kRows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_fn()(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t*>(a.W), dims, strides,
+    const CUresult r = lm::encode_fn()(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t*>(a.W), dims, strides,
                                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;

@@ -56,15 +56,19 @@ namespace wide {
 
 using tc::bulk_g2s_plain;
 using tc::elect_one;
+using tc::idesc_bf16;
 using tc::smem_desc;
 using tc::tc_commit;
 using tc::tc_fence_after;
 using tc::tc_fence_before;
+using tc::tc_mma_bf16_ta;
 using tc::tma_load_2d;
 using tc::tmem_alloc;
 using tc::tmem_dealloc;
 using tc::tmem_relinquish;
+using tc::tmem_st16;
 using tc::tmem_wait_ld;
+using tc::tmem_wait_st;
 
 constexpr int kKc = 256;          // k per chunk = 16 k-blocks
 constexpr int kBlocksPerChunk = 16;
@@ -102,14 +106,6 @@ struct WideArgs {
 __host__ __device__ constexpr int xhalf_bytes(int NP) { return 8 * 2 * 3 * NP * 16; }
 __host__ __device__ constexpr int xchunk_bytes(int NP) { return 2 * xhalf_bytes(NP) + NP * 4; }
 
-// D = A * B (accumulate == 0) or D += A * B; A (bf16, row = lane, two k per column) in tensor memory, B in shared memory.
-__device__ __forceinline__ void tc_mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
 // C accumulator columns of this warp's 32 lanes.
 template <int C>
 __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t* v);
@@ -124,30 +120,17 @@ __device__ __forceinline__ void tmem_ld<12>(uint32_t addr, uint32_t* v) {
     tmem_ld<8>(addr, v);
     tmem_ld<4>(addr + 8, v + 8);
 }
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-          "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(addr)
-        : "memory");
-}
 // Asynchronous copy of B bytes global -> shared; src_bytes 0 writes zeros.
 template <int B>
 __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, uint32_t src_bytes) {
     if constexpr (B == 16) asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
     else asm volatile("cp.async.ca.shared.global.L2::256B [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(src_bytes), "n"(B) : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 template <int R>
 __device__ __forceinline__ void regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R>
 __device__ __forceinline__ void regs_fewer() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
-
-// Instruction descriptor: D = fp32, A = B = bf16, both K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
-}
 
 // ------------------------------------------------------------------ weight unpack
 // What the unpack of one k-block needs of its scale s = sh + sl, each as a bf16 number in both halves of a word.

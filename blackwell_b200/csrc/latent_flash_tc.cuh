@@ -70,36 +70,11 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t* v) {
           "r"(v[31]), "r"(addr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-          "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(addr)
-        : "memory");
-}
-// D (+)= A B of bf16, M = 128: A in shared memory, or in tensor memory (row = lane, two k per column)
-__device__ __forceinline__ void flash_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t more) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(more), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void flash_mma_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more), "r"(0u) : "memory");
-}
 // 128-byte swizzle.  K-major rows of 128 bytes: 8-row groups `sbo` bytes apart.  MN-major: rows are k, 8-row groups `sbo` bytes apart,
 // panels of 64 columns `lbo` bytes apart.
 __device__ __forceinline__ uint64_t flash_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
-// fp32 D, bf16 A and B, M = 128, N = n; B MN-major where mn is set
-__host__ __device__ constexpr uint32_t flash_idesc(int n, bool mn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
-}
-
 template <int ND, int NV>
 __global__ void __launch_bounds__(kTcFlashThreads, 2)
 latent_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
@@ -167,7 +142,7 @@ latent_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     } else if (warp == 5) {
         // The whole warp walks the loop, one elected lane issues.  S of the next tile goes out before this tile's second product, once
         // the P that lay where it goes has been multiplied.
-        constexpr uint32_t id_s = flash_idesc(kTcFlashK, false), id_o = flash_idesc(V, true);
+        constexpr uint32_t id_s = tc::idesc_bf16(kTcFlashK), id_o = tc::idesc_bf16(V, true);
         const bool elected = tc::elect_one();
         auto scores = [&](int j) {
             wait(Sh::kFullK, j & 1);
@@ -177,7 +152,7 @@ latent_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int p = 0; p < NP; ++p)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)   // 16 k = 32 bytes further inside the swizzle atom
-                        flash_mma(tmem + (j & 1) * 64, flash_desc(sq + p * 2 * kTcPanel, 16, 1024) + 2 * k,
+                        tc::tc_mma_bf16(tmem + (j & 1) * 64, flash_desc(sq + p * 2 * kTcPanel, 16, 1024) + 2 * k,
                                   flash_desc(sk + p * kTcPanel, 16, 1024) + 2 * k, id_s, p + k > 0 ? 1u : 0u);
                 tc::tc_commit(bar(Sh::kFullS + (j & 1)));
                 tc::tc_commit(bar(Sh::kEmptyK));
@@ -198,8 +173,8 @@ latent_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int k = 0; k < 4; ++k) {   // 16 keys: two 8-row groups
                     const uint64_t v = flash_desc(sv, kTcPanel, 1024) + k * (2048 >> 4);
                     const uint32_t p = tmem + (j & 1) * 64 + 8 * k;
-                    flash_mma_ta(tmem + Sh::kOCol, p + 32, v, id_o, j + k > 0 ? 1u : 0u);
-                    flash_mma_ta(tmem + Sh::kOCol, p, v, id_o, 1u);
+                    tc::tc_mma_bf16_ta(tmem + Sh::kOCol, p + 32, v, id_o, j + k > 0 ? 1u : 0u);
+                    tc::tc_mma_bf16_ta(tmem + Sh::kOCol, p, v, id_o, 1u);
                 }
                 tc::tc_commit(bar(Sh::kDoneO + (j & 1)));
             }
@@ -264,10 +239,10 @@ latent_flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
                     split_bf16(__uint_as_float(s[2 * (c + i)]), __uint_as_float(s[2 * (c + i) + 1]), hi[i], lo[i]);
-                tmem_st16(at + c, hi);
-                tmem_st16(at + 32 + c, lo);
+                tc::tmem_st16(at + c, hi);
+                tc::tmem_st16(at + 32 + c, lo);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc::tmem_wait_st();
             tc::tc_fence_before();
             __syncwarp();
             mbar_arrive_by(lane == 0, bar(Sh::kFullP + (j & 1)));

@@ -196,18 +196,6 @@ __host__ __device__ constexpr int tc_smem_bytes(int NT, bool split) { return 102
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
-// Instruction descriptor: D fp32, A = B = bf16, both K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-}
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-
 // SPLIT: one tile per cluster of `ksplit` CTAs; otherwise persistent CTAs walk the tiles, weight rows fastest while the
 // weights stay in L2, activation rows fastest when they do not (`ksplit` != 0 there).
 template <int NT, bool SPLIT>
@@ -294,7 +282,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     } else if (warp == 1) {
         // the whole warp walks the loop, one elected lane issues (see elect_one)
-        const uint32_t idesc = idesc_bf16(NT);
+        const uint32_t idesc = tc::idesc_bf16(NT);
         const bool elected = tc::elect_one();
         int n = 0, w = 0;
         bool ok = true;
@@ -311,7 +299,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     const uint64_t db = desc_sw128(smem_u32(stage0 + s * BYTES + kTcRows * 128));
 #pragma unroll
                     for (int k = 0; k < kTcK / 16; ++k)   // 16 k = 32 bytes further inside the swizzle atom
-                        tc_mma_f16(tmem + d * NT, da + 2 * k, db + 2 * k, idesc, kb > kb0 || k > 0);
+                        tc::tc_mma_bf16(tmem + d * NT, da + 2 * k, db + 2 * k, idesc, kb > kb0 || k > 0);
                     tc::tc_commit(empty(s));
                 }
                 __syncwarp();

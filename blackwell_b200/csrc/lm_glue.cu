@@ -595,8 +595,10 @@ static cudaError_t gated_norm_as(A* out, long ldout, const float* o, long ldo, c
     }
     const bool wide = part > 512;
     auto kern = gate_first ? (wide ? gated_norm_runs_kernel<A, 8, true, true> : gated_norm_runs_kernel<A, 4, true, true>)
-                           : (vec ? (wide ? gated_norm_runs_kernel<A, 8, false, true> : gated_norm_runs_kernel<A, 4, false, true>)
-                                  : gated_norm_runs_kernel<A, 4, false, false>);
+                : vec && wide ? gated_norm_runs_kernel<A, 8, false, true> : gated_norm_runs_kernel<A, 4, false, false>;
+    if constexpr (sizeof(A) == 4) {
+        if (!gate_first && vec && !wide) kern = gated_norm_runs_kernel<A, 4, false, true>;
+    }
     return launch_pdl(kern, dim3((unsigned)(all + 7) / 8), dim3(256), 0, st, out, ldout, o, ldo, gate, ldg, w, T, groups, part, eps);
 }
 

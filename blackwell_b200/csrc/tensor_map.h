@@ -13,6 +13,8 @@ constexpr int kMapCols = 64;   // columns of a box: one 128-byte swizzle atom
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// The driver's tensor-map encoder, looked up through the runtime so that the library carries no link-time dependency on libcuda (it
+// must load on machines without a driver).
 inline EncodeTiledFn encode_fn() {
     static EncodeTiledFn fn = nullptr;
     static std::once_flag once;
