@@ -2,14 +2,15 @@
 //
 // With eight (or four) query heads per KV head the scalar kernel spends more instructions per cache byte than an SM
 // can issue at HBM speed; here the heads of one KV head form the 16 rows of an MMA tile (rows >= the group size are
-// zero), K and V rows stream through shared memory (cp.async, three buffers per warp, XOR-swizzled 16-byte chunks,
+// zero), K and V rows stream through shared memory (cp.async, two or three buffers per warp, XOR-swizzled 16-byte chunks,
 // read back with ldmatrix), and a warp handles 16 positions per step:
 //     S = Q K^T   : 8 k-steps x 2 position tiles                 (Q fragments live in registers)
 //     online softmax on the accumulator fragment (row = head: quad shuffles)
 //     O += P V    : 16 dimension tiles, P taken straight from the S fragment
 // Q and P are split into a binary16 high part and a binary16 remainder and multiplied twice, so the products carry
 // ~22 significant bits although the operands of one MMA are binary16; K and V are binary16 in the cache already.
-// Splits, per-warp merge and the last-arriver split merge are those of the scalar kernel.
+// Splits and per-warp merge are those of the scalar kernel; up to eight splits merge as a cluster, more of them as there, by the one that
+// arrives last.
 #pragma once
 #include <cuda_fp16.h>
 #include <limits.h>

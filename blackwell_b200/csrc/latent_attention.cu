@@ -150,7 +150,7 @@ cudaError_t latent_expanded(const LatentArgs& a, const Rows& r, cudaStream_t st)
     if (e != cudaSuccess) return e;
     // tcgen05 for every number of rows: with the products of keys and values, 16 heads of 128 (64 of them rotated again) and 128 values,
     // mma.sync / tcgen05: 12.5 / 10.2 us at 17 rows, 14.3 / 11.9 at 64, 28 / 19.4 at 256, 75 / 41 at 1024, 449 / 134 at 4096; 17 rows
-    // after 4000 keys 270 / 101, 300 rows 290 / 116; 64 heads at 300 rows 40 / 25.  Error against 64 bits the same in six digits.
+    // after 4000 keys 270 / 101, 300 rows 290 / 116; 64 heads at 300 rows 40 / 25.  Error of the attention against 64 bits the same in six digits.
     if (flash_tc_can(a, r))
         return a.dim == 64 ? (a.V == 64 ? flash_tc<1, 1>(a, r, st) : flash_tc<1, 2>(a, r, st))
                            : (a.V == 64 ? flash_tc<2, 1>(a, r, st) : flash_tc<2, 2>(a, r, st));

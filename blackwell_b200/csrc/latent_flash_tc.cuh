@@ -10,7 +10,7 @@
 //   O += P V       V from shared memory as it lies there ([key][column]: B is MN-major)
 // O stays in tensor memory.  It is brought to a new maximum only when that grew by more than 2^8 (exp2 of the difference is exact
 // bookkeeping: P and the sum use the same base, and the last step divides one by the other); otherwise the softmax never waits for
-// the second product.
+// the second product (the conditional rescaling published with FlashAttention-4).
 // What bounds it: per 64 keys and 128 rows 896 cycles of the tensor pipe (384 for 192 columns of S, 512 for P V with its remainders)
 // against some 500 issue slots of each softmax warp.
 // Measured 1.6 us a tile where a block has its SM to itself, 1.9 us for the two tiles of two blocks: the softmax is the chain (a second

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(256) gated_norm_runs_kernel(A* out, long ldout
 // bf16, a head per group without padding, everything aligned, the gate last, up to KV * 128 columns: a warp per group, which requests
 // outputs, gates and weight before it sums.  Two round trips to memory one after the other bounded the kernel above here: 2,502 rows
 // of 32 x 128 columns 40 us, now 26.5 (31 with four groups a warp; 82 MB are 13 us, the exact divisions of the gates as long again),
-// 4,096 rows of 8 x 512 40.8 -> 30.4, 32 rows of 8 x 512 5.9 -> 4.9.
+// 4,096 rows of 8 x 512 40.8 -> 27, 32 rows of 8 x 512 5.9 -> 4.9.
 template <int KV>
 __global__ void __launch_bounds__(256) gated_norm_heads_kernel(bf16* out, long ldout, const float* o, long ldo, const bf16* gate, long ldg,
                                                                const float* w, int T, int groups, int V, float eps) {

@@ -72,7 +72,7 @@ bool recurrence_chunk_supported(const RecurrenceArgs& a) { return a.N <= 256 && 
 
 cudaError_t recurrence_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st) {
     if (a.groups < 1 || a.heads % a.groups != 0 || a.delta || !recurrence_chunk_supported(a)) return cudaErrorInvalidValue;
-    // narrow state tiles while the wide ones leave SMs idle or two narrow CTAs share an SM
+    // narrow state tiles while the wide ones of one run leave SMs idle or two narrow CTAs share an SM (several runs take the same tiles)
     const int wide = (pad8(a.V) + 63) / 64 * a.heads, sms = sm_count(current_device());
     const bool pairs = ChunkSmem(a.N, 32, 2).total <= 112 * 1024;
     const bool narrow = a.V <= 32 || wide <= (pairs ? sms : sms / 2) || ChunkSmem(a.N, 64, 1).total > kMaxDynSmem;
@@ -88,7 +88,7 @@ cudaError_t delta_chunk(const RecurrenceArgs& a, const Runs& rs, cudaStream_t st
     if (a.groups < 1 || a.heads % a.groups != 0 || !a.delta || !a.chunk_scratch || !a.log_decay || !a.weight ||
         !delta_chunk_supported(a))
         return cudaErrorInvalidValue;
-    // wide state tiles only where the narrow ones need more than one round of CTAs
+    // wide state tiles only where the narrow ones of one run need more than one round of CTAs (several runs take the same tiles)
     const int sms = sm_count(current_device()), narrow = (pad8(a.V) + 31) / 32 * a.heads;
     const bool wide = a.V > 32 && narrow > sms && DeltaSmem(a.N, 64, 1).total <= kMaxDynSmem;
     if (pad16(a.N) <= 128) return wide ? delta_inst<1, 64>(a, rs, st) : delta_inst<1, 32>(a, rs, st);

@@ -363,7 +363,8 @@ typedef struct bw_decode_config {
     int use_graph;            /* capture the step once and replay it */
     const char* weights_dir;  /* read during bw_decode_create only */
     int compute_f32;          /* config.json models: 1 = 32-bit activations and products (0: bfloat16) */
-    int max_portion;          /* config.json models: most tokens of one sequence per pass (0: automatic) */
+    int max_portion;          /* config.json models: most tokens of one sequence per pass, and rows of the work buffers.  0: up to 4,096
+                               * (512 with compute_f32), and work buffers for min(4,096 or 512, batch * max_seq) rows */
 } bw_decode_config;
 int bw_decode_create(const bw_decode_config* cfg, bw_decode** out);
 int bw_decode_get_config(const bw_decode* d, bw_decode_config* out);
