@@ -19,7 +19,7 @@ namespace wide {
 
 // ----------------------------------------------------------------------------------------------------------
 // Activation prep of the tensor-core kernel: quantizes every sequence once (int8 rule; plain / RMSNorm / SwiGLU, or int8 as
-// it comes) and stores x = xq x_sc as three bf16 parts in units of u (gemm_w4a8_wide.cuh) in the layout of the MMA's B operand:
+// it comes) and stores x = xq x_sc as three bf16 parts in units of u (gemm_w4a8_wide.cuh; `six`: for six products) in the layout of the MMA's B operand:
 //   chunk c: [half 0..1][block 0..7][k half][x1, x2, x3][NP rows x 16 B: eight bf16]   then   [NP] units u
 // Half h holds the chunk's blocks whose index has bit 2 equal to h, in order.  The eight elements of a k half are in the order in
 // which the unpack takes the nibbles of a word: 0 4 1 5 2 6 3 7.  k-blocks >= K/16 of the last chunk are zero (their weights
@@ -27,7 +27,7 @@ namespace wide {
 // sequence's results non-finite.  Zeroes the arrival counters of equal shares (`ncounters`, or 0).  Grid (ceil(chunks / 8), M), 256
 // threads of eight elements, a warp per chunk; starts early under programmatic dependent launch.
 // ----------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int NP, int nchunks,
+__global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const GemvArgs a, int NP, int nchunks, int six,
                                                      unsigned int* counters, int ncounters) {
     __shared__ float part[8];
     pdl_trigger();
@@ -59,18 +59,23 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
         }
     }
     // u = 2^e with e the exponent of the chunk's largest |x| / 128 (so |x| < 256 u), within what has a normal reciprocal or 2^-127
-    float f[8], big = 0.f;
+    float f[8], big = 0.f, sum = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         f[i] = (float)(int8_t)q[i];
         big = fmaxf(big, fabsf(f[i]));
+        sum += fabsf(f[i]);
     }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);   // of the block
     if (big == 0.f && fabsf(sc) < INFINITY) sc = 0.f;   // (0 times a scale far above the chunk's)
     float top = big * (fabsf(sc) * 0.0078125f);
 #pragma unroll
     for (int i = 16; i > 0; i >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, i));
     const uint32_t eb = min(max(__float_as_uint(top) & 0x7F800000u, 0x00800000u), 0x7F000000u);
-    const float rs = sc * __uint_as_float(eb == 0x7F000000u ? 0x00400000u : 0x7F000000u - eb);   // x_sc / u: exact
+    const float ru = __uint_as_float(eb == 0x7F000000u ? 0x00400000u : 0x7F000000u - eb), rs = sc * ru;   // 1 / u; x_sc / u: exact
+    // x1's places (see kFine) times 1.5 * 2^23: adding and taking that away rounds to them
+    const float mean = __uint_as_float(__float_as_uint(sum * (fabsf(sc) * 0.0625f)) & 0x7F800000u) * ru;
+    const float places = (six ? 1.f : fminf(mean * kFine, 1.f)) * kMagicFloat;
     const int c = e0 / kKc, b = (e0 >> 4) % kBlocksPerChunk;
     if (c >= nchunks) return;
     uint32_t o[3][4];
@@ -80,7 +85,7 @@ __global__ void __launch_bounds__(256) prep_x_kernel(unsigned char* xb, const Ge
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const float v = f[i + 4 * j];
-            p[0][j] = rintf(v * rs);
+            p[0][j] = __bfloat162float(__float2bfloat16_rn(__fadd_rn(__fmul_rn(v, rs), places) - places));
             const float r = fmaf(v, rs, -p[0][j]);   // exact: the product's upper bits are gone
             p[1][j] = __bfloat162float(__float2bfloat16_rn(r));
             p[2][j] = r - p[1][j];
@@ -682,7 +687,8 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
 
-    e = launch_pdl(prep_x_kernel, dim3((lay.nchunks + 7) / 8, M), dim3(256), 0, st, scratch + lay.xb_off, a, lay.NE, lay.nchunks,
+    const int six = lay.NE == 16 || a.K <= kSixK;
+    e = launch_pdl(prep_x_kernel, dim3((lay.nchunks + 7) / 8, M), dim3(256), 0, st, scratch + lay.xb_off, a, lay.NE, lay.nchunks, six,
                    reinterpret_cast<unsigned int*>(scratch), lay.csize == 1 ? lay.tiles * kWorkers : 0);
     count_launch(1);
     if (e != cudaSuccess) return e;
@@ -697,7 +703,7 @@ cudaError_t launch(const GemvArgs& a, int M, cudaStream_t st) {
     t.partial = reinterpret_cast<float*>(scratch + lay.part_off);
     t.tickets = reinterpret_cast<unsigned int*>(scratch);
     t.status = a.status;
-    t.N = a.N; t.M = M; t.nchunks = lay.nchunks; t.tiles = lay.tiles; t.csize = lay.csize; t.six = a.K <= kSixK;
+    t.N = a.N; t.M = M; t.nchunks = lay.nchunks; t.tiles = lay.tiles; t.csize = lay.csize; t.six = six;
     switch (lay.NE) {
         case 16: return launch_n<16>(map_w, t, lay.grid, st);
         case 32: return launch_n<32>(map_w, t, lay.grid, st);

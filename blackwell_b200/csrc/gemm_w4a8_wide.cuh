@@ -10,16 +10,16 @@
 //   Activations: x = xq x_sc is cut into x1 + x2 + x3 in units of a power of two u per (sequence, chunk), u the place of the eighth
 //   bit of the chunk's largest |x|: x1 = x rounded to whole units (|x1| <= 256), x2 the rest as a bf16 number, x3 what is still
 //   left as another.  Of an element 2^-19 u is lost at most, 2^-26 of the chunk's largest |x|, and never more than 2^-18 of itself.
-// Products: q sh x1 | q sh x2, q sh x3, q sl x1, q sl x2, and q sl x3 where the chains of sums are short (WideArgs::six): without
-// it up to 2^-15 u |w| more is lost, never more than 2^-14 of the element's own product.
-// So this is fixed point over 256 k of a sequence, not 24 bits of every block.  Where activations of about one size meet weights of about
-// one size that is 8e-8 of a result with five products and 3e-8 with six, less than the sums of the other forms lose.  Where one block of a
-// chunk is f times the others and its weights are zero, the others' bits are what counts: 4,096 x 4096, 2-norm against 64 bits, five
-// products / six (12 sequences) / every block scaled by itself: f = 4 2.9e-7 / 0.7e-7 / 1.5e-7, f = 64 4.5e-6 / 5.5e-7 / 1.5e-7, f = 1,024
-// 2.2e-5 / 2.6e-6 / 1.5e-7 (quantizing to int8 loses 5e-3).  Finer places of x1 for such blocks do not help: the first sum is then
-// no longer exact (below) and blocks of very different sizes lose 2.8e-7 where they now lose 1.1e-7.  bw_set_tuning key 24 < 0 chooses
-// the forms that scale every block by itself.
-// The first product has an accumulator of its own: x1 and, where the scales of a row's chunk share an exponent, q sh are whole
+// Products: q sh x1 | q sh x2, q sh x3, q sl x1, q sl x2, and q sl x3 where the chains of sums are short (WideArgs::six).  Without
+// it up to 2^-15 u |w| more would be lost; x1 then has finer places where its block is far below the chunk's largest (kFine), so that it
+// is 2^-20 of the block's mean |x| and 2^-23 of the element at most.
+// So this is fixed point over 256 k of a sequence, not 24 bits of every block.  On what the path meets it loses less than the sums of
+// the other forms do (beside kFine and preferred()).  Where one block of a chunk is f times the others and meets zero weights, the
+// others' bits are what counts: 4,096 x 4096, 2-norm against 64 bits, five products / six (12 sequences) / every block scaled by itself:
+// f = 64 1.2e-7 / 5.5e-7 / 1.7e-7, f = 1,024 1.2e-7 / 2.6e-6 / 1.7e-7; one element of every block 64 times the others 5e-7 / 5e-7 / 1.7e-7
+// (quantizing to int8 loses 5e-3).  Finer places help there and cost where blocks of very different sizes all count: the first sum is
+// then no longer exact (below).  bw_set_tuning key 24 < 0 chooses the forms that scale every block by itself.
+// The first product has an accumulator of its own: x1 (in whole units) and, where the scales of a row's chunk share an exponent, q sh are whole
 // numbers of one unit below 2^8 in magnitude, so its sum over 256 k stays below 2^24 units and is exact -- the tensor core cuts off
 // what an addition shifts out, which in one accumulator would cost up to a unit of the last place at every step, always towards
 // zero.  The others are 2^-5 to 2^-22 of the first; what is cut off there does not count.  The sum of both times u joins the fp32
@@ -78,6 +78,11 @@ constexpr int kWorkers = 16;                         // worker warps
 constexpr int kStageBytes = kWBytes + kRows * 32;    // and the scales: [blocks 0-7, 8-15][row][16 bytes]
 constexpr int kThreads = 128 + kWorkers * 32;        // two MMA issuers, activations, weights, workers
 constexpr int kScaleSlots = 4;    // chunks whose units u are in shared memory
+// Five products: x1 has places of kFine times the power of two below its block's mean |x|, where that is less than u.  Error against 64 bits
+// (2-norm, 1e-8; 5,632 x 2048, whole units / this / 2^-6, 2^-7 in a numpy restatement / every block scaled by itself): silu(g) u of normal g and
+// u 23 / 10 / 8, 8 / 13, one channel in 200 30 times the others 46 / 9 / 8, 8 / 13, block sizes spread evenly over 2^12 with such weights 21 / 27 /
+// 28, 30 / 13.  With six products the error is 5 to 9 on all but the last (11) without it, and the finer places would cost the last.
+constexpr float kFine = 0.03125f;
 constexpr int kSlots = 2;         // A slots of a row group, four k-blocks each (eight in one slot, at 32 sequences: 86 against 78 us)
 // Registers by role: the launch gives every thread 96; the first four warps keep 32, the workers take 112.
 constexpr int kRegsFew = 32, kRegsWork = 112;

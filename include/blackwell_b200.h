@@ -52,8 +52,8 @@ int bw_gemv_int4_warp(float* y_out, const void* x_packed, const float* x_scale, 
  * (K % 32 == 0, 16-byte aligned W and x) in one of the tcgen05 kernels, 64 sequences per launch; operands the
  * tensor-core kernel cannot take fall back to passes of 16 through the mma.sync kernel (or 8 through dp4a).
  *   The tcgen05 kernel's usual form takes activations in fixed point over 256 k of a sequence: of x = x_q * x_scale at most 2^-26 of the
- * largest |x| there is lost (2^-22 above 16 sequences with K > 3072), and never more than 2^-18 (2^-14) of x itself.  Key 24 < 0
- * chooses the forms that scale every block of 16 by itself. */
+ * largest |x| there is lost and never more than 2^-18 of x itself; above 16 sequences with K > 3072 2^-22 of the largest, and never more than
+ * 2^-20 of the mean |x| of its block of 16 and 2^-23 of x.  Key 24 < 0 chooses the forms that scale every block by itself. */
 int bw_gemv_w4a8(float* y_out, const int8_t* x_q, const float* x_scale, const uint8_t* W_packed,
                  const uint16_t* W_scale_f16, int K, int N, int M, void* stream);
 

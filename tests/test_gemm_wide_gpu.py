@@ -264,8 +264,9 @@ def test_a_call_that_may_not_grow_the_scratch_is_still_taken(k, M, K):
 @pytest.mark.parametrize("M,K,N,factor", [(17, 1024, 300, 64), (12, 2048, 300, 1024), (20, 3104, 300, 4), (32, 4096, 300, 64), (64, 4096, 300, 1024)])
 def test_blocks_far_below_the_largest_of_their_chunk(k, M, K, N, factor):
     """One block in 16 carries larger activations on weights that are zero.  Of an element min(2^-19 u, 2^-18 |x|) is lost, u = 2^-7 of
-    the power of two below the chunk's largest |x|, and min(2^-15 u, 2^-14 |x|) more with five products.  These roundings are independent and
-    of both signs: their 2-norm bounds that of the error, beside the fp32 sums.  Without x3 at all 2^-9 |x| would be lost."""
+    the power of two below the chunk's largest |x|; with five products min(2^-15 p, 2^-14 |x|) + 2^-23 |x| more, p the lesser of u and 2^-5 of
+    the power of two below the block's mean |x|.  These roundings are independent and of both signs: their 2-norm bounds that of the error,
+    beside the fp32 sums.  Without x3 at all 2^-9 |x| would be lost."""
     import torch
 
     W, sc16, _ = synth.int4_weights(N, K, seed=K, full_range=True)
@@ -285,7 +286,43 @@ def test_blocks_far_below_the_largest_of_their_chunk(k, M, K, N, factor):
     u = np.repeat(2.0 ** (np.floor(np.log2(top)) - 7), 256, 1)[:, :K]
     lost = np.minimum(2.0 ** -19 * u, 2.0 ** -18 * x)
     if M > 16 and K > 3072:
-        lost += np.minimum(2.0 ** -15 * u, 2.0 ** -14 * x)
+        mean = np.repeat(x.reshape(M, -1, 16).mean(2), 16, 1)
+        p = np.minimum(u, 2.0 ** (np.floor(np.log2(mean)) - 5))
+        lost += np.minimum(2.0 ** -15 * p, 2.0 ** -14 * x) + 2.0 ** -23 * x
     bound = np.sqrt((lost ** 2 @ (w ** 2).T).sum()) + (K // 256 + 2) ** 0.5 * 2.0 ** -24 * np.linalg.norm(ref)
     assert np.linalg.norm(y.cpu().numpy() - ref) < bound
     assert bound < 2.0 ** -12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("kind", ["normal", "silu", "channels", "tails", "lognormal"])
+@pytest.mark.parametrize("M,K,N", [(48, 2048, 3072), (64, 5632, 2048), (20, 12288, 1000)])
+def test_no_further_from_64_bits_than_the_form_that_scales_every_block(k, M, K, N, kind):
+    """Activations as the products meet them: after a norm, silu(g) u, a few large channels, long tails, channels of many sizes."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    n = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    x = n(M, K)
+    if kind == "silu":
+        x = torch.nn.functional.silu(x) * n(M, K)
+    elif kind == "channels":
+        x[:, ::200] *= 30
+    elif kind == "tails":
+        x = x / ((n(M, K) ** 2 + n(M, K) ** 2 + n(M, K) ** 2) / 3).sqrt()
+    elif kind == "lognormal":
+        x = x * n(1, K).exp()
+    W, sc = synth.int4_weights_device(N, K, 41)
+    xq, xs = torch.empty((M, K), dtype=torch.int8, device="cuda"), torch.empty((M, K // 16), device="cuda")
+    k.quantize_int8(xq, xs, x.contiguous(), M * K)
+    q = torch.stack([W & 15, W >> 4], 2).view(N, K).double() - 8
+    each = lambda v, s: (v.double().view(len(v), -1, 16) * s.double()[..., None]).view(len(v), K)
+    want, err = each(xq, xs) @ each(q, sc).T, []
+    for form in (1, -1):
+        y = torch.empty((M, N), device="cuda")
+        k.set_tuning(24, form)
+        try:
+            k.gemv_w4a8(y, xq, xs, W, sc, K, N, M)
+        finally:
+            k.set_tuning(24, 1)
+        err.append(float((y.double() - want).norm() / want.norm()))
+    assert err[0] < err[1] < 4e-7, err
